@@ -83,16 +83,16 @@ int tab_quantize_launch(const float* x, const float* ths, int64_t* qx, int32_t* 
     if (N == 0) return TAB_OK;
     if (misaligned(btn, 3)) return TAB_E_ALIGNMENT;
     cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-    if (btn) {
+    if ((long long)H * W == 0) {
+        if (!btn) return TAB_OK;
         cudaError_t e = cudaMemsetAsync(btn, 0, sizeof(int32_t) * (size_t)N, s);
-        if (e != cudaSuccess) return record_cuda_error(e);
+        return e == cudaSuccess ? TAB_OK : record_cuda_error(e);
     }
-    if ((long long)H * W == 0) return TAB_OK;
     if (!x || !ths || !qx) return TAB_E_NULL_POINTER;
     if (misaligned(x, 3) || misaligned(ths, 3) || misaligned(qx, 7)) return TAB_E_ALIGNMENT;
     if ((long long)H * W >= (1LL << 31)) return TAB_E_TOO_LARGE;
     const int bits = (bitwidth == 1) ? 1 : 2;                      // TAB_GEMM.cu:267,309
-    return quantize_dispatch(x, ths, qx, bits == 2 ? btn : nullptr, bits, N, H, W, C, s);
+    return quantize_dispatch(x, ths, qx, btn, bits, N, H, W, C, s);
 }
 
 size_t tab_conv2d_workspace_bytes(int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW) {
@@ -315,16 +315,7 @@ int tab_quantize_auto_launch(const float* x, float scale, void* state, float* th
     if ((long long)H * W >= (1LL << 31)) return TAB_E_TOO_LARGE;
     double* sums = reinterpret_cast<double*>(state);
     unsigned* bar = reinterpret_cast<unsigned*>(sums + N) + 1;
-    int rc = quantize_auto_dispatch(x, scale, sums, bar, ths, qx, bitwidth == 1 ? 1 : 2, N, H, W, C, device_status_word(), s);
-    if (rc != TAB_E_TOO_LARGE) return rc;
-    // shapes the one-launch form does not take: sums, thresholds, quantiser as launches of their own (x is not modified)
-    rc = residual_abs_sum_dispatch(const_cast<float*>(x), nullptr, sums, N, per_image, s);
-    if (rc != TAB_OK) return rc;
-    rc = tab_threshold_from_sums_launch(sums, ths, scale, N, per_image, stream);
-    if (rc != TAB_OK) return rc;
-    cudaError_t e = cudaMemsetAsync(sums, 0, sizeof(double) * (size_t)N, s);
-    if (e != cudaSuccess) return record_cuda_error(e);
-    return quantize_dispatch(x, ths, qx, nullptr, bitwidth == 1 ? 1 : 2, N, H, W, C, s, nullptr, false);
+    return quantize_auto_dispatch(x, scale, sums, bar, ths, qx, bitwidth == 1 ? 1 : 2, N, H, W, C, device_status_word(), s);
 }
 
 int tab_quantize_i16_launch(const int16_t* x, const float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C, tab_stream_t stream) {

@@ -11,14 +11,14 @@
 // its 8 channels into one byte per plane with compares and predicated ORs and stores those bytes
 // itself - no shuffles, votes or redux (a first version merged nibbles with redux.sync and was bound
 // by that instruction's pipe at 37 % of DRAM bandwidth).
-// General path (any C, any alignment): one warp per word, two coalesced 32-bit loads per lane, the
-// two 32-bit halves come straight out of __ballot_sync.
+// Any other C or alignment: the same division of labour with the widest loads the rows allow (quantize_any_kernel).
 //
 // Inside a convolution call the same launch also does the call's small set-up jobs (QuantExtras), so that they cost no
 // launch of their own: all CTAs share the expansion of the packed weights to the bytes the tensor-core kernel
 // multiplies, and the first CTA of every image clears that image's |y| sum (the first of all the completion counter).
 #include <mutex>
 #include "tab_kernels.cuh"
+#include "umma_common.cuh"
 
 namespace tab {
 
@@ -211,59 +211,202 @@ quantize_c64_kernel(const void* __restrict__ x, const float* __restrict__ ths,
             int tot = 0;
 #pragma unroll
             for (int i = 0; i < QTHREADS / 32; i++) tot += wsum[i];
-            if (tot) atomicAdd(btn + n, tot);                 // integer: order-independent, exact
+            if (gridDim.x == 1) btn[n] = tot;                 // the image's only CTA
+            else if (tot) atomicAdd(btn + n, tot);            // integer: order-independent, exact
         }
     }
+    if (BITS == 1 && btn != nullptr && blockIdx.x == 0 && threadIdx.x == 0) btn[n] = 0;
     pdl_launch_dependents();                                  // the next kernel may be scheduled once every CTA got here
 }
 
-// One warp per output word; works for every C and alignment.  grid = (ctas_per_image, N).
-template <int BITS, bool IN16>
-__global__ void __launch_bounds__(QTHREADS)
-quantize_generic_kernel(const void* __restrict__ x, const float* __restrict__ ths,
-                        uint64_t* __restrict__ qx, int* __restrict__ btn,
-                        long long pixels_per_image, int C, int PC, const QuantExtras ex) {
-    const int n = blockIdx.y;
-    quant_prologue(ex, n);
-    const float t = __ldg(ths + n);
-    const float nt = -t;
-    const int lane = threadIdx.x & 31;
-    const int warp = threadIdx.x >> 5;
-    const long long words_per_image = pixels_per_image * PC;
-    const float* xi = reinterpret_cast<const float*>(x) + (IN16 ? 0 : (long long)n * pixels_per_image * C);
-    const int16_t* xs = reinterpret_cast<const int16_t*>(x) + (IN16 ? (long long)n * pixels_per_image * C : 0);
-    uint64_t* qi = qx + (long long)n * words_per_image * BITS;
-    int cnt = 0;
+// ---- any channel count, any alignment ------------------------------------------------------------------------------------
+// Eight consecutive channels of one pixel, as many elements per load as the rows' alignment allows: V = 8 (C % 8 == 0), 4, 2
+// or 1.  Channels from `valid` on are not read and come back as 0.  Rows whose length is no multiple of 32 bytes share
+// sectors between lanes and between the loads of one lane, so these loads may stay in L1 (no streaming hint).
+template <int V>
+__device__ __forceinline__ f8 ld8(const float* p, int valid) {
+    f8 r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = 0.f;
+    if (V == 8) {
+        if (valid > 0) r = ld_stream_f8(p);
+    } else if (V == 4) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 4)
+            if (valid > i) { const float4 q = __ldg(reinterpret_cast<const float4*>(p + i)); r.v[i] = q.x; r.v[i + 1] = q.y; r.v[i + 2] = q.z; r.v[i + 3] = q.w; }
+    } else if (V == 2) {
+#pragma unroll
+        for (int i = 0; i < 8; i += 2)
+            if (valid > i) { const float2 q = __ldg(reinterpret_cast<const float2*>(p + i)); r.v[i] = q.x; r.v[i + 1] = q.y; }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (valid > i) r.v[i] = __ldg(p + i);
+    }
+    return r;
+}
+template <int V>
+__device__ __forceinline__ f8 ld8(const int16_t* p, int valid) {                   // V is 8 or 1 here
+    f8 r;
+#pragma unroll
+    for (int i = 0; i < 8; i++) r.v[i] = 0.f;
+    if (V == 8) {
+        if (valid > 0) {
+            const uint4 q = __ldg(reinterpret_cast<const uint4*>(p));
+            const uint32_t w[4] = {q.x, q.y, q.z, q.w};
+#pragma unroll
+            for (int i = 0; i < 4; i++) { r.v[2 * i] = (float)(int16_t)(w[i] & 0xFFFFu); r.v[2 * i + 1] = (float)(int16_t)(w[i] >> 16); }
+        }
+    } else {
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            if (valid > i) r.v[i] = (float)__ldg(p + i);
+    }
+    return r;
+}
 
-    for (long long w = (long long)blockIdx.x * (QTHREADS / 32) + warp; w < words_per_image;
-         w += (long long)gridDim.x * (QTHREADS / 32)) {
-        const long long pix = w / PC;
-        const int pc = (int)(w - pix * PC);
-        const int c0 = pc * 64 + lane, c1 = c0 + 32;
-        const float* row = xi + pix * C;
-        const int16_t* rows = xs + pix * C;
-        const bool in0 = c0 < C, in1 = c1 < C;
-        const float a = in0 ? (IN16 ? (float)__ldg(rows + c0) : __ldg(row + c0)) : 0.f;
-        const float b = in1 ? (IN16 ? (float)__ldg(rows + c1) : __ldg(row + c1)) : 0.f;
+// How lanes share the words of an image.  L = 8: lane `byte` of a group of eight owns channels 8*byte .. 8*byte + 7 of a
+// word and writes that byte of every plane; L = 1 (C <= 8, a network's first layer): one lane per word.  A pass of a CTA
+// is QTHREADS / L words, a step QUNROLL passes.
+template <int L> __host__ __device__ constexpr int words_per_pass() { return QTHREADS / L; }
+struct WordAt { long long off; int valid; };                                       // element offset in the image, real channels of the lane's eight
+template <int L>
+__device__ __forceinline__ WordAt word_at(long long w, int C, int PC, const FastDiv& dPC, bool wide) {
+    const long long pix = L == 1 ? w : (wide ? w / PC : (long long)dPC.div((uint32_t)w));
+    const int c0 = L == 1 ? 0 : (int)(w - pix * PC) * 64 + (int)(threadIdx.x & 7) * 8;
+    WordAt a;
+    a.off = pix * C + c0;
+    a.valid = C - c0;
+    return a;
+}
+// Quantises a lane's eight channels and writes its share of word w; returns the number of nonzero ternary values.
+template <int BITS, int L>
+__device__ __forceinline__ int put8(const f8& x, int valid, float t, uint64_t* qi, long long w) {
+    const unsigned mask = valid >= 8 ? 0xFFu : (valid <= 0 ? 0u : (1u << valid) - 1u);
+    unsigned pos = 0, neg = 0;
+    const float nt = -t;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
         if (BITS == 2) {
-            const bool pa = in0 && a > t, pb = in1 && b > t;
-            const bool na = in0 && !pa && a < nt, nb = in1 && !pb && b < nt;
-            const unsigned s_lo = __ballot_sync(0xFFFFFFFFu, na), s_hi = __ballot_sync(0xFFFFFFFFu, nb);
-            const unsigned m_lo = __ballot_sync(0xFFFFFFFFu, pa || na), m_hi = __ballot_sync(0xFFFFFFFFu, pb || nb);
-            if (lane == 0) {
-                uint2* o = reinterpret_cast<uint2*>(qi + w * 2);
-                o[0] = make_uint2(s_lo, s_hi);
-                o[1] = make_uint2(m_lo, m_hi);
-                cnt += __popc(m_lo) + __popc(m_hi);
-            }
+            pos |= (x.v[i] > t) ? (1u << i) : 0u;
+            neg |= (x.v[i] < nt) ? (1u << i) : 0u;
         } else {
-            const unsigned b_lo = __ballot_sync(0xFFFFFFFFu, in0 && a < t);
-            const unsigned b_hi = __ballot_sync(0xFFFFFFFFu, in1 && b < t);
-            if (lane == 0) *reinterpret_cast<uint2*>(qi + w) = make_uint2(b_lo, b_hi);
+            neg |= (x.v[i] < t) ? (1u << i) : 0u;
         }
     }
-    if (BITS == 2 && btn != nullptr && lane == 0 && cnt) atomicAdd(btn + n, cnt);
+    pos &= mask;
+    neg &= mask & ~pos;                                                            // ternary: the "+1" branch is tested first
+    if (L == 1) {
+        qi[w * BITS] = neg;
+        if (BITS == 2) qi[w * BITS + 1] = pos | neg;
+    } else {
+        unsigned char* o = reinterpret_cast<unsigned char*>(qi) + w * (8 * BITS) + (threadIdx.x & 7);
+        o[0] = (unsigned char)neg;
+        if (BITS == 2) o[8] = (unsigned char)(pos | neg);
+    }
+    return BITS == 2 ? __popc(pos | neg) : 0;
+}
+
+// Same division of labour as quantize_c64_kernel for every other C and alignment.  grid = (ctas_per_image, N).
+// Bound by HBM where rows are vectors, by the L1's load path where they are not; the pixel of a word comes from a
+// multiply-high, every lane has QUNROLL * 8 channels in flight.  It replaces a warp-per-word ballot kernel, which had two
+// loads in flight per lane behind a 64-bit division.  B200, us before / after: binary 64x27x31x200 31.0 / 8.6 (5.2 TB/s),
+// ternary 64x56x56x70 57.4 / 22.8, 64x28x28x511 65.8 / 33.2 (single-element loads, 3.3 TB/s), 64x224x224x3 296 / 22.8.
+template <int BITS, bool IN16, int V, int L>
+__global__ void __launch_bounds__(QTHREADS, 4)
+quantize_any_kernel(const void* __restrict__ x, const float* __restrict__ ths, uint64_t* __restrict__ qx, int* __restrict__ btn,
+                    long long words_per_image, long long elems_per_image, int C, int PC, const FastDiv dPC, const QuantExtras ex) {
+    const int n = (int)(gridDim.y - 1u - blockIdx.y);         // back to front, as above
+    const unsigned bx = gridDim.x - 1u - blockIdx.x;
+    quant_prologue(ex, n);
+    const float t = __ldg(ths + n);
+    const bool wide = words_per_image >= (1LL << 31);
+    const int slot = threadIdx.x / L;
+    const float* xf = reinterpret_cast<const float*>(x) + (IN16 ? 0 : (long long)n * elems_per_image);
+    const int16_t* xs = reinterpret_cast<const int16_t*>(x) + (IN16 ? (long long)n * elems_per_image : 0);
+    uint64_t* qi = qx + (long long)n * words_per_image * BITS;
+    constexpr int PASS = words_per_pass<L>(), STEP = PASS * QUNROLL;
+    int cnt = 0;
+    for (long long w0 = (long long)bx * STEP + slot; w0 < words_per_image; w0 += (long long)gridDim.x * STEP) {
+        f8 v[QUNROLL];
+        int valid[QUNROLL];
+#pragma unroll
+        for (int u = 0; u < QUNROLL; u++) {
+            const long long w = w0 + u * PASS;
+            valid[u] = 0;
+            if (w < words_per_image) {
+                const WordAt a = word_at<L>(w, C, PC, dPC, wide);
+                valid[u] = a.valid;
+                if (IN16) v[u] = ld8<(V == 8 ? 8 : 1)>(xs + a.off, a.valid);
+                else v[u] = ld8<V>(xf + a.off, a.valid);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < QUNROLL; u++) {
+            const long long w = w0 + u * PASS;
+            if (w < words_per_image) cnt += put8<BITS, L>(v[u], valid[u], t, qi, w);
+        }
+    }
+    if (BITS == 2 && btn != nullptr) {
+        __shared__ int wsum[QTHREADS / 32];
+        cnt = __reduce_add_sync(0xFFFFFFFFu, cnt);
+        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = cnt;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int tot = 0;
+#pragma unroll
+            for (int i = 0; i < QTHREADS / 32; i++) tot += wsum[i];
+            if (gridDim.x == 1) btn[n] = tot;                 // the image's only CTA
+            else if (tot) atomicAdd(btn + n, tot);            // integer: order-independent, exact
+        }
+    }
+    if (BITS == 1 && btn != nullptr && blockIdx.x == 0 && threadIdx.x == 0) btn[n] = 0;
     pdl_launch_dependents();
+}
+
+// Elements per load that C and the address of x allow (rows start at multiples of C elements): 8, 4, 2 or 1.
+static int load_width(const void* x, int C, bool in16) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(x);
+    if (in16) return C % 8 == 0 && (a & 15) == 0 ? 8 : 1;
+    if (C % 8 == 0 && (a & 31) == 0) return 8;
+    if (C % 4 == 0 && (a & 15) == 0) return 4;
+    return C % 2 == 0 && (a & 7) == 0 ? 2 : 1;
+}
+
+// CTAs per image: every CTA the same whole number of steps (a ragged last step, or a nearly empty extra wave, costs a
+// whole step's time), at most about six waves of eight CTAs per SM over all images.
+static unsigned ctas_per_image(long long words_per_image, long long words_per_step, int N) {
+    const long long steps = (words_per_image + words_per_step - 1) / words_per_step;
+    const long long cap = 148LL * 8 * 6;
+    const long long iters = ((long long)N * steps + cap - 1) / cap;        // steps per CTA
+    const long long per_image = (steps + iters - 1) / iters;
+    return (unsigned)(per_image < 1 ? 1 : per_image);
+}
+
+// BTN_W is cleared by a memset only where several CTAs add to an image's count; else the kernel writes it.
+static int clear_counts(int32_t* btn, int bits, dim3 grid, cudaStream_t stream) {
+    if (!btn || bits == 1 || grid.x == 1) return TAB_OK;
+    const cudaError_t e = cudaMemsetAsync(btn, 0, sizeof(int32_t) * (size_t)grid.y, stream);
+    return e == cudaSuccess ? TAB_OK : record_cuda_error(e);
+}
+
+template <int BITS, bool IN16>
+static int launch_quantize_any(const void* x, const float* ths, uint64_t* q, int32_t* btn, int N, long long pixels, int C,
+                               cudaStream_t stream, const QuantExtras& ex) {
+    const int PC = (C + 63) / 64;
+    const long long wpi = pixels * PC;
+    const FastDiv dPC = make_fastdiv((uint32_t)PC);
+    const int V = load_width(x, C, IN16);
+    const bool one = C <= 8;                                               // one lane per word
+    const dim3 grid(ctas_per_image(wpi, (long long)QTHREADS / (one ? 1 : 8) * QUNROLL, N), (unsigned)N);
+    const int rc = clear_counts(btn, BITS, grid, stream);
+    if (rc != TAB_OK) return rc;
+#define TAB_QANY(VV) (one ? launch_pdl(quantize_any_kernel<BITS, IN16, VV, 1>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, pixels * C, C, PC, dPC, ex) \
+                          : launch_pdl(quantize_any_kernel<BITS, IN16, VV, 8>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, pixels * C, C, PC, dPC, ex))
+    if (V == 8) return TAB_QANY(8);
+    if (IN16 || V == 1) return TAB_QANY(1);
+    return V == 4 ? TAB_QANY((IN16 ? 1 : 4)) : TAB_QANY((IN16 ? 1 : 2));
+#undef TAB_QANY
 }
 
 int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn, int bits,
@@ -287,38 +430,18 @@ int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn
     const bool fast = (C % 64 == 0) && ((reinterpret_cast<uintptr_t>(x) & 31) == 0);
     uint64_t* q = reinterpret_cast<uint64_t*>(qx);
     if (fast) {
-        // CTAs per image: every CTA the same whole number of 128-word steps (a ragged last step, or a nearly empty extra
-        // wave, costs a whole step's time), at most about six waves of eight CTAs per SM over all images
-        const long long words_per_step = in16 ? 2 * QWORDS_PER_ITER : QWORDS_PER_ITER;
-        const long long steps = (wpi + words_per_step - 1) / words_per_step;
-        const long long cap = 148LL * 8 * 6;
-        const long long iters = ((long long)N * steps + cap - 1) / cap;    // steps per CTA
-        long long per_image = (steps + iters - 1) / iters;
-        if (per_image < 1) per_image = 1;
-        dim3 grid((unsigned)per_image, (unsigned)N);
+        const dim3 grid(ctas_per_image(wpi, in16 ? 2 * QWORDS_PER_ITER : QWORDS_PER_ITER, N), (unsigned)N);
+        const int rc = clear_counts(btn, bits, grid, stream);
+        if (rc != TAB_OK) return rc;
         if (in16) {
             if (bits == 2) return launch_pdl(quantize_c64_kernel<2, true>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, ex);
             return launch_pdl(quantize_c64_kernel<1, true>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, ex);
         }
         if (bits == 2) return launch_pdl(quantize_c64_kernel<2, false>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, ex);
         return launch_pdl(quantize_c64_kernel<1, false>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, ex);
-    } else {
-        long long steps = (wpi + (QTHREADS / 32) - 1) / (QTHREADS / 32);
-        long long per_image = steps;
-        const long long target_total = 148LL * 8 * 8;
-        if ((long long)N * per_image > target_total) {
-            per_image = (target_total + N - 1) / N;
-            if (per_image < 1) per_image = 1;
-            if (per_image > steps) per_image = steps;
-        }
-        dim3 grid((unsigned)per_image, (unsigned)N);
-        if (in16) {
-            if (bits == 2) return launch_pdl(quantize_generic_kernel<2, true>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, pixels, C, PC, ex);
-            return launch_pdl(quantize_generic_kernel<1, true>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, pixels, C, PC, ex);
-        }
-        if (bits == 2) return launch_pdl(quantize_generic_kernel<2, false>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, pixels, C, PC, ex);
-        return launch_pdl(quantize_generic_kernel<1, false>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, pixels, C, PC, ex);
     }
+    if (in16) return bits == 2 ? launch_quantize_any<2, true>(x, ths, q, btn, N, pixels, C, stream, ex) : launch_quantize_any<1, true>(x, ths, q, btn, N, pixels, C, stream, ex);
+    return bits == 2 ? launch_quantize_any<2, false>(x, ths, q, btn, N, pixels, C, stream, ex) : launch_quantize_any<1, false>(x, ths, q, btn, N, pixels, C, stream, ex);
 }
 
 // ---- thresholds and bit-planes of a tensor in one launch ----------------------------------------------------------------
@@ -326,51 +449,66 @@ int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn
 // and the quantisation against them, as two phases of one persistent grid: per-image sums of |x| (double atomics), a
 // grid-wide counter (all CTAs are resident: the grid is sized by the occupancy calculator; the wait is bounded and
 // reports in *status), then every CTA quantises, last unit first, the units it has just summed - the end of its share is
-// what the L2 still holds.  A unit is one CTA step of 128 words of one image.
+// what the L2 still holds, and its last unit is still in registers.  A unit is one CTA step (QUNROLL passes) of one image; a
+// CTA owns consecutive units, so that its sum leaves the registers once per image and not once per unit.
+// FULL: C % 64 == 0 and 32-byte rows (every lane has eight real channels); else V and L as in quantize_any_kernel.
 constexpr uint32_t QA_WAIT_LIMIT = 1u << 22;
 
-template <int BITS>
-__global__ void __launch_bounds__(QTHREADS)
+template <int BITS, int V, int L, bool FULL>
+__global__ void __launch_bounds__(QTHREADS, 4)
 quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restrict__ sums, unsigned* __restrict__ bar,
-                     float* __restrict__ ths_out, uint64_t* __restrict__ qx, long long words_per_image, int steps_per_image,
-                     long long units, int N, int* __restrict__ status) {
+                     float* __restrict__ ths_out, uint64_t* __restrict__ qx, long long words_per_image, long long elems_per_image, int C, int PC,
+                     const FastDiv dPC, long long steps_per_image, long long units, int N, int* __restrict__ status) {
     pdl_wait();
-    const int byte = threadIdx.x & 7, grp = threadIdx.x >> 3;
-    const double per_image = (double)words_per_image * 64.0;
+    constexpr int PASS = words_per_pass<L>(), STEP = PASS * QUNROLL;
+    const int slot = threadIdx.x / L;
+    const bool wide = words_per_image >= (1LL << 31);
+    const double per_image = (double)elems_per_image;
     __shared__ double wsum[QTHREADS / 32];
     __shared__ float s_t;
-    // phase 1: sums
-    for (long long u = blockIdx.x; u < units; u += gridDim.x) {
-        const long long n = u / steps_per_image;
-        const long long w0 = (u - n * steps_per_image) * QWORDS_PER_ITER;
-        const float* xi = x + n * words_per_image * 64;
-        f8 v[QUNROLL];
-        bool live[QUNROLL];
+    auto at = [&](long long w) -> WordAt {
+        if (FULL) return WordAt{w * 64 + (long long)(threadIdx.x & 7) * 8, 8};
+        return word_at<L>(w, C, PC, dPC, wide);
+    };
+    f8 v[QUNROLL];
+    auto load_unit = [&](long long n, long long st) {
+        const float* xi = x + n * elems_per_image;
 #pragma unroll
         for (int k = 0; k < QUNROLL; k++) {
-            const long long w = w0 + k * (QTHREADS / 8) + grp;
-            live[k] = w < words_per_image;
-            if (live[k]) v[k] = ld_stream_f8(xi + w * 64 + byte * 8);
-        }
-        double acc = 0.0;
+            const long long w = st * STEP + k * PASS + slot;
 #pragma unroll
-        for (int k = 0; k < QUNROLL; k++)
-            if (live[k]) {
-                const float* q = v[k].v;
-                acc += (((double)fabsf(q[0]) + (double)fabsf(q[1])) + ((double)fabsf(q[2]) + (double)fabsf(q[3]))) +
-                       (((double)fabsf(q[4]) + (double)fabsf(q[5])) + ((double)fabsf(q[6]) + (double)fabsf(q[7])));
+            for (int i = 0; i < 8; i++) v[k].v[i] = 0.f;
+            if (w < words_per_image) { const WordAt a = at(w); v[k] = ld8<V>(xi + a.off, a.valid); }
+        }
+    };
+    // phase 1: sums
+    const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1LL) / gridDim.x;     // grid <= units: never empty
+    long long n = ub / steps_per_image, st = ub - n * steps_per_image;
+    double acc = 0.0;
+    for (long long u = ub; u < ue; u++) {
+        load_unit(n, st);
+#pragma unroll
+        for (int k = 0; k < QUNROLL; k++) {
+            const float* q = v[k].v;
+            acc += (((double)fabsf(q[0]) + (double)fabsf(q[1])) + ((double)fabsf(q[2]) + (double)fabsf(q[3]))) +
+                   (((double)fabsf(q[4]) + (double)fabsf(q[5])) + ((double)fabsf(q[6]) + (double)fabsf(q[7])));
+        }
+        const bool image_ends = st + 1 == steps_per_image;
+        if (image_ends || u + 1 == ue) {
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
+            __syncthreads();                                  // wsum of the previous image has been read
+            if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
+            __syncthreads();
+            if (threadIdx.x == 0) {
+                double t = 0.0;
+#pragma unroll
+                for (int i = 0; i < QTHREADS / 32; i++) t += wsum[i];
+                atomicAdd(sums + n, t);
             }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o);
-        __syncthreads();                                      // wsum of the previous unit has been read
-        if ((threadIdx.x & 31) == 0) wsum[threadIdx.x >> 5] = acc;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double t = 0.0;
-#pragma unroll
-            for (int i = 0; i < QTHREADS / 32; i++) t += wsum[i];
-            atomicAdd(sums + n, t);
+            acc = 0.0;
         }
+        if (u + 1 < ue) { if (image_ends) { n++; st = 0; } else st++; }
     }
     // grid-wide counter
     __threadfence();
@@ -391,46 +529,27 @@ quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restric
     }
     if (!__syncthreads_or(flag)) return;
     if (blockIdx.x == 0 && ths_out)
-        for (int n = threadIdx.x; n < N; n += QTHREADS) ths_out[n] = (float)((double)scale * (__ldcg(sums + n) / per_image));
-    // phase 2: the CTA's units again, last first
-    const long long mine = units > blockIdx.x ? (units - 1 - blockIdx.x) / gridDim.x : -1;      // index of its last unit
-    for (long long k = mine; k >= 0; k--) {
-        const long long u = blockIdx.x + k * gridDim.x;
-        const long long n = u / steps_per_image;
-        const long long w0 = (u - n * steps_per_image) * QWORDS_PER_ITER;
-        __syncthreads();
-        if (threadIdx.x == 0) s_t = (float)((double)scale * (__ldcg(sums + n) / per_image));
-        __syncthreads();
-        const float t = s_t, nt = -t;
-        const float* xi = x + n * words_per_image * 64;
-        unsigned char* qi = reinterpret_cast<unsigned char*>(qx + n * words_per_image * BITS);
-        f8 v[QUNROLL];
-        long long w[QUNROLL];
-#pragma unroll
-        for (int q = 0; q < QUNROLL; q++) {
-            w[q] = w0 + q * (QTHREADS / 8) + grp;
-            if (w[q] < words_per_image) v[q] = ld_stream_f8(xi + w[q] * 64 + byte * 8);
+        for (int m = threadIdx.x; m < N; m += QTHREADS) ths_out[m] = (float)((double)scale * (__ldcg(sums + m) / per_image));
+    // phase 2: the CTA's units again, last first (v still holds the last one)
+    long long tn = -1;
+    float t = 0.f;
+    for (long long u = ue - 1; u >= ub; u--) {
+        if (u != ue - 1) {
+            if (st == 0) { n--; st = steps_per_image - 1; } else st--;
+            load_unit(n, st);
         }
+        if (n != tn) {
+            __syncthreads();
+            if (threadIdx.x == 0) s_t = (float)((double)scale * (__ldcg(sums + n) / per_image));
+            __syncthreads();
+            t = s_t;
+            tn = n;
+        }
+        uint64_t* qi = qx + n * words_per_image * BITS;
 #pragma unroll
-        for (int q = 0; q < QUNROLL; q++) {
-            if (w[q] >= words_per_image) continue;
-            if (BITS == 2) {
-                unsigned pos = 0, neg = 0;
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    pos |= (v[q].v[i] > t) ? (1u << i) : 0u;
-                    neg |= (v[q].v[i] < nt) ? (1u << i) : 0u;
-                }
-                neg &= ~pos;
-                unsigned char* o = qi + w[q] * 16 + byte;
-                o[0] = (unsigned char)neg;
-                o[8] = (unsigned char)(pos | neg);
-            } else {
-                unsigned b = 0;
-#pragma unroll
-                for (int i = 0; i < 8; i++) b |= (v[q].v[i] < t) ? (1u << i) : 0u;
-                qi[w[q] * 8 + byte] = (unsigned char)b;
-            }
+        for (int k = 0; k < QUNROLL; k++) {
+            const long long w = st * STEP + k * PASS + slot;
+            if (w < words_per_image) put8<BITS, L>(v[k], FULL ? 8 : at(w).valid, t, qi, w);
         }
     }
     // the CTA that gets here last leaves the state block zero again (every CTA has read the sums it needs)
@@ -438,42 +557,64 @@ quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restric
     flag = 0;
     if (threadIdx.x == 0) flag = (atomicAdd(bar + 1, 1u) == gridDim.x - 1u) ? 1 : 0;
     if (__syncthreads_or(flag)) {
-        for (int n = threadIdx.x; n < N; n += QTHREADS) sums[n] = 0.0;
+        for (int m = threadIdx.x; m < N; m += QTHREADS) sums[m] = 0.0;
         if (threadIdx.x == 0) { bar[0] = 0u; bar[1] = 0u; }
     }
     pdl_launch_dependents();
 }
 
-// TAB_E_TOO_LARGE: the caller runs the separate launches instead (C not a multiple of 64, unaligned x).
-int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
-                           int N, int H, int W, int C, int* status, cudaStream_t stream) {
-    const long long wpi = (long long)H * W * (C / 64);
-    if (C % 64 != 0 || (reinterpret_cast<uintptr_t>(x) & 31) || wpi == 0 || N == 0) return TAB_E_TOO_LARGE;
-    const long long spi = (wpi + QWORDS_PER_ITER - 1) / QWORDS_PER_ITER;
-    if (spi >= (1LL << 31)) return TAB_E_TOO_LARGE;
-    const long long units = spi * N;
+template <int BITS, int V, int L, bool FULL>
+static int launch_quantize_auto(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx,
+                                int N, int H, int W, int C, int* status, cudaStream_t stream) {
+    const int PC = (C + 63) / 64;
+    const long long pixels = (long long)H * W, wpi = pixels * PC, step = (long long)words_per_pass<L>() * QUNROLL;
+    const long long spi = (wpi + step - 1) / step, units = spi * N;
     static std::mutex mu;
-    static int capacity[64][2] = {};                          // resident CTAs per device, per bitwidth
+    static int capacity[64] = {};                             // resident CTAs, per device
     int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return TAB_E_TOO_LARGE;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return record_cuda_error(e);
     int cap = 0;
     {
         std::lock_guard<std::mutex> lock(mu);
-        int& c = capacity[dev][bits == 2 ? 1 : 0];
-        if (!c) {
+        cap = dev < 64 ? capacity[dev] : 0;
+        if (!cap) {
             int per_sm = 0, sms = 0;
-            cudaError_t e = bits == 2 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_auto_kernel<2>, QTHREADS, 0)
-                                      : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_auto_kernel<1>, QTHREADS, 0);
-            if (e != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return record_cuda_error(cudaGetLastError());
-            c = per_sm * sms;
+            e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, quantize_auto_kernel<BITS, V, L, FULL>, QTHREADS, 0);
+            if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+            if (e != cudaSuccess) return record_cuda_error(e);
+            cap = per_sm * sms;
+            if (dev < 64) capacity[dev] = cap;
         }
-        cap = c;
     }
-    if (cap < 1) return TAB_E_TOO_LARGE;
     const unsigned grid = (unsigned)(units < cap ? units : cap);
-    uint64_t* q = reinterpret_cast<uint64_t*>(qx);
-    if (bits == 2) return launch_pdl(quantize_auto_kernel<2>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out, q, wpi, (int)spi, units, N, status);
-    return launch_pdl(quantize_auto_kernel<1>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out, q, wpi, (int)spi, units, N, status);
+    return launch_pdl(quantize_auto_kernel<BITS, V, L, FULL>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out,
+                      reinterpret_cast<uint64_t*>(qx), wpi, pixels * C, C, PC, make_fastdiv((uint32_t)PC), spi, units, N, status);
+}
+
+template <int BITS>
+static int quantize_auto_by_width(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx,
+                                  int N, int H, int W, int C, int* status, cudaStream_t s) {
+    const int V = load_width(x, C, false);
+#define TAB_QAUTO(VV, LL, FF) return launch_quantize_auto<BITS, VV, LL, FF>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, s)
+    if (C <= 8) {
+        if (V == 8) TAB_QAUTO(8, 1, false);
+        if (V == 4) TAB_QAUTO(4, 1, false);
+        if (V == 2) TAB_QAUTO(2, 1, false);
+        TAB_QAUTO(1, 1, false);
+    }
+    if (V == 8 && C % 64 == 0) TAB_QAUTO(8, 8, true);
+    if (V == 8) TAB_QAUTO(8, 8, false);
+    if (V == 4) TAB_QAUTO(4, 8, false);
+    if (V == 2) TAB_QAUTO(2, 8, false);
+    TAB_QAUTO(1, 8, false);
+#undef TAB_QAUTO
+}
+
+int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
+                           int N, int H, int W, int C, int* status, cudaStream_t stream) {
+    return bits == 2 ? quantize_auto_by_width<2>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream)
+                     : quantize_auto_by_width<1>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream);
 }
 
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream) {

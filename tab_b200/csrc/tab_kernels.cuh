@@ -66,12 +66,12 @@ struct QuantExtras {
     int wbits = 2, PC = 1, C = 64;       // of the weights
 };
 
-// quantize_sm100.cu: bits is 1 or 2; btn may be null; btn must already be zero.  in16: x holds int16 instead of float.
+// quantize_sm100.cu: bits is 1 or 2; btn may be null, else it receives the per-image counts (zeros for bits 1).  in16: x holds int16 instead of float.
 int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn, int bits,
                       int N, int H, int W, int C, cudaStream_t stream, const QuantExtras* extras = nullptr, bool in16 = false);
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream);
 // Thresholds scale * mean|x[n]| and the bit-planes against them in one launch (sums: N doubles, bar: two words, all zero
-// before and after); TAB_E_TOO_LARGE when the shape needs the separate launches.
+// before and after).
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
                            int N, int H, int W, int C, int* status, cudaStream_t stream);
 // Device word that records a bounded wait that ran out (shared with the tensor-core kernel); null if unavailable.

@@ -171,8 +171,7 @@ def new_state(N, device):
 
 def quantize_auto(X, scale, bitwidth, N, H, W, C, state=None):
     """``Quantize`` with the thresholds computed on the way: ``thresholds[n] = scale * mean|X[n]|``.  One launch (sums, a
-    grid-wide meeting point, quantisation) where C is a multiple of 64, else the three launches it replaces.  Returns
-    ``(QX, thresholds)``.  ``state``: a block from ``new_state(N, device)`` to reuse (zero before and after)."""
+    grid-wide meeting point, quantisation).  Returns ``(QX, thresholds)``.  ``state``: a block from ``new_state(N, device)`` to reuse (zero before and after)."""
     _check_input(X, "X", torch.float32)
     N, H, W, C = int(N), int(H), int(W), int(C)
     if X.numel() != N * H * W * C:

@@ -619,3 +619,57 @@ def test_error_behaviour(cuda):
     # after the rejected calls the device path still works
     yy = TAB.Conv2d(x, qw2, t, btn, 0, 1, 1, 1, 1, 1, 4, 4, 64, 4, 3, 3)
     assert not yy.any().item()
+
+
+# ------------------------------------------------------------------- quantisers: channel counts that fill no word, odd alignments
+
+@pytest.mark.parametrize("off", [0, 1, 2, 4])
+@pytest.mark.parametrize("C", [1, 2, 3, 4, 6, 8, 9, 12, 40, 64, 66, 72, 127, 196])
+def test_quantize_any_width_and_alignment(cuda, conv_path, C, off):
+    """Every load width (8, 4, 2, 1 elements by C and by the start of x), one and eight lanes per word, one and several
+    CTAs per image, special values; bit-planes and counts are compared exactly."""
+    if conv_path != "tensor":
+        pytest.skip("no convolution in this test")
+    for N, H, W in ((3, 5, 7), (2, 40, 31)):
+        x, ths = make_input(C + off, N, H, W, C)
+        x.reshape(-1)[: 5] = np.array([np.nan, np.inf, -np.inf, ths[0], -ths[0]], np.float32)[: x.size]
+        ths[-1] = -0.25                                                    # zeros of channel tails must not count as above it
+        buf = torch.empty(x.size + off, device=cuda)
+        buf[off:] = dev_t(x, cuda).reshape(-1)
+        for bw in (2, 1):
+            q, b = TAB.Quantize(buf[off:], dev_t(ths, cuda), bw, N, H, W, C)
+            qo, bo = O.quantize(x, ths, bw, N, H, W, C)
+            assert np.array_equal(q.cpu().numpy(), qo) and np.array_equal(b.cpu().numpy(), bo)
+
+
+@pytest.mark.parametrize("C", [3, 8, 40, 64, 66, 100, 127])
+@pytest.mark.parametrize("N,H,W", [(1, 3, 2), (5, 40, 31), (700, 3, 3)])
+def test_quantize_auto_any_channels(cuda, conv_path, N, H, W, C):
+    """Thresholds and bit-planes from one launch for every load width.  The thresholds are double sums rounded once to
+    float, so another order of summation gives the same float unless the sum sits within 1e-13 of a rounding boundary."""
+    if conv_path != "tensor":
+        pytest.skip("no convolution in this test")
+    from tab_b200 import ops
+    x, _ = make_input(C + N, N, H, W, C)
+    ths = (np.float64(np.float32(0.7)) * np.abs(x).reshape(N, -1).sum(axis=1, dtype=np.float64) / (H * W * C)).astype(np.float32)
+    state = ops.new_state(N, cuda)
+    for bw in (2, 1):
+        for _ in range(2):                                                 # the state block is left zero
+            q, t = ops.quantize_auto(dev_t(x, cuda), 0.7, bw, N, H, W, C, state)
+            assert np.array_equal(t.cpu().numpy(), ths)
+            qo, _b = O.quantize(x, ths, bw, N, H, W, C)
+            assert np.array_equal(q.cpu().numpy(), qo)
+    assert not state.cpu().numpy().any()
+
+
+@pytest.mark.parametrize("C", [5, 24, 65, 72])
+def test_quantize_i16_any_channels(cuda, conv_path, C):
+    if conv_path != "tensor":
+        pytest.skip("no convolution in this test")
+    from tab_b200 import ops
+    rng = np.random.default_rng(C)
+    x = rng.integers(-40, 41, size=(3, 9, 11, C)).astype(np.int16)
+    ths = np.array([3.0, 0.0, 17.5], np.float32)
+    for bw in (2, 1):
+        q = ops.quantize_i16(dev_t(x, cuda), dev_t(ths, cuda), bw, 3, 9, 11, C)
+        assert np.array_equal(q.cpu().numpy(), O.quantize(x.astype(np.float32), ths, bw, 3, 9, 11, C)[0])
