@@ -68,8 +68,8 @@ size_t tab_conv2d_workspace_bytes(int type, int p1, int p2, int s1, int s2,
 
 /*
  * Compute path of the convolution entry points, per calling thread (results are identical bit for bit):
- *   TAB_PATH_AUTO (default)   the bit-planes are expanded to int8 inside a persistent tcgen05 kernel (s8 MMA, exact);
- *                             shapes that kernel does not cover fall back to TAB_PATH_POPCOUNT
+ *   TAB_PATH_AUTO (default)   the bit-planes are expanded to 4-bit floats (or, with byte weights, to int8) inside a
+ *                             persistent tcgen05 kernel (exact); shapes that kernel does not cover fall back to TAB_PATH_POPCOUNT
  *   TAB_PATH_POPCOUNT         bit-packed LOP3/POPC kernel with a carry-save popcount tree - the reference's formulation
  *                             (TAB_GEMM.cu:25-147); this is also what tab_conv2d_packed_launch runs
  *   TAB_PATH_POPCOUNT_PLAIN   the same kernel with one POPC per word
@@ -79,14 +79,14 @@ enum { TAB_PATH_AUTO = 0, TAB_PATH_POPCOUNT = 1, TAB_PATH_POPCOUNT_PLAIN = 2 };
 int tab_conv2d_set_path(int path);
 /* Name and tile of the kernel the calling thread's most recent tensor-core convolution launched ("none" before the first, or
    when the last convolution ran the popcount kernel), e.g. "conv_umma_persist_kernel<1,256,4,0,2,0> grid 15x15 halves +next":
-   template arguments (row blocks per tile, filters per tile, ring stages, resident filters, fused epilogue, TMA epilogue,
-   ",pair" on clusters of two CTAs), the virtual grid per image, " halves" when the last round of tiles is worked as half-width
+   template arguments (row blocks per tile, most filters per tile, ring stages, resident filters, fused epilogue, TMA epilogue,
+   ",pair" on clusters of two CTAs, ",e2m1" on 4-bit operands), the virtual grid per image, " halves" when the last round of tiles is worked as half-width
    tiles, " +next" when the launch also quantises its result for the next layer.  Static storage per thread. */
 const char* tab_last_conv_kernel(void);
 /*
  * Every wait inside the tensor-core kernel and inside tab_quantize_auto_launch's kernel is bounded; a wait that ran out makes
  * the kernel record a code and return early, leaving its outputs incomplete.  This call synchronises the current device,
- * returns that code (0 = none; 11-17: a role of the tensor-core kernel gave up on an mbarrier; 21, 22: the grid-wide
+ * returns that code (0 = none; 11-18: a role of the tensor-core kernel gave up on an mbarrier; 21, 22: the grid-wide
  * meeting point of tab_conv2d_bits_next_launch / tab_quantize_auto_launch, which needs the launch's CTAs resident together -
  * other work occupying the device for tenths of a second can cause it) and clears it.  A non-zero code invalidates the
  * outputs of every launch on the device since the previous call.
@@ -101,7 +101,7 @@ int tab_device_status(void);
  * [KN][KH][KW][C] at bitwidth 2 for types 0,2 and bitwidth 1 for types 1,3.  btn (int32[KN]) is read
  * for type 2 only and may be NULL otherwise.  OH = (H + 2*p1 - KH + 1) / s1, OW likewise (integer
  * division, TAB_GEMM.cu:354-357).  y receives N*OH*OW*KN floats.  workspace must be 256-byte aligned.
- * Two launches: the quantiser (which also expands the weights to bytes) and the GEMM.  The first tensor-core call on a
+ * Two launches: the quantiser (which also expands the weights to nibbles) and the GEMM.  The first tensor-core call on a
  * device looks up a driver entry point and a device symbol: make it outside any stream capture.
  */
 int tab_conv2d_launch(const float* x, const int64_t* qw, const float* ths, const int32_t* btn,
@@ -186,6 +186,21 @@ int tab_conv2d_bits_i16_launch(const int64_t* qx, const int8_t* w8, int16_t* y16
                                void* state, float* next_ths, float next_scale, tab_stream_t stream);
 int tab_quantize_i16_launch(const int16_t* x, const float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C,
                             tab_stream_t stream);
+/*
+ * The GEMM stage on 4-bit weights: half the bytes of tab_expand_weights_launch's and twice the rate of the tensor cores (e2m1
+ * operands, fp32 accumulators that hold every sum exactly).  What tab_conv2d_launch runs; the byte form above stays for callers
+ * that keep byte weights.
+ *   tab_pack_weights_launch     tab_expand_weights_launch's bytes -> 32 bytes per 64-channel word, [KN][KH][KW][Cp/2], in the
+ *                               kernel's own channel order (opaque to the caller); both pointers 16-byte aligned
+ *   tab_conv2d_packed4_launch   tab_conv2d_bits_launch / _i16_launch / _next_launch in one entry point: y is float or, with
+ *                               y_is_int16, int16 (no residual then); residual, state with next_ths, and next_qx with
+ *                               next_bitwidth are optional as there.  TAB_E_TOO_LARGE also when KH*KW*C >= 2^24.
+ */
+int tab_pack_weights_launch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, tab_stream_t stream);
+int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int y_is_int16, int type, int p1, int p2, int s1, int s2,
+                              int N, int H, int W, int C, int KN, int KH, int KW,
+                              const float* residual, void* state, float* next_ths, float next_scale,
+                              int64_t* next_qx, int next_bitwidth, tab_stream_t stream);
 /*
  * Quantize with the thresholds every caller of the reference computes first, ths[n] = scale * mean|x[n]| (the notebook does it
  * with framework reductions before calling Quantize, TAB_GPU.cpp:53-58 takes them as an argument): one launch sums |x| per

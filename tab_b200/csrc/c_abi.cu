@@ -161,19 +161,20 @@ static int conv2d_impl(const float* x, const int64_t* qw, const float* ths, cons
         return TAB_E_ALIGNMENT;
     if ((long long)H * W >= (1LL << 31)) return TAB_E_TOO_LARGE;
     int64_t* qx = reinterpret_cast<int64_t*>(workspace);
-    int8_t* w8 = reinterpret_cast<int8_t*>(workspace) + bits_bytes(type, N, H, W, C);
-    unsigned* counter = reinterpret_cast<unsigned*>(w8 + w8_bytes(C, KN, KH, KW));
+    uint8_t* w4 = reinterpret_cast<uint8_t*>(workspace) + bits_bytes(type, N, H, W, C);
+    unsigned* counter = reinterpret_cast<unsigned*>(w4 + w8_bytes(C, KN, KH, KW));
     tc_forget_last_kernel();
     if (g_conv_path == TAB_PATH_AUTO && !misaligned(y, 15) && !misaligned(residual, 15)) {
         TcConvParams p = tc_geometry(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, oh, ow);
-        p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = w8; p.y = y; p.residual = residual; p.abs_sums = abs_sums;
+        p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = reinterpret_cast<const int8_t*>(w4); p.e2m1 = 1;
+        p.y = y; p.residual = residual; p.abs_sums = abs_sums;
         if (next_ths) { p.ths_out = next_ths; p.ths_scale = next_scale; p.done_counter = counter; }
         if (tc_conv_covers(p)) {
             // launch 1: quantise (TAB_GEMM.cu:419-426) + weight expansion + clears; launch 2: the GEMM
             QuantExtras ex;
             ex.zero_sums = abs_sums;
             ex.zero_counter = next_ths ? counter : nullptr;
-            ex.qw = reinterpret_cast<const uint64_t*>(qw); ex.w8 = w8;
+            ex.qw = reinterpret_cast<const uint64_t*>(qw); ex.w4 = w4;
             ex.words = (long long)KN * KH * KW * p.PC; ex.wbits = weight_bits(type); ex.PC = p.PC; ex.C = C;
             rc = quantize_dispatch(x, ths, qx, nullptr, act_bits(type), N, H, W, C, s, &ex);
             if (rc != TAB_OK) return rc;
@@ -228,12 +229,12 @@ int tab_expand_weights_launch(const int64_t* qw, int8_t* w8, int bitwidth, int K
 
 size_t tab_conv2d_state_bytes(int N) { return N < 0 ? 0 : round256((size_t)N * 8 + 16); }   // sums, completion counter, two grid-barrier words
 
-// Shared by the two GEMM-stage entry points: y (float) or y16 (int16) receives the result.
+// Shared by the GEMM-stage entry points: y (float) or y16 (int16) receives the result; e2m1: w8 points to 4-bit weights.
 // next_qx (optional, with next_ths): the result quantised at next_bits against next_ths, as tab_quantize_launch would write it.
 static int bits_impl(const int64_t* qx, const int8_t* w8, float* y, int16_t* y16, int type, int p1, int p2, int s1, int s2,
                      int N, int H, int W, int C, int KN, int KH, int KW,
                      const float* residual, void* state, float* next_ths, float next_scale, tab_stream_t stream,
-                     int64_t* next_qx = nullptr, int next_bits = 0) {
+                     int64_t* next_qx = nullptr, int next_bits = 0, bool e2m1 = false) {
     int rc = conv_args_ok(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW);
     if (rc != TAB_OK) return rc;
     const long long oh = ((long long)H + 2LL * p1 - KH + 1) / s1, ow = ((long long)W + 2LL * p2 - KW + 1) / s2;
@@ -253,7 +254,7 @@ static int bits_impl(const int64_t* qx, const int8_t* w8, float* y, int16_t* y16
         return TAB_E_ALIGNMENT;
     if (y16 && (long long)KH * KW * C > 32767) return TAB_E_TOO_LARGE;   // |y| <= KH*KW*C must fit 16 bits
     TcConvParams p = tc_geometry(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, oh, ow);
-    p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = w8; p.y = y; p.y16 = y16; p.residual = residual;
+    p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = w8; p.e2m1 = e2m1 ? 1 : 0; p.y = y; p.y16 = y16; p.residual = residual;
     if (next_ths) {
         p.abs_sums = reinterpret_cast<double*>(state);
         p.done_counter = reinterpret_cast<unsigned*>(reinterpret_cast<double*>(state) + N);
@@ -297,6 +298,23 @@ int tab_conv2d_bits_next_launch(const int64_t* qx, const int8_t* w8, void* y, in
     if (y_is_int16 && residual) return TAB_E_BAD_ARGUMENT;
     return bits_impl(qx, w8, y_is_int16 ? nullptr : static_cast<float*>(y), y_is_int16 ? static_cast<int16_t*>(y) : nullptr,
                      type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, residual, state, next_ths, next_scale, stream, next_qx, next_bitwidth);
+}
+
+int tab_pack_weights_launch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, tab_stream_t stream) {
+    if (KN < 0 || KH < 1 || KW < 1 || C < 1) return TAB_E_BAD_ARGUMENT;
+    if (KN == 0) return TAB_OK;
+    if (!w8 || !w4) return TAB_E_NULL_POINTER;
+    if (misaligned(w8, 15) || misaligned(w4, 15)) return TAB_E_ALIGNMENT;
+    return pack_weights_dispatch(w8, w4, KN, KH, KW, C, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int y_is_int16, int type, int p1, int p2, int s1, int s2,
+                              int N, int H, int W, int C, int KN, int KH, int KW,
+                              const float* residual, void* state, float* next_ths, float next_scale,
+                              int64_t* next_qx, int next_bitwidth, tab_stream_t stream) {
+    if (y_is_int16 && residual) return TAB_E_BAD_ARGUMENT;
+    return bits_impl(qx, reinterpret_cast<const int8_t*>(w4), y_is_int16 ? nullptr : static_cast<float*>(y), y_is_int16 ? static_cast<int16_t*>(y) : nullptr,
+                     type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, residual, state, next_ths, next_scale, stream, next_qx, next_bitwidth, true);
 }
 
 int tab_quantize_auto_launch(const float* x, float scale, void* state, float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C,

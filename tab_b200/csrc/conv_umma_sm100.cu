@@ -1,8 +1,9 @@
 // TAB convolution on the 5th-generation tensor cores: a persistent, warp-specialised implicit GEMM that reads the
-// activations as the bit-planes tab_quantize_launch writes (TAB_GEMM.cu:196-197) and multiplies them as int8.
+// activations as the bit-planes tab_quantize_launch writes (TAB_GEMM.cu:196-197) and multiplies them as 4-bit floats
+// (template argument E2M1; weights expanded by the call or by tab_pack_weights_launch) or as int8 (tab_expand_weights_launch).
 //
 // Replaces the reference's PadKernel, Img2RowKernel (TAB_GEMM.cuh:73-115) and TNN/TBN/BTN/BNNGEMM (TAB_GEMM.cu:25-147).
-// The quantised values {-1,0,+1} times {-1,0,+1} accumulate exactly in int32 (at most KH*KW*C terms), so y = sum a*w
+// The quantised values {-1,0,+1} times {-1,0,+1} accumulate exactly in int32 or fp32 (at most KH*KW*C terms, below 2^24 for fp32), so y = sum a*w
 // directly and none of the per-type corrections of the popcount formulas is needed: zero words of binary activations
 // decode to +1 (the reference's padding rule), channel tails decode to 0.
 //
@@ -49,8 +50,9 @@ __host__ __device__ constexpr int extra_warps(int fused, bool tepi, int tn) { re
 // Kernels that can work a tile as two halves of tn/2 filters (their filter boxes hold tn/2 filters): one row block, the
 // widest tile, streamed filters, transposing epilogue, single CTAs.
 __host__ __device__ constexpr bool split_capable(int mt, int tn, bool resident, bool tepi, bool pair) { return mt == 1 && tn == 256 && !resident && !tepi && !pair; }
-constexpr int NXT = 160;                                                   // expander threads: 5 warps, and a sixth (192) where the
-                                                                           // second MMA warp has nothing to issue (one row block per tile)
+// log2 of the taps whose words lie together in one 128-byte row of the filters: one or two words per tap, of the row's two
+// (bytes) or four (4-bit operands).
+__host__ __device__ constexpr int resident_taps_log2(int PC, bool e2m1) { return e2m1 ? (PC == 1 ? 2 : (PC == 2 ? 1 : 0)) : (PC == 1 ? 1 : 0); }
 constexpr int XUNROLL = 4;                                                 // (pixel, word) items a thread has in flight
 
 // Build-time diagnostic (-DTAB_PROF, never in the shipped library): cycles one representative warp of each role spends
@@ -254,13 +256,6 @@ __device__ __noinline__ void quantize_tail(const QuantTailArgs p, float* ths_sme
 }
 
 // ---- expander: bit-planes -> int8 patch rows ---------------------------------------------------------------------------
-// Four quantised values from the low four bits of a magnitude and a sign nibble: bytes 0x00 / 0x01 / 0xFF.
-__device__ __forceinline__ uint32_t expand4(uint32_t mnib, uint32_t snib) {
-    const uint32_t m01 = (mnib * 0x00204081u) & 0x01010101u;               // bit i -> byte i (the shifted copies do not overlap)
-    const uint32_t s01 = (snib * 0x00204081u) & 0x01010101u;
-    return m01 | (s01 * 0xFFu);
-}
-
 // The (sign, magnitude) words of XUNROLL items of a patch, held in registers between the loads and the expansion.
 // Nothing is computed on them before store_items: an instruction that consumes a loaded register would make the thread
 // wait for that load, and the point of loading a patch ahead is not to wait.
@@ -324,6 +319,59 @@ __device__ __forceinline__ void store_items(const TcConvParams& p, const RawItem
                 const uint32_t o2 = expand4((m16 >> 8) & 15u, (s16 >> 8) & 15u), o3 = expand4(m16 >> 12, s16 >> 12);
                 sts_v4(rowaddr + ((uint32_t)((4 * w + q) ^ (r & 7)) << 4), o0, o1, o2, o3);
             }
+        }
+    }
+}
+
+// ---- expander: bit-planes -> e2m1 patch rows ----------------------------------------------------------------------------
+// A patch row (128 bytes) holds four 64-channel words of 32 bytes.  Item = (row, two words): 32 bytes of planes in, 64 bytes
+// out, so that the arithmetic for the row's pixel is done once for two words.
+struct RawPair { uint64_t sg[2], mg[2]; };
+
+__device__ __forceinline__ void load_pair(const TcConvParams& p, RawPair& raw, int Rbase, int nrows, int cq, int pa, int pb, int it) {
+    const int nw = min(4, p.PC - 4 * cq);
+    const int two = nw > 2 ? 1 : 0;                                        // log2 of the row's items
+    raw.sg[0] = raw.sg[1] = 0;
+    raw.mg[0] = raw.mg[1] = p.abits == 1 ? ~0ull : 0ull;
+    const int r = it >> two;
+    if (r >= nrows) return;
+    const int w0 = (it & two) * 2;
+    const uint32_t R = (uint32_t)(Rbase + r);
+    const uint32_t n = p.dVHW.div(R);
+    const uint32_t rem = R - n * (uint32_t)(p.VH * p.VW);
+    const uint32_t i = p.dVW.div(rem);
+    const uint32_t j = rem - i * (uint32_t)p.VW;
+    const int ih = (int)i * p.s1 + pa - p.p1, iw = (int)j * p.s2 + pb - p.p2;
+    if ((int)n >= p.N || (unsigned)ih >= (unsigned)p.H || (unsigned)iw >= (unsigned)p.W) return;
+    const long long widx = (((long long)n * p.H + ih) * p.W + iw) * p.PC + 4 * cq + w0;
+    const bool second = w0 + 1 < nw;
+    if (p.abits == 2) {
+        const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p.qx + 2 * widx);
+        const ulonglong2 v = __ldg(q);
+        raw.sg[0] = v.x; raw.mg[0] = v.y;
+        if (second) { const ulonglong2 u = __ldg(q + 1); raw.sg[1] = u.x; raw.mg[1] = u.y; }
+    } else {
+        raw.sg[0] = __ldg(p.qx + widx);
+        if (second) raw.sg[1] = __ldg(p.qx + widx + 1);
+    }
+}
+__device__ __forceinline__ void store_pair(const TcConvParams& p, const RawPair& raw, uint32_t buf, int nrows, int cq, int it) {
+    const int nw = min(4, p.PC - 4 * cq);
+    const int two = nw > 2 ? 1 : 0;
+    const int r = it >> two;
+    if (r >= nrows) return;
+    const int w0 = (it & two) * 2;
+    const uint32_t rowaddr = buf + (uint32_t)r * IROW;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const int w = w0 + k;
+        if (w >= nw) break;
+        const int real = p.C - 64 * (4 * cq + w);                          // real channels in this word (>= 1)
+        const uint64_t mg = real >= 64 ? raw.mg[k] : raw.mg[k] & ((1ull << real) - 1ull), sg = raw.sg[k] & mg;
+#pragma unroll
+        for (int h = 0; h < 2; h++) {
+            const uint4 o = nibbles32((uint32_t)(mg >> (32 * h)), (uint32_t)(sg >> (32 * h)));
+            sts_v4(rowaddr + ((uint32_t)((2 * w + h) ^ (r & 7)) << 4), o.x, o.y, o.z, o.w);
         }
     }
 }
@@ -410,13 +458,73 @@ __device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const 
     }
 }
 
+// A 32x32 block of integers staged row by row (row r: 128 bytes, 16-byte chunks XOR-swizzled by r % 8), written out for filter
+// counts that are no multiple of four and for partial last blocks.  W columns per lane - 2 where rows start on even elements, else 1 - so that an
+// instruction writes W whole rows of the block, 32 * W consecutive elements of which are real: a lane writing its own row
+// instead (32 rows per instruction) took the L1 32 wavefronts for every store.
+template <int FUSED, int W, bool E2M1>
+__device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRows& sr, int nbase, int lane, uint32_t stage, double& dsum0, double& dsum1) {
+    constexpr int LPR = 32 / W, BATCH = 4;                                 // lanes per row; rows in flight per lane
+    constexpr bool has_res = FUSED == 2;
+    const int sub = lane / LPR, c = (lane % LPR) * W;
+    const bool col_ok = nbase + c < p.KN;
+#pragma unroll 1
+    for (int i0 = 0; i0 < LPR; i0 += BATCH) {
+        int m[BATCH];
+        float res[BATCH][W];
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) {
+            m[b] = __shfl_sync(0xFFFFFFFFu, sr.m_own, (i0 + b) * W + sub);
+            if (!col_ok) m[b] = -1;
+#pragma unroll
+            for (int k = 0; k < W; k++) res[b][k] = has_res && m[b] >= 0 ? __ldg(p.residual + (long long)m[b] * p.KN + nbase + c + k) : 0.f;
+        }
+#pragma unroll
+        for (int b = 0; b < BATCH; b++) {
+            const int r = (i0 + b) * W + sub;
+            const uint32_t at = stage + r * 128 + (((c >> 2) ^ (r & 7)) << 4) + (c & 3) * 4;
+            int raw[W];
+#pragma unroll
+            for (int k = 0; k < W; k++) raw[k] = lds_b32(at + 4 * k);
+            if (m[b] < 0) continue;
+            const long long e = (long long)m[b] * p.KN + nbase + c;
+            if (!has_res && p.y16 != nullptr) {
+                if (E2M1)
+#pragma unroll
+                    for (int k = 0; k < W; k++) raw[k] = __float_as_int(__int_as_float(raw[k]) + 12582912.f);   // low half: the integer
+                if (W == 2) *reinterpret_cast<uint32_t*>(p.y16 + e) = __byte_perm((uint32_t)raw[0], (uint32_t)raw[W - 1], 0x5410);
+                else p.y16[e] = (int16_t)raw[0];
+                continue;
+            }
+            float o[W];
+#pragma unroll
+            for (int k = 0; k < W; k++) o[k] = (E2M1 ? __int_as_float(raw[k]) + 0.f : (float)raw[k]) + res[b][k];
+            if (W == 2) *reinterpret_cast<float2*>(p.y + e) = make_float2(o[0], o[W - 1]);
+            else p.y[e] = o[0];
+            if (has_res && p.abs_sums != nullptr) {
+                double a = 0.0;
+#pragma unroll
+                for (int k = 0; k < W; k++) a += (double)fabsf(o[k]);
+                if (sr.fast) { if (r < sr.split) dsum0 += a; else dsum1 += a; }
+                else {
+                    const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
+                    if (img < p.N) atomicAdd(p.abs_sums + img, a);
+                }
+            }
+        }
+    }
+}
+
 // Columns [c0, c1) (multiples of 32, relative to the tile's first filter n0) of one 128-row accumulator block whose
 // TMEM address (column 0, this warp's lane quarter) is taddr.  The residual of a block is fetched one block ahead -
 // for the first block by the caller, before it waits for the accumulator (res / res_loaded) - because a load issued
 // when the block is processed costs the warp its whole DRAM latency.
-template <int FUSED>
+// down: the blocks are taken from the last to the first (the caller's residual is the last one's).  freed: barrier to arrive on
+// (once, lane 0) when the first block has been read out of tensor memory, 0 = none.
+// E2M1: the accumulators are floats (integer-valued) instead of integers.
+template <int FUSED, bool E2M1>
 __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t taddr, const SlabRows& sr, int n0, int c0, int c1,
-                                             int lane, uint32_t stage, float4 (&res)[8], bool res_loaded, PendingSums& ps) {
+                                             int lane, uint32_t stage, float4 (&res)[8], bool res_loaded, PendingSums& ps, bool down, uint32_t freed) {
     const bool vec4 = (p.KN & 3) == 0;
     const bool small_acc = p.Kw < (1 << 15);                               // |accumulator| <= 64 * Kw < 2^21: the bias conversion is exact
     constexpr bool has_res = FUSED == 2;
@@ -425,16 +533,42 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
     const int VHW = p.VH * p.VW;
     unsigned isum_own = 0;                                                 // integer data: |y| total of the lane's own row
     double dsum0 = 0.0, dsum1 = 0.0;                                       // float data: totals per image in the transposed domain
+    if (n0 + c1 > p.KN) c1 = max(c0, (p.KN - n0 + 31) / 32 * 32);          // blocks without a real filter are left out
+    if (E2M1 && freed != 0 && c0 >= c1 && lane == 0) mbar_arrive(freed);   // (this warp reads none)
+    const int cstride = down ? -32 : 32;
+    int cb = down ? c1 - 32 : c0;
 #pragma unroll 1
-    for (int cb = c0; cb < c1; cb += 32) {
+    for (int left = (c1 - c0) >> 5; left > 0; left--, cb += cstride) {
         const int nbase = n0 + cb;
-        if (nbase >= p.KN) break;                                          // uniform over the warp
         uint32_t v[32];
         tmem_ld32(taddr + (uint32_t)cb, v);
-        if (vec4 && nbase + 32 <= p.KN) {
+        if (E2M1 && freed != 0) {
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive(freed);
+            freed = 0;
+        }
+        const int real = p.KN - nbase;                                     // filters of this block that exist (the others' accumulators are 0)
+        if (vec4 && real >= 32) {
             // compact output whose rows start on 16-byte boundaries: the block is transposed as 16-bit values (half the
             // shared-memory traffic; on the 64-filter layers that traffic, next to the MMAs' operand reads, is the bound)
             const bool pack16 = !has_res && p.y16 != nullptr && (p.KN & 7) == 0;
+            if (E2M1 && !has_res && (sr.fast || p.y16 != nullptr)) {
+                // y is the accumulator itself.  |y| sums of the lane's own row: whole numbers below 2^23 add exactly in float
+                // (sr.fast bounds |y| by 2^18)
+                if (sr.fast) {
+                    float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        f0 += fabsf(__uint_as_float(v[j])); f1 += fabsf(__uint_as_float(v[j + 1]));
+                        f2 += fabsf(__uint_as_float(v[j + 2])); f3 += fabsf(__uint_as_float(v[j + 3]));
+                    }
+                    isum_own += sr.m_own >= 0 ? __float2uint_rn((f0 + f1) + (f2 + f3)) : 0u;
+                }
+                if (p.y16 != nullptr)                                      // the low 16 bits become the integer (|y| < 2^15)
+#pragma unroll
+                    for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + 12582912.f);
+            }
             if (pack16) {
 #pragma unroll
                 for (int q = 0; q < 4; q++)                                // row `lane`: 64 bytes, 16-byte chunk q at (q ^ (lane / 2 % 4))
@@ -445,7 +579,7 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                 for (int q = 0; q < 8; q++)
                     sts_v4(stage + lane * 128 + ((q ^ (lane & 7)) << 4), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             }
-            if (sr.fast && !has_res) {                                     // y is the accumulator itself: sum |acc| of the lane's own row
+            if (!E2M1 && sr.fast && !has_res) {                            // y is the accumulator itself: sum |acc| of the lane's own row
                 unsigned r0 = 0, r1 = 0, r2 = 0, r3 = 0;                   // (row `lane` of the slab), in integers, before the transposition;
 #pragma unroll                                                             // four independent |x| + acc chains (one SAD instruction each)
                 for (int j = 0; j < 32; j += 4) {
@@ -487,7 +621,13 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                             make_uint2(__byte_perm((uint32_t)raw.x, (uint32_t)raw.y, 0x5410), __byte_perm((uint32_t)raw.z, (uint32_t)raw.w, 0x5410));
                         if (sr.slow) {
                             const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
-                            if (img < p.N) atomicAdd(p.abs_sums + img, (double)abs(raw.x) + (double)abs(raw.y) + (double)abs(raw.z) + (double)abs(raw.w));
+                            if (img < p.N) {
+                                const int a4[4] = {raw.x, raw.y, raw.z, raw.w};
+                                double tot = 0.0;
+#pragma unroll
+                                for (int j = 0; j < 4; j++) tot += (double)(E2M1 ? abs((int)(int16_t)(a4[j] & 0xFFFF)) : abs(a4[j]));
+                                atomicAdd(p.abs_sums + img, tot);
+                            }
                         }
                     }
                 }
@@ -499,7 +639,10 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
             for (int i = 0; i < 8; i++) {
                 const int r = 4 * i + rsub;
                 const int4 raw = lds_v4(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
-                if (small_acc) {                                           // int -> float by the 1.5 * 2^23 bias, no I2F
+                if (E2M1) {                                                // + 0: a sum of products of zeros may be -0
+                    o[i].x = __int_as_float(raw.x) + 0.f; o[i].y = __int_as_float(raw.y) + 0.f;
+                    o[i].z = __int_as_float(raw.z) + 0.f; o[i].w = __int_as_float(raw.w) + 0.f;
+                } else if (small_acc) {                                    // int -> float by the 1.5 * 2^23 bias, no I2F
                     o[i].x = __int_as_float(raw.x + 0x4B400000) - 12582912.f; o[i].y = __int_as_float(raw.y + 0x4B400000) - 12582912.f;
                     o[i].z = __int_as_float(raw.z + 0x4B400000) - 12582912.f; o[i].w = __int_as_float(raw.w + 0x4B400000) - 12582912.f;
                 } else {
@@ -510,8 +653,8 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
 #pragma unroll
                 for (int i = 0; i < 8; i++) { o[i].x += res[i].x; o[i].y += res[i].y; o[i].z += res[i].z; o[i].w += res[i].w; }
                 // the next block's residual, in flight while this block is stored and summed
-                res_loaded = vec4 && cb + 32 < c1 && nbase + 64 <= p.KN;
-                if (res_loaded) slab_load_residual(p, sr, nbase + 32, lane, res);
+                res_loaded = left > 1 && nbase + cstride + 32 <= p.KN;
+                if (res_loaded) slab_load_residual(p, sr, nbase + cstride, lane, res);
             }
 #pragma unroll
             for (int i = 0; i < 8; i++)
@@ -541,24 +684,25 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                 }
             }
             __syncwarp();
-        } else {
+        } else {                                                           // KN is no multiple of four, or a partial last block
             res_loaded = false;
-            if (sr.m_own >= 0) {                                           // ragged right edge / odd filter counts: a row per lane
-                float* yrow = p.y + (long long)sr.m_own * p.KN;
-                const float* rrow = has_res ? p.residual + (long long)sr.m_own * p.KN : nullptr;
-                double rsum = 0.0;
 #pragma unroll
-                for (int i = 0; i < 32; i++) {
-                    if (nbase + i < p.KN) {
-                        float ov = (float)(int)v[i];
-                        if (rrow) ov += __ldg(rrow + nbase + i);
-                        if (!has_res && p.y16 != nullptr) p.y16[(long long)sr.m_own * p.KN + nbase + i] = (int16_t)(int)v[i];
-                        else yrow[nbase + i] = ov;
-                        if (FUSED) rsum += (double)fabsf(ov);
-                    }
+            for (int q = 0; q < 8; q++)
+                sts_v4(stage + lane * 128 + ((q ^ (lane & 7)) << 4), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
+            if (!has_res && want_sum && sr.m_own >= 0) {
+                unsigned r0 = 0, r1 = 0;
+#pragma unroll
+                for (int j = 0; j < 32; j += 2) {
+                    r0 = __sad(E2M1 ? __float2int_rn(__uint_as_float(v[j])) : (int)v[j], 0, r0);
+                    r1 = __sad(E2M1 ? __float2int_rn(__uint_as_float(v[j + 1])) : (int)v[j + 1], 0, r1);
                 }
-                if (want_sum && sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, rsum);
+                if (sr.fast) isum_own += r0 + r1;
+                else if (sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, (double)r0 + (double)r1);
             }
+            __syncwarp();
+            if (p.KN & 1) ragged_block<FUSED, 1, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
+            else ragged_block<FUSED, 2, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
+            __syncwarp();
         }
     }
     if (sr.fast) {
@@ -637,16 +781,28 @@ __device__ __forceinline__ void tepi_request_residual(const void* tmR, const Tep
 // stages the patch of its own 128 rows and fetches TNI/2 filters of every slice; the even CTA's MMA warp issues the pair's
 // MMAs and its commits arrive on the "empty" / "accumulator full" barriers of both CTAs, while the "full" / "accumulator
 // empty" barriers it waits on live in the even CTA and collect the arrivals of both.
-template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false>
+// E2M1 measured (B200, us, GPU time of the whole call, bytes / 4-bit): 1x1 25088x1024x1024 96 / 58, 3x3 16x112x112x256->64 90 / 73, prepared
+// 3x3 64x14x14x256->256 20.6 / 17.7, ResNet-18-shaped network at batch 256 1201 / 1133.  What bounds it then is no longer the
+// tensor pipe: expanders and load latency (1x1), the epilogue's stores (64 filters), the filter slices from the L2 (256 filters).
+// E2M1: 4-bit operands (see umma_e2m1), twice the channels per operand byte and per instruction: a row holds four words
+// instead of two, a ring stage up to 256 channels of a tap, and with one or two words per pixel several taps.  The 16
+// columns of scales do not fit beside two 256-column accumulators: those overlap by 16 columns, which the epilogue reads
+// first, and the next tile's MMAs wait for that ("freed") instead of only for the tile before last.
+template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false, bool E2M1 = false>
 __global__ void __launch_bounds__(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI), 1)
 conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
                          const TcConvParams p, int* __restrict__ status,
-                         const int prow, const int nrows, const int nst, const int tiles_m, const int tiles_n, const int split_from) {
+                         const int prow, const int nrows, const int nst, const int tiles_m, const int tiles_n, const int split_from, const int tnw) {
     static_assert(!PAIR || (MT == 1 && !BRES && !TEPI), "CTA pairs: one row block per CTA, streamed filters, transposing epilogue");
     constexpr bool SPLIT = split_capable(MT, TNI, BRES, TEPI, PAIR);
-    constexpr int BROWS = PAIR ? TNI / 2 : TNI;                            // filters of a slice this CTA holds
-    constexpr int BSTAGE = BROWS * IROW;
+    const int brows = PAIR ? tnw / 2 : tnw;                                // filters of a slice this CTA holds
+    const int bstage = brows * IROW;
     constexpr int ACOLS = MT * TNI;                                        // columns of one accumulator buffer
+    constexpr int WPR = E2M1 ? 4 : 2, WBYTES = E2M1 ? 32 : 64;             // 64-channel words per operand row, bytes of a word
+    constexpr int ABUF = E2M1 && ACOLS == 256 ? 240 : ACOLS;               // columns between the two accumulator buffers
+    constexpr int SFCOL = ABUF + ACOLS;                                    // E2M1: 16 columns of scales behind them
+    constexpr int TCOLS = !E2M1 ? 2 * ACOLS : (SFCOL + 16 <= 256 ? 256 : 512);
+    static_assert(!E2M1 || !PAIR, "CTA pairs multiply bytes");
     constexpr int NXW = 5 + extra_warps(FUSED, TEPI, TNI) + (MT == 1 ? 1 : 0);   // expander warps: 0, 12 and up, and warp 3 when it has no MMAs to issue
     constexpr int NX = 32 * NXW;
     static_assert(2 * ACOLS <= 512, "two accumulator buffers must fit the 512 TMEM columns");
@@ -656,13 +812,14 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     const uint32_t sbase = (raw + 1023u) & ~1023u;
     unsigned char* smem = smem_raw + (sbase - raw);
     const uint32_t sPatch = sbase;                                         // [2][prow][128 B], prow % 8 == 0
-    const uint32_t sRing = sbase + 2 * prow * IROW;                        // [nst][TNI][128 B]
-    const int tail = 2 * prow * IROW + nst * BSTAGE;
+    const uint32_t sRing = sbase + 2 * prow * IROW;                        // [nst][brows][128 B]
+    const int tail = 2 * prow * IROW + nst * bstage;
     const uint32_t fullB = sbase + tail, emptyB = fullB + 64;              // [8] each
     const uint32_t fullP = emptyB + 64, emptyP = fullP + 16, accFull = emptyP + 16, accEmpty = accFull + 16;
     const uint32_t tslot = accEmpty + 16;                                  // = fullB + 192
     volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(smem + tail + 192);
     volatile int* deadp = reinterpret_cast<volatile int*>(smem + tail + 200);     // set by a role whose bounded wait ran out
+    const uint32_t accFreed = fullB + 208;                                 // E2M1: the columns both accumulators share have been read
     const uint32_t resB = sbase + tail + 256;                              // [8 epilogue warps][2]: residual arrived (TEPI)
     const uint32_t sStage = sbase + tail + 1024;                           // [8 epilogue warps][4 KB, or 2 x 4 KB with TEPI]; 1024-byte aligned
 
@@ -671,7 +828,10 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     const int s1 = p.s1, s2 = p.s2;
     const bool UNIT = s1 == 1 && s2 == 1;                                  // one plane: flat tap loops
     const int PA = p.PA, PB = p.PB, VW = p.VW;
-    const int T = p.KH * p.KW, ncp = (p.PC + 1) >> 1;
+    const int T = p.KH * p.KW, ncp = (p.PC + WPR - 1) / WPR;
+    const int tlog = resident_taps_log2(p.PC, E2M1);                       // 2^tlog taps have their words in one 128-byte filter row
+    const int tpst = UNIT ? 1 << tlog : 1;                                 // taps per ring stage (planes take their taps one by one)
+    const bool overlap = ABUF != ACOLS && MT * tnw > ABUF;                 // the accumulators in use reach into each other
     // SPLIT: the tiles from split_from on (the last, partly filled round of the grid) are worked as two halves of TNI/2
     // filters each, numbered after the whole tiles: twice as many CTAs share the round and it takes about half as long.
     const int sfrom = SPLIT ? split_from : tiles_m * tiles_n;
@@ -692,15 +852,22 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         mbar_init(emptyP, MT); mbar_init(emptyP + 8, MT);
         mbar_init(accFull, MT); mbar_init(accFull + 8, MT);
         mbar_init(accEmpty, PAIR ? 16 : 8); mbar_init(accEmpty + 8, PAIR ? 16 : 8);   // one arrival per epilogue warp (of both CTAs)
+        if (E2M1) mbar_init(accFreed, 4);                                  // one arrival per warp that reads them
         if (TEPI) for (int i = 0; i < 16; i++) mbar_init(resB + 8 * i, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == 1) { if (PAIR) tmem_alloc_pair(tslot, (uint32_t)(2 * ACOLS)); else tmem_alloc(tslot, (uint32_t)(2 * ACOLS)); }
+    if (warp == 1) { if (PAIR) tmem_alloc_pair(tslot, (uint32_t)TCOLS); else tmem_alloc(tslot, (uint32_t)TCOLS); }
     tc_fence_before();
     __syncthreads();
     if (PAIR) cluster_sync_all();                                          // both CTAs' barriers exist before either arrives on the other's
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    if (E2M1) {                                                            // scales 2^0 in all lanes
+        if (warp >= 4 && warp < 8) tmem_fill16(tmem_base + SFCOL + ((uint32_t)((warp & 3) * 32) << 16), 0x7F7F7F7Fu);
+        tc_fence_before();
+        __syncthreads();
+        tc_fence_after();
+    }
     // Programmatic launch: the set-up above overlapped the tail of the previous kernel (the quantiser); from here on its
     // output is read.  The next kernel may be scheduled when every CTA has finished its tiles (not earlier: a grid
     // waiting in griddepcontrol.wait was measured to slow the MMA warp of the tiles still running).
@@ -721,6 +888,50 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         PatchIter cur = {cta0, 0, 0};
         unsigned q = 0;
         bool dead = false;
+        if constexpr (E2M1) {
+            // The patches as one sequence of chunks of one item per thread.  Three chunks are loaded ahead, in registers that
+            // are named and not rotated: a move of a register whose load is in flight would wait for it.
+            struct At { int t, cp, pl, base; };
+            auto items_of = [&](int cp) { return nrows << (p.PC - 4 * cp > 2 ? 1 : 0); };
+            auto advance = [&](At& a) {
+                a.base += NX;
+                if (a.base >= items_of(a.cp)) {
+                    a.base = 0;
+                    if (++a.pl == planes) { a.pl = 0; if (++a.cp == ncp) { a.cp = 0; a.t += step; } }
+                }
+            };
+            auto fetch = [&](RawPair& into, At& a) {
+                if (a.t >= ntiles) return;
+                const int pa = UNIT ? 0 : a.pl / PB;
+                load_pair(p, into, tile_row0(a.t), nrows, a.cp, pa, UNIT ? 0 : a.pl - pa * PB, a.base + xt);
+                advance(a);
+            };
+            At at = {cta0, 0, 0, 0}, ahead = at;
+            auto stage = [&](const RawPair& mine) -> bool {
+                if (at.t >= ntiles || dead) return false;
+                const unsigned pb = q & 1;
+                if (at.base == 0 && q >= 2 && !mbar_wait_prof<0>(prof_on, emptyP + 8 * pb, ((q >> 1) - 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 11); *deadp = 1; } return false; }
+                PROF_T0;
+                store_pair(p, mine, sPatch + (uint32_t)(pb * prow) * IROW, nrows, at.cp, at.base + xt);
+                const bool last = at.base + NX >= items_of(at.cp);
+                advance(at);
+                if (last) {
+                    fence_async_smem();
+                    mbar_arrive(fullP + 8 * pb);
+                    q++;
+                }
+                PROF_ADD(1, prof_on);
+                return true;
+            };
+            RawPair r0, r1, r2, r3;
+            fetch(r0, ahead); fetch(r1, ahead); fetch(r2, ahead);
+            for (;;) {
+                fetch(r3, ahead); if (!stage(r0)) break;
+                fetch(r0, ahead); if (!stage(r1)) break;
+                fetch(r1, ahead); if (!stage(r2)) break;
+                fetch(r2, ahead); if (!stage(r3)) break;
+            }
+        } else {
         // One patch: wait for its buffer, expand the words loaded earlier (mine), hand the patch to the MMA warp.
         auto stage_patch = [&](const RawItems& mine) {
             const unsigned pb = q & 1;
@@ -760,19 +971,19 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             raw = ahead;
             cur = nxt;
         }
+        }
     } else if (warp == 2) {
         // ---- filter producer ---------------------------------------------------------------------------------------------
         if (BRES) {
             if (elect_one()) {
-                mbar_expect_tx(fullB, (uint32_t)(nst * BSTAGE));
-                if (p.PC == 1) {
-                    // one 64-byte word per tap: a 128-byte-wide slot holds taps 2j and 2j + 1 (the box of the last slot of
-                    // an odd tap count ends beyond the row and is zero-filled there)
-                    for (int j = 0; j < nst; j++) tma_load_2d(sRing + j * BSTAGE, &tmB, j * 128, 0, fullB);
+                mbar_expect_tx(fullB, (uint32_t)(nst * bstage));
+                if (tlog > 0) {
+                    // 2^tlog taps share a 128-byte-wide slot (the box of the last slot may end beyond the row and is zero-filled there)
+                    for (int j = 0; j < nst; j++) tma_load_2d(sRing + j * bstage, &tmB, j * 128, 0, fullB);
                 } else {
                     for (int cp = 0; cp < ncp; cp++)
                         for (int tap = 0; tap < T; tap++)
-                            tma_load_2d(sRing + (cp * T + tap) * BSTAGE, &tmB, (tap * p.PC + 2 * cp) * 64, 0, fullB);
+                            tma_load_2d(sRing + (cp * T + tap) * bstage, &tmB, (tap * p.PC + WPR * cp) * WBYTES, 0, fullB);
                 }
             }
             __syncwarp();
@@ -783,8 +994,22 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             (void)prof_on;
             for (int t = cta0; t < ntiles && !dead; t += cstep) {
                 const int hf = half_of(t);
-                const int n0 = (tile_of(t) % tiles_n) * TNI + (PAIR ? (int)crank * BROWS : 0) + (hf == 2 ? TNI / 2 : 0);
+                const int n0 = (tile_of(t) % tiles_n) * tnw + (PAIR ? (int)crank * brows : 0) + (hf == 2 ? tnw / 2 : 0);
                 for (int cp = 0; cp < ncp && !dead; cp++) {
+                    if (E2M1 && UNIT) {                                    // tpst taps per stage
+                        for (int tap = 0; tap < T; tap += tpst, g++) {
+                            const unsigned slot = g % SB;
+                            if (g >= (unsigned)SB && !mbar_wait_prof<2>(prof_on, emptyB + 8 * slot, ((g / SB) - 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 12); *deadp = 1; } break; }
+                            if (elect_one()) {
+                                const int kx = (tap * p.PC + WPR * cp) * WBYTES;
+                                mbar_expect_tx(fullB + 8 * slot, (uint32_t)(SPLIT && hf ? bstage / 2 : bstage));
+                                tma_load_2d(sRing + slot * bstage, &tmB, kx, n0, fullB + 8 * slot);
+                                if (SPLIT && !hf) tma_load_2d(sRing + slot * bstage + bstage / 2, &tmB, kx, n0 + tnw / 2, fullB + 8 * slot);
+                            }
+                            __syncwarp();
+                        }
+                        continue;
+                    }
                     // same tap order as the MMA warp: plane by plane
                     for (int pa = 0; pa < PA && !dead; pa++)
                     for (int pbb = 0; pbb < PB && !dead; pbb++)
@@ -794,16 +1019,16 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                         if (g >= (unsigned)SB && !mbar_wait_prof<2, PAIR>(prof_on, emptyB + 8 * slot, ((g / SB) - 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 12); *deadp = 1; } break; }
                         if (elect_one()) {
                             if (PAIR) {                                    // both halves are counted on the even CTA's barrier
-                                if (crank == 0) mbar_expect_tx(fullB + 8 * slot, 2u * (uint32_t)BSTAGE);
-                                tma_load_2d_pair(sRing + slot * BSTAGE, &tmB, ((kh * p.KW + kw) * p.PC + 2 * cp) * 64, n0, fullB + 8 * slot);
-                            } else if (SPLIT) {                            // boxes of TNI/2 filters: two for a whole tile
-                                const int kx = ((kh * p.KW + kw) * p.PC + 2 * cp) * 64;
-                                mbar_expect_tx(fullB + 8 * slot, (uint32_t)(hf ? BSTAGE / 2 : BSTAGE));
-                                tma_load_2d(sRing + slot * BSTAGE, &tmB, kx, n0, fullB + 8 * slot);
-                                if (!hf) tma_load_2d(sRing + slot * BSTAGE + BSTAGE / 2, &tmB, kx, n0 + TNI / 2, fullB + 8 * slot);
+                                if (crank == 0) mbar_expect_tx(fullB + 8 * slot, 2u * (uint32_t)bstage);
+                                tma_load_2d_pair(sRing + slot * bstage, &tmB, ((kh * p.KW + kw) * p.PC + WPR * cp) * WBYTES, n0, fullB + 8 * slot);
+                            } else if (SPLIT) {                            // boxes of tnw/2 filters: two for a whole tile
+                                const int kx = ((kh * p.KW + kw) * p.PC + WPR * cp) * WBYTES;
+                                mbar_expect_tx(fullB + 8 * slot, (uint32_t)(hf ? bstage / 2 : bstage));
+                                tma_load_2d(sRing + slot * bstage, &tmB, kx, n0, fullB + 8 * slot);
+                                if (!hf) tma_load_2d(sRing + slot * bstage + bstage / 2, &tmB, kx, n0 + tnw / 2, fullB + 8 * slot);
                             } else {
-                                mbar_expect_tx(fullB + 8 * slot, (uint32_t)BSTAGE);
-                                tma_load_2d(sRing + slot * BSTAGE, &tmB, ((kh * p.KW + kw) * p.PC + 2 * cp) * 64, n0, fullB + 8 * slot);
+                                mbar_expect_tx(fullB + 8 * slot, (uint32_t)bstage);
+                                tma_load_2d(sRing + slot * bstage, &tmB, ((kh * p.KW + kw) * p.PC + WPR * cp) * WBYTES, n0, fullB + 8 * slot);
                             }
                         }
                         __syncwarp();
@@ -818,7 +1043,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         //      accumulators, the same operands and the same barrier phases (both warps follow every stage, so a parity
         //      wait never sees a phase other than the current or the previous one); the "empty" and "accumulator full"
         //      barriers then count one commit from each.  With one row block warp 3 idles. -----------------------------------
-        constexpr uint32_t IDESC = PAIR ? umma_idesc_pair(TNI) : umma_idesc(TNI);
+        const uint32_t whole = E2M1 ? umma_idesc_e2m1(tnw, UTM) : (PAIR ? umma_idesc_pair(tnw) : umma_idesc(tnw));
         constexpr uint32_t MB_UNITS = (UTM * IROW) >> 4;                   // next 128-row block of the patch, in 16-byte units
         const int mw = warp == 1 ? 0 : 1;
         const bool prof_on = warp == 1 && lane == 0;
@@ -830,34 +1055,35 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         if (BRES && !dead && !mbar_wait_prof<5, PAIR>(prof_on, fullB, 0)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 15); *deadp = 1; } }
         // descriptor address of the resident filter slice of (channel pair, tap); with one channel word two taps share a slot
         auto resident_b = [&](int cp, int tap) -> uint32_t {
-            return p.PC == 1 ? ((sRing + (uint32_t)(tap >> 1) * BSTAGE) >> 4) + (uint32_t)(tap & 1) * 4u
-                             : (sRing + (uint32_t)(cp * T + tap) * BSTAGE) >> 4;
+            if (tlog == 0) return (sRing + (uint32_t)(cp * T + tap) * bstage) >> 4;
+            return ((sRing + (uint32_t)(tap >> tlog) * bstage) >> 4) + (uint32_t)(tap & ((1 << tlog) - 1)) * (uint32_t)(p.PC * WBYTES / 16);
         };
-        uint32_t idesc = IDESC;
+        uint32_t idesc = whole;
         auto mma = [&](uint32_t d, uint64_t da, uint64_t db, uint32_t acc_flag) {
-            if (PAIR) umma_i8_pair(d, da, db, IDESC, acc_flag); else umma_i8(d, da, db, SPLIT ? idesc : IDESC, acc_flag);
+            if (E2M1) umma_e2m1(d, da, db, SPLIT ? idesc : whole, tmem_base + SFCOL, acc_flag);
+            else if (PAIR) umma_i8_pair(d, da, db, whole, acc_flag); else umma_i8(d, da, db, SPLIT ? idesc : whole, acc_flag);
         };
         auto commit = [&](uint32_t bar) { if (PAIR) umma_commit_pair(bar); else umma_commit(bar); };
         for (int t = cta0; t < ntiles && !dead; t += cstep, a++) {
             const unsigned buf = a & 1;
             if (a >= 2 && !mbar_wait_prof<3, PAIR>(prof_on, accEmpty + 8 * buf, ((a >> 1) - 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 13); *deadp = 1; } break; }
+            if (E2M1 && overlap && a >= 1 && !mbar_wait_prof<3>(prof_on, accFreed, (a - 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 18); *deadp = 1; } break; }
             tc_fence_after();
-            const uint32_t acc = tmem_base + buf * ACOLS;
-            if (SPLIT) idesc = half_of(t) ? umma_idesc(TNI / 2) : IDESC;
+            const uint32_t acc = tmem_base + buf * ABUF;
+            if (SPLIT) idesc = half_of(t) ? (E2M1 ? umma_idesc_e2m1(tnw / 2, UTM) : umma_idesc(tnw / 2)) : whole;
             uint32_t accumulate = 0;                                       // 0 for the tile's first MMAs
             for (int cp = 0; cp < ncp && !dead; cp++) {
-                const bool four = 2 * cp + 1 < p.PC;                       // both 64-channel words of the pair exist
-                // the MMAs of one tap: 2 or 4 K steps of 32 bytes, MT row blocks each
+                constexpr int KSTEP = E2M1 ? 64 : 32;                      // channels per instruction
+                const int ks = (min(p.C - 4 * KSTEP * cp, 4 * KSTEP) + KSTEP - 1) / KSTEP;      // K steps that hold real channels
+                // the MMAs of one tap: up to 4 K steps of 32 bytes, MT row blocks each
                 auto issue_tap = [&](uint64_t da, uint64_t db, uint32_t acc_first) {
                     for (int mb = mb_lo; mb < mb_hi; mb++) {
                         const uint32_t d = acc + mb * TNI;
                         const uint64_t dam = da + mb * MB_UNITS;
                         mma(d, dam, db, acc_first);
-                        mma(d, dam + 2, db + 2, 1u);
-                        if (four) {
-                            mma(d, dam + 4, db + 4, 1u);
-                            mma(d, dam + 6, db + 6, 1u);
-                        }
+                        if (ks > 1) mma(d, dam + 2, db + 2, 1u);
+                        if (ks > 2) mma(d, dam + 4, db + 4, 1u);
+                        if (ks > 3) mma(d, dam + 6, db + 6, 1u);
                     }
                 };
                 if (UNIT) {
@@ -877,6 +1103,28 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                             if (cp == ncp - 1) commit(accFull + 8 * buf);
                         }
                         __syncwarp();
+                    } else if (E2M1) {
+                        for (int tap = 0; tap < T; g++) {
+                            const unsigned slot = g % SB;
+                            if (!mbar_wait_prof<5>(prof_on, fullB + 8 * slot, (g / SB) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 15); *deadp = 1; } break; }
+                            tc_fence_after();
+                            const int tend = min(tap + tpst, T);
+                            const bool issuer = elect_one();
+                            uint32_t b = (sRing + slot * bstage) >> 4;
+                            for (; tap < tend; tap++, b += (uint32_t)(p.PC * WBYTES / 16)) {
+                                if (issuer) issue_tap(((uint64_t)UMMA_DESC_HI << 32) | (arow + (uint32_t)kw * (IROW >> 4)),
+                                                      ((uint64_t)UMMA_DESC_HI << 32) | b, (cp > 0 || tap > 0) ? 1u : 0u);
+                                if (++kw == p.KW) { kw = 0; arow += (uint32_t)VW * (IROW >> 4); }
+                            }
+                            if (issuer) {
+                                commit(emptyB + 8 * slot);
+                                if (tend == T) {
+                                    commit(emptyP + 8 * pb);
+                                    if (cp == ncp - 1) commit(accFull + 8 * buf);
+                                }
+                            }
+                            __syncwarp();
+                        }
                     } else {
                         for (int tap = 0; tap < T; tap++, g++) {
                             const unsigned slot = g % SB;
@@ -884,7 +1132,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                             tc_fence_after();
                             if (elect_one()) {
                                 issue_tap(((uint64_t)UMMA_DESC_HI << 32) | (arow + (uint32_t)kw * (IROW >> 4)),
-                                          ((uint64_t)UMMA_DESC_HI << 32) | ((sRing + slot * BSTAGE) >> 4), (cp > 0 || tap > 0) ? 1u : 0u);
+                                          ((uint64_t)UMMA_DESC_HI << 32) | ((sRing + slot * bstage) >> 4), (cp > 0 || tap > 0) ? 1u : 0u);
                                 commit(emptyB + 8 * slot);
                                 if (tap == T - 1) {
                                     commit(emptyP + 8 * pb);
@@ -912,7 +1160,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                             const unsigned slot = g % SB;
                             if (!mbar_wait_prof<5, PAIR>(prof_on, fullB + 8 * slot, (g / SB) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 15); *deadp = 1; } break; }
                             tc_fence_after();
-                            bsm = sRing + slot * BSTAGE;
+                            bsm = sRing + slot * bstage;
                         }
                         if (elect_one()) {
                             issue_tap(((uint64_t)UMMA_DESC_HI << 32) | (patch + (uint32_t)(ih * VW + iw) * (IROW >> 4)),
@@ -938,7 +1186,8 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         (void)prof_on;
         const uint32_t sbuf = sStage + (uint32_t)ew * 8192u;               // two 4 KB block buffers
         const uint32_t mres = resB + 16u * (uint32_t)ew;                   // their "residual arrived" barriers
-        const int emb = MT == 2 ? wg : 0, ec0 = MT == 2 ? 0 : wg * (TNI / 2), ec1 = MT == 2 ? TNI : (wg + 1) * (TNI / 2);
+        const int emb = MT == 2 ? wg : 0, chalf = (tnw / 32 + 1) / 2 * 32;  // columns of the first of two warps that share a row block
+        const int ec0 = MT == 2 || wg == 0 ? 0 : chalf, ec1 = MT == 2 || wg == 1 ? tnw : chalf;
         constexpr bool has_res = FUSED == 2;
         const bool want_sum = FUSED && p.abs_sums != nullptr;
         const bool small_acc = p.Kw < (1 << 15);                           // |accumulator| <= 64 * Kw < 2^21: the bias conversion is exact
@@ -949,12 +1198,12 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         PendingSums pending;
         if (has_res && lane == 0) {                                        // the residual of the warp's first block
             TepiIter first = {cta0, ec0};
-            first.settle(ec0, step, ntiles, tiles_n, TNI, p.KN);
-            if (first.t < ntiles) tepi_request_residual(&tmR, tepi_box(p, slab_row(first.t), (first.t % tiles_n) * TNI + first.cb), sbuf, mres);
+            first.settle(ec0, step, ntiles, tiles_n, tnw, p.KN);
+            if (first.t < ntiles) tepi_request_residual(&tmR, tepi_box(p, slab_row(first.t), (first.t % tiles_n) * tnw + first.cb), sbuf, mres);
         }
         for (int t = cta0; t < ntiles && !dead; t += step, a++) {
             const unsigned buf = a & 1;
-            const int n0 = (t % tiles_n) * TNI, Rw = slab_row(t);
+            const int n0 = (t % tiles_n) * tnw, Rw = slab_row(t);
             // the lane's own row, for the |y| sums: lanes of image wimg0 and of wimg0 + 1 are totalled separately ("fast":
             // the slab touches at most two images and row totals stay below 2^26), else every lane adds its own total
             const uint32_t R = (uint32_t)(Rw + lane);
@@ -969,7 +1218,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             //  what bounds this epilogue, and the prefetches were half as many requests again - 5 % of the launch.)
             if (!mbar_wait_prof<6>(prof_on, accFull + 8 * buf, (a >> 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 16); *deadp = 1; } break; }
             tc_fence_after();
-            const uint32_t taddr = tmem_base + buf * ACOLS + (uint32_t)(emb * TNI) + ((uint32_t)((warp & 3) * 32) << 16);
+            const uint32_t taddr = tmem_base + buf * ABUF + (uint32_t)(emb * TNI) + ((uint32_t)((warp & 3) * 32) << 16);
 #pragma unroll 1
             for (int cb = ec0; cb < ec1 && n0 + cb < p.KN; cb += 32, blk++) {
                 const unsigned k = blk & 1;
@@ -983,9 +1232,9 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                         // the other buffer's last store must have finished reading it before the next residual lands there
                         bulk_wait_read<0>();
                         TepiIter nx = {t, cb};
-                        nx.next(ec0, ec1, step, ntiles, tiles_n, TNI, p.KN);
+                        nx.next(ec0, ec1, step, ntiles, tiles_n, tnw, p.KN);
                         if (nx.t < ntiles)
-                            tepi_request_residual(&tmR, tepi_box(p, slab_row(nx.t), (nx.t % tiles_n) * TNI + nx.cb), sbuf + (k ^ 1u) * 4096u, mres + 8u * (k ^ 1u));
+                            tepi_request_residual(&tmR, tepi_box(p, slab_row(nx.t), (nx.t % tiles_n) * tnw + nx.cb), sbuf + (k ^ 1u) * 4096u, mres + 8u * (k ^ 1u));
                     }
                     if (!mbar_wait_prof<7>(prof_on, mres + 8u * k, (blk >> 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 17); *deadp = 1; } break; }
 #pragma unroll
@@ -1001,7 +1250,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
                 }
 #pragma unroll
                 for (int j = 0; j < 32; j++) {
-                    const float f = small_acc ? __int_as_float((int)v[j] + 0x4B400000) - 12582912.f : (float)(int)v[j];
+                    const float f = E2M1 ? __uint_as_float(v[j]) + 0.f : small_acc ? __int_as_float((int)v[j] + 0x4B400000) - 12582912.f : (float)(int)v[j];
                     o[j] = has_res ? o[j] + f : f;
                 }
                 if (want_sum && row_ok) {
@@ -1076,25 +1325,30 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         (void)prof_on;
         for (int t = cta0; t < ntiles && !dead; t += cstep, a++) {
             const unsigned buf = a & 1;
-            const int hf = half_of(t), wcols = hf ? TNI / 2 : TNI;         // columns of the accumulator in use
-            const int R0 = tile_row0(t), n0 = (tile_of(t) % tiles_n) * TNI + (hf == 2 ? TNI / 2 : 0);
+            const int hf = half_of(t), wcols = hf ? tnw / 2 : tnw;         // columns of the accumulator in use
+            const int R0 = tile_row0(t), n0 = (tile_of(t) % tiles_n) * tnw + (hf == 2 ? tnw / 2 : 0);
             // two warps per TMEM lane quarter: they split the row blocks of a two-block tile, else the columns.  Row data
             // and the first block's residual are fetched before the accumulator is waited for.
             const int wg = (warp - 4) >> 2;
-            const int emb = MT == 2 ? wg : 0, ec0 = MT == 2 ? 0 : wg * (wcols / 2), ec1 = MT == 2 ? TNI : (wg + 1) * (wcols / 2);
+            const int emb = MT == 2 ? wg : 0, chalf = (wcols / 32 + 1) / 2 * 32;
+            const int ec0 = MT == 2 || wg == 0 ? 0 : chalf, ec1 = MT == 2 || wg == 1 ? wcols : chalf;
             SlabRows sr;
             slab_rows<FUSED>(p, R0 + emb * UTM + (warp & 3) * 32, lane, sr);
             float4 res[8];
             bool res_loaded = false;
-            if (FUSED == 2 && (p.KN & 3) == 0 && n0 + ec0 + 32 <= p.KN) {
-                slab_load_residual(p, sr, n0 + ec0, lane, res);
+            // the warp that reads the columns which overlap the other accumulator begins with them
+            const bool first_in_line = E2M1 && overlap && wg == (buf ? 0 : 1), down = first_in_line && buf == 0;
+            const int clast = n0 + ec1 <= p.KN ? ec1 : ec0 + max(0, (p.KN - n0 - ec0 + 31) / 32 * 32);     // end of the blocks with real filters
+            const int cfirst = down ? clast - 32 : ec0;
+            if (FUSED == 2 && (p.KN & 3) == 0 && ec0 < clast && n0 + cfirst + 32 <= p.KN) {
+                slab_load_residual(p, sr, n0 + cfirst, lane, res);
                 res_loaded = true;
             }
             if (!mbar_wait_prof<6, PAIR>(prof_on, accFull + 8 * buf, (a >> 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 16); *deadp = 1; } break; }
             tc_fence_after();
             PROF_T0;
-            slab_columns<FUSED>(p, tmem_base + buf * ACOLS + (uint32_t)(emb * TNI) + ((uint32_t)((warp & 3) * 32) << 16), sr, n0, ec0, ec1,
-                                lane, sStage + (warp - 4) * 4096, res, res_loaded, pending);
+            slab_columns<FUSED, E2M1>(p, tmem_base + buf * ABUF + (uint32_t)(emb * TNI) + ((uint32_t)((warp & 3) * 32) << 16), sr, n0, ec0, ec1,
+                                lane, sStage + (warp - 4) * 4096, res, res_loaded, pending, down, first_in_line ? accFreed : 0u);
             tc_fence_before();
             __syncwarp();
             if (lane == 0) { if (PAIR) mbar_arrive_cluster(accEmpty + 8 * buf, 0u); else mbar_arrive(accEmpty + 8 * buf); }
@@ -1115,7 +1369,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     __syncthreads();
     if (PAIR) cluster_sync_all();                                          // the other CTA no longer reads this one's memory nor arrives on its barriers
     pdl_launch_dependents();
-    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, (uint32_t)(2 * ACOLS)); else tmem_dealloc(tmem_base, (uint32_t)(2 * ACOLS)); }
+    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, (uint32_t)TCOLS); else tmem_dealloc(tmem_base, (uint32_t)TCOLS); }
     if (FUSED) {
         if (p.next_qx != nullptr) quantize_tail(quant_tail_args(p), reinterpret_cast<float*>(smem), status);   // the patch area is free now
         else fused_finish(p);
@@ -1282,25 +1536,47 @@ static int pair_clusters();
 static bool pair_launch_possible() { return pair_clusters() >= 1; }
 
 // A tile shape and what it needs.
-struct TcPlan { int mt, tn, sb; bool resident, pair; int prow, nrows, nst, smem; long long tiles_m, tiles_n; };
+struct TcPlan { int mt, tn, tnw, sb; bool resident, pair; int prow, nrows, nst, smem; long long tiles_m, tiles_n; };
+
+// First tile that is worked as two halves (see SPLIT in the kernel), ntiles = none: a last round of the persistent grid
+// that fills at most half of it is split, so that it takes about half as long.
+static long long split_point(long long ntiles, int sms, bool capable) {
+#ifdef TAB_TUNE
+    if (const char* env = getenv("TAB_SPLIT")) if (atoi(env) == 0) return ntiles;      // build-time diagnostic only
+#endif
+    const long long grid = ntiles < sms ? ntiles : sms, rest = grid > 0 ? ntiles % grid : 0;
+    return capable && ntiles > grid && rest != 0 && 2 * rest <= grid ? ntiles - rest : ntiles;
+}
 
 // pair: clusters of two CTAs; a tile is 256 rows (128 per CTA) x tn filters, a ring stage holds tn/2 filters per CTA.
-static bool plan_shape(const TcConvParams& p, int mt, int tn, int sb, TcPlan* out, bool pair = false) {
+static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, TcPlan* out, bool pair = false) {
     const long long halo = (long long)((p.KH - 1) / p.s1) * p.VW + (p.KW - 1) / p.s2;
     const long long nrows = 128LL * mt + halo, prow = (nrows + 7) / 8 * 8;
     const long long fixed = 2 * prow * IROW + 1024 + 8 * (p.tepi ? 8192 : 4096) + 1024;   // patches, barriers, epilogue buffers, alignment
-    const long long nres = p.PC == 1 ? ((long long)p.KH * p.KW + 1) / 2 : (long long)p.KH * p.KW * ((p.PC + 1) / 2);   // slots of resident filters
+    const int tlog = resident_taps_log2(p.PC, p.e2m1 != 0), wpr = p.e2m1 ? 4 : 2;
+    const long long taps = (long long)p.KH * p.KW;
+    const long long nres = tlog ? (taps + (1 << tlog) - 1) >> tlog : taps * ((p.PC + wpr - 1) / wpr);   // slots of resident filters
     TcPlan pl;
     pl.mt = mt; pl.tn = tn; pl.sb = sb; pl.pair = pair;
-    pl.resident = !pair && p.KN <= tn && fixed + nres * tn * IROW <= UMMA_SMEM_MAX;
-    const long long smem = pl.resident ? fixed + nres * tn * IROW : fixed + (long long)sb * (pair ? tn / 2 : tn) * IROW;
+    // The filters are shared out evenly over as few tiles of at most tn as hold them, in whole 32-column blocks of the
+    // epilogue: 130 filters are multiplied as 160 columns and not as 256, 300 as twice 160 and not as 256 + 256.
+    pl.tiles_n = (p.KN + tn - 1) / tn;
+    pl.tnw = (int)((p.KN + pl.tiles_n - 1) / pl.tiles_n + 31) / 32 * 32;
+    const long long tnw = pl.tnw;
+    pl.resident = !pair && p.KN <= tn && fixed + nres * tnw * IROW <= UMMA_SMEM_MAX;
+    const long long smem = pl.resident ? fixed + nres * tnw * IROW : fixed + (long long)sb * (pair ? tnw / 2 : tnw) * IROW;
     if (smem > UMMA_SMEM_MAX) return false;
     pl.prow = (int)prow; pl.nrows = (int)nrows; pl.nst = pl.resident ? (int)nres : sb; pl.smem = (int)smem;
     const long long Mv = (long long)(p.N - 1) * p.VH * p.VW + (long long)(p.OH - 1) * p.VW + p.OW;   // last useful virtual row + 1
     pl.tiles_m = (Mv + 128LL * mt - 1) / (128LL * mt);
     if (pair) pl.tiles_m = (pl.tiles_m + 1) / 2;
-    pl.tiles_n = (p.KN + tn - 1) / tn;
     if (pl.tiles_m * pl.tiles_n >= (1LL << 31) - 65536) return false;      // tile and work-item indices are ints
+    // tiles whose last round is worked in halves: both halves whole epilogue blocks
+    const bool halves = split_point(pl.tiles_m * pl.tiles_n, sms, split_capable(mt, tn, pl.resident, p.tepi != 0, pair)) < pl.tiles_m * pl.tiles_n;
+    if (halves && pl.tnw % 64 != 0) {
+        const long long more = (long long)sb * 32 * IROW;
+        if (smem + more <= UMMA_SMEM_MAX) { pl.tnw += 32; pl.smem = (int)(smem + more); }
+    }
     *out = pl;
     return true;
 }
@@ -1321,23 +1597,23 @@ static bool tc_plan(const TcConvParams& p, int sms, TcPlan* best) {
     if (const char* env = getenv("TAB_TILE")) {
         int mt = 0, tn = 0, pair = 0;
         if (sscanf(env, "%d,%d,%d", &mt, &tn, &pair) == 3) {
-            if (pair) return tn == 256 && mt == 1 && !p.tepi && p.residual == nullptr && plan_shape(p, 1, 256, 8, best, true);
+            if (pair) return !p.e2m1 && tn == 256 && mt == 1 && !p.tepi && p.residual == nullptr && plan_shape(p, sms, 1, 256, 8, best, true);
             for (const auto& c : cands)
-                if (c[0] == mt && c[1] == tn) return plan_shape(p, mt, tn, c[2], best);
+                if (c[0] == mt && c[1] == tn) return plan_shape(p, sms, mt, tn, c[2], best);
             return false;
         }
     }
 #endif
     TcPlan lone;
-    const bool fits_whole = plan_shape(p, 1, 256, 4, &lone) && lone.resident;      // a block that stays in shared memory is fetched once anyway
-    if (tn0 == 256 && !p.tepi && !fits_whole && p.PA * p.PB == 1 && p.KH * p.KW > 1 && p.residual == nullptr && pair_launch_possible() &&
-        plan_shape(p, 1, 256, 8, best, true) &&
+    const bool fits_whole = plan_shape(p, sms, 1, 256, 4, &lone) && lone.resident;      // a block that stays in shared memory is fetched once anyway
+    if (tn0 == 256 && !p.e2m1 && !p.tepi && !fits_whole && p.PA * p.PB == 1 && p.KH * p.KW > 1 && p.residual == nullptr && pair_launch_possible() &&
+        plan_shape(p, sms, 1, 256, 8, best, true) &&
         best->tiles_m * best->tiles_n * 2 > sms) return true;              // with a round of tiles for the pairs or less, single CTAs measured faster
     bool found = false;
     for (const auto& c : cands) {
         if (c[1] > tn0) continue;
         TcPlan pl;
-        if (!plan_shape(p, c[0], c[1], c[2], &pl)) continue;
+        if (!plan_shape(p, sms, c[0], c[1], c[2], &pl)) continue;
         if (!found) { *best = pl; found = true; }
         if (pl.tiles_m * pl.tiles_n * 2 > sms) { *best = pl; break; }      // enough tiles: take it; else keep looking for more tiles
         if (pl.tiles_m * pl.tiles_n > best->tiles_m * best->tiles_n) *best = pl;
@@ -1356,6 +1632,7 @@ static bool grid_in_range(const TcConvParams& p) {
 static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
     if ((long long)p.N * p.H * p.W >= (1LL << 31) || (long long)p.M >= (1LL << 31) - 512) return false;
     if ((long long)p.KH * p.KW * p.PC >= (1LL << 20)) return false;
+    if (p.e2m1 && (long long)p.KH * p.KW * p.C >= (1LL << 24)) return false;       // sums the fp32 accumulators may not hold exactly
     const bool tepi_ok = (p.KN & 3) == 0 && !(reinterpret_cast<uintptr_t>(p.y) & 15) && !(reinterpret_cast<uintptr_t>(p.residual) & 15) &&
                          (long long)p.KN * p.OW * p.OH * 4 < (1LL << 40);
     bool tepi_pays = p.residual != nullptr && p.y16 == nullptr && p.KN <= 64 && (long long)p.KH * p.KW * p.C <= 1024;
@@ -1376,17 +1653,7 @@ static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
     return true;
 }
 
-// First tile that is worked as two halves (see SPLIT in the kernel), ntiles = none: a last round of the persistent grid
-// that fills at most half of it is split, so that it takes about half as long.
-static long long split_point(long long ntiles, int sms, bool capable) {
-#ifdef TAB_TUNE
-    if (const char* env = getenv("TAB_SPLIT")) if (atoi(env) == 0) return ntiles;      // build-time diagnostic only
-#endif
-    const long long grid = ntiles < sms ? ntiles : sms, rest = grid > 0 ? ntiles % grid : 0;
-    return capable && ntiles > grid && rest != 0 && 2 * rest <= grid ? ntiles - rest : ntiles;
-}
-
-template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false>
+template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false, bool E2M1 = false>
 static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcConvParams& p, const TcPlan& pl,
                             int sms, int* status, cudaStream_t stream) {
     static std::mutex mu;
@@ -1397,7 +1664,7 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
     {
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 64 || !configured[dev]) {
-            e = cudaFuncSetAttribute(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, UMMA_SMEM_MAX);
+            e = cudaFuncSetAttribute(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, cudaFuncAttributeMaxDynamicSharedMemorySize, UMMA_SMEM_MAX);
             if (e != cudaSuccess) return record_cuda_error(e);
             if (dev >= 0 && dev < 64) configured[dev] = true;
         }
@@ -1406,23 +1673,22 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
     if (PAIR) {
         const long long pairs = std::min<long long>(sms / 2, pair_clusters());
         const unsigned grid = 2u * (unsigned)(ntiles < pairs ? ntiles : pairs);
-        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream, 2u,
-                                  tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles);
+        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream, 2u,
+                                  tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles, pl.tnw);
     }
     const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);
-    const long long split_from = split_point(ntiles, sms, split_capable(MT, TNI, BRES, TEPI, PAIR));
-    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream,
-                      tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)split_from);
+    const long long split_from = split_point(ntiles, sms, split_capable(MT, TNI, BRES, TEPI, PAIR) && pl.tnw % 64 == 0);
+    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream,
+                      tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)split_from, pl.tnw);
 }
 
-template <int MT, int TNI, int SB>
+template <int MT, int TNI, int SB, bool E2M1>
 static int launch_persist(const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcConvParams& p, const TcPlan& pl,
                           int sms, int* status, cudaStream_t stream) {
     const int fused = p.residual ? 2 : (p.abs_sums ? 1 : 0);
     const bool tepi = p.tepi != 0;
-#define TAB_LAUNCH(BR, FU, TE) return launch_persist_u<MT, TNI, SB, BR, FU, TE>(tmB, tmY, tmR, p, pl, sms, status, stream)
     if (pl.pair) {
-        if constexpr (MT == 1 && TNI == 256) {
+        if constexpr (MT == 1 && TNI == 256 && !E2M1) {
             if (fused == 2) return TAB_E_TOO_LARGE;                        // the planner does not pair layers with a residual
             if (fused == 1) return launch_persist_u<1, 256, SB, false, 1, false, true>(tmB, tmY, tmR, p, pl, sms, status, stream);
             return launch_persist_u<1, 256, SB, false, 0, false, true>(tmB, tmY, tmR, p, pl, sms, status, stream);
@@ -1430,10 +1696,19 @@ static int launch_persist(const CUtensorMap& tmB, const CUtensorMap& tmY, const 
             return TAB_E_TOO_LARGE;
         }
     }
-#define TAB_LAUNCH_F(BR, TE) do { if (fused == 2) TAB_LAUNCH(BR, 2, TE); if (fused == 1) TAB_LAUNCH(BR, 1, TE); TAB_LAUNCH(BR, 0, TE); } while (0)
-    if (pl.resident) { if (tepi) TAB_LAUNCH_F(true, true); TAB_LAUNCH_F(true, false); }
-    if (tepi) TAB_LAUNCH_F(false, true);
-    TAB_LAUNCH_F(false, false);
+#define TAB_LAUNCH(BR, FU, TE) return launch_persist_u<MT, TNI, SB, BR, FU, TE, false, E2M1>(tmB, tmY, tmR, p, pl, sms, status, stream)
+    if (tepi) {                                                            // residual layers of at most 64 filters
+        if constexpr (TNI == 64) {
+            if (fused != 2) return TAB_E_TOO_LARGE;
+            if (pl.resident) TAB_LAUNCH(true, 2, true);
+            TAB_LAUNCH(false, 2, true);
+        } else {
+            return TAB_E_TOO_LARGE;
+        }
+    }
+#define TAB_LAUNCH_F(BR) do { if (fused == 2) TAB_LAUNCH(BR, 2, false); if (fused == 1) TAB_LAUNCH(BR, 1, false); TAB_LAUNCH(BR, 0, false); } while (0)
+    if (pl.resident) TAB_LAUNCH_F(true);
+    TAB_LAUNCH_F(false);
 #undef TAB_LAUNCH_F
 #undef TAB_LAUNCH
 }
@@ -1459,6 +1734,20 @@ static int pair_clusters() {
         known[dev] = ok ? clusters + 1 : 1;
     }
     return known[dev] - 1;
+}
+
+template <bool E2M1>
+static int launch_plan(const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcConvParams& p, const TcPlan& pl,
+                       int sms, int* status, cudaStream_t stream) {
+#define TAB_PLAN(MT, TN, SB) return launch_persist<MT, TN, SB, E2M1>(tmB, tmY, tmR, p, pl, sms, status, stream)
+    if (pl.pair) {
+        if constexpr (!E2M1) TAB_PLAN(1, 256, 8);
+        return TAB_E_TOO_LARGE;
+    }
+    if (pl.tn == 64) { if (pl.mt == 2) TAB_PLAN(2, 64, 6); TAB_PLAN(1, 64, 6); }
+    if (pl.tn == 128) { if (pl.mt == 2) TAB_PLAN(2, 128, 4); TAB_PLAN(1, 128, 6); }
+    TAB_PLAN(1, 256, 4);
+#undef TAB_PLAN
 }
 
 static thread_local char g_last_kernel[112] = "none";
@@ -1487,7 +1776,7 @@ int tc_conv_dispatch(TcConvParams p, cudaStream_t stream) {
     alignas(64) CUtensorMap tmB, tmY, tmR;
     // filter boxes: a pair's CTA and a kernel that can work tiles in halves fetch half a tile's filters per copy
     const bool half_box = pl.pair || split_capable(pl.mt, pl.tn, pl.resident, p.tepi != 0, pl.pair);
-    if (!make_map_2d(&tmB, p.w8, (unsigned long long)p.Kw * 64, (unsigned long long)p.KN, (unsigned)(half_box ? pl.tn / 2 : pl.tn))) return TAB_E_TOO_LARGE;
+    if (!make_map_2d(&tmB, p.w8, (unsigned long long)p.Kw * (p.e2m1 ? 32 : 64), (unsigned long long)p.KN, (unsigned)(half_box ? pl.tnw / 2 : pl.tnw))) return TAB_E_TOO_LARGE;
     tmY = tmB; tmR = tmB;                                                   // placeholders when the epilogue does not use them
     if (p.tepi) {
         const int bw = p.VW >= 32 ? 32 : p.VW, bh = 32 / bw;
@@ -1495,13 +1784,10 @@ int tc_conv_dispatch(TcConvParams p, cudaStream_t stream) {
         if (p.residual && !make_map_4d(&tmR, p.residual, p.KN, p.OW, p.OH, p.N, bw, bh)) return TAB_E_TOO_LARGE;
     }
     int* status = umma_status_ptr();
-    const bool halves = split_point(pl.tiles_m * pl.tiles_n, sms, half_box && !pl.pair) < pl.tiles_m * pl.tiles_n;
+    const bool halves = split_point(pl.tiles_m * pl.tiles_n, sms, half_box && !pl.pair && pl.tnw % 64 == 0) < pl.tiles_m * pl.tiles_n;
     snprintf(g_last_kernel, sizeof(g_last_kernel), "conv_umma_persist_kernel<%d,%d,%d,%d,%d,%d%s> grid %dx%d%s%s", pl.mt, pl.tn, pl.sb, (int)pl.resident,
-             p.residual ? 2 : (p.abs_sums ? 1 : 0), p.tepi, pl.pair ? ",pair" : "", p.VH, p.VW, halves ? " halves" : "", p.next_qx ? " +next" : "");
-    if (pl.pair) return launch_persist<1, 256, 8>(tmB, tmY, tmR, p, pl, sms, status, stream);
-    if (pl.tn == 64) return pl.mt == 2 ? launch_persist<2, 64, 6>(tmB, tmY, tmR, p, pl, sms, status, stream) : launch_persist<1, 64, 6>(tmB, tmY, tmR, p, pl, sms, status, stream);
-    if (pl.tn == 128) return pl.mt == 2 ? launch_persist<2, 128, 4>(tmB, tmY, tmR, p, pl, sms, status, stream) : launch_persist<1, 128, 6>(tmB, tmY, tmR, p, pl, sms, status, stream);
-    return launch_persist<1, 256, 4>(tmB, tmY, tmR, p, pl, sms, status, stream);
+             p.residual ? 2 : (p.abs_sums ? 1 : 0), p.tepi, pl.pair ? ",pair" : (p.e2m1 ? ",e2m1" : ""), p.VH, p.VW, halves ? " halves" : "", p.next_qx ? " +next" : "");
+    return p.e2m1 ? launch_plan<true>(tmB, tmY, tmR, p, pl, sms, status, stream) : launch_plan<false>(tmB, tmY, tmR, p, pl, sms, status, stream);
 }
 
 }  // namespace tab

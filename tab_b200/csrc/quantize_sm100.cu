@@ -34,30 +34,58 @@ template <int WB>
 __device__ __forceinline__ void expand_group(const uint64_t* __restrict__ qw, int8_t* __restrict__ w8, long long idx, int PC, int C) {
     const long long word = idx >> 2;
     const int grp = (int)(idx & 3);
-    const int pc = (int)(word % PC);
-    const int cbase = pc * 64 + grp * 16;
     uint32_t s16, m16;
     if (WB == 2) {
-        m16 = (uint32_t)(qw[word * 2 + 1] >> (grp * 16)) & 0xFFFFu;
-        s16 = (uint32_t)(qw[word * 2] >> (grp * 16)) & m16;
+        const uint64_t sg = __ldg(qw + word * 2), mg = __ldg(qw + word * 2 + 1);
+        m16 = (uint32_t)(mg >> (grp * 16)) & 0xFFFFu;
+        s16 = (uint32_t)(sg >> (grp * 16));
     } else {
-        s16 = (uint32_t)(qw[word] >> (grp * 16)) & 0xFFFFu;     // bit = 1 means -1
         m16 = 0xFFFFu;
+        s16 = (uint32_t)(__ldg(qw + word) >> (grp * 16));                  // bit = 1 means -1
     }
-    uint32_t o[4];
+    if (C & 63) {                                                          // only then is there a word with a tail, the last of PC
+        const int pc = word < (1LL << 31) ? (int)((uint32_t)word % (uint32_t)PC) : (int)(word % PC);
+        const int real = C - (pc * 64 + grp * 16);
+        if (real < 16) m16 &= real > 0 ? (1u << real) - 1u : 0u;
+    }
+    s16 &= m16;
+    *reinterpret_cast<uint4*>(w8 + word * 64 + grp * 16) =
+        make_uint4(expand4(m16 & 15u, s16 & 15u), expand4((m16 >> 4) & 15u, (s16 >> 4) & 15u),
+                   expand4((m16 >> 8) & 15u, (s16 >> 8) & 15u), expand4(m16 >> 12, s16 >> 12));
+}
+
+// One thread per 32 channels of packed weights: 16 bytes of e2m1 nibbles into [KN][KH*KW*PC][32], in the order nibbles32 gives
+// them; channels beyond C become 0.
+template <int WB>
+__device__ __forceinline__ void expand_half(const uint64_t* __restrict__ qw, uint8_t* __restrict__ w4, long long idx, int PC, int C) {
+    const long long word = idx >> 1;
+    const int h = (int)(idx & 1);
+    const uint32_t* q = reinterpret_cast<const uint32_t*>(qw + word * WB) + h;
+    uint32_t s = __ldg(q), m = WB == 2 ? __ldg(q + 2) : 0xFFFFFFFFu;
+    if (C & 63) {
+        const int pc = word < (1LL << 31) ? (int)((uint32_t)word % (uint32_t)PC) : (int)(word % PC);
+        const int real = C - (pc * 64 + h * 32);
+        if (real < 32) m &= real > 0 ? (1u << real) - 1u : 0u;
+    }
+    *reinterpret_cast<uint4*>(w4 + word * 32 + h * 16) = nibbles32(m, s & m);
+}
+
+__global__ void pack_weights_kernel(const int8_t* __restrict__ w8, uint8_t* __restrict__ w4, long long halves) {
+    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (idx >= halves) return;
+    uint32_t m = 0, s = 0;
 #pragma unroll
-    for (int w = 0; w < 4; w++) {
-        uint32_t r = 0;
+    for (int k = 0; k < 2; k++) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(w8 + idx * 32) + k);
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int b = 0; b < 4; b++) {
-            const int i = 4 * w + b;
-            int v = ((m16 >> i) & 1u) ? (((s16 >> i) & 1u) ? -1 : 1) : 0;
-            if (cbase + i >= C) v = 0;
-            r |= (uint32_t)(v & 0xFF) << (8 * b);
+        for (int i = 0; i < 16; i++) {
+            const uint32_t b = (q[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+            m |= (b & 1u) << (16 * k + i);
+            s |= (b >> 7) << (16 * k + i);
         }
-        o[w] = r;
     }
-    *reinterpret_cast<uint4*>(w8 + word * 64 + grp * 16) = make_uint4(o[0], o[1], o[2], o[3]);
+    *reinterpret_cast<uint4*>(w4 + idx * 16) = nibbles32(m, s & m);
 }
 
 template <int WB>
@@ -74,9 +102,9 @@ __device__ __forceinline__ void quant_prologue(const QuantExtras& ex, int n) {
     pdl_wait();
     if (ex.qw != nullptr) {                                                // the weights, spread over all CTAs of the launch
         const long long stride = (long long)gridDim.x * gridDim.y * blockDim.x;
-        for (long long idx = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; idx < ex.words * 4; idx += stride) {
-            if (ex.wbits == 2) expand_group<2>(ex.qw, ex.w8, idx, ex.PC, ex.C);
-            else expand_group<1>(ex.qw, ex.w8, idx, ex.PC, ex.C);
+        for (long long idx = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; idx < ex.words * 2; idx += stride) {
+            if (ex.wbits == 2) expand_half<2>(ex.qw, ex.w4, idx, ex.PC, ex.C);
+            else expand_half<1>(ex.qw, ex.w4, idx, ex.PC, ex.C);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -383,6 +411,17 @@ static unsigned ctas_per_image(long long words_per_image, long long words_per_st
     return (unsigned)(per_image < 1 ? 1 : per_image);
 }
 
+// A launch that also expands weights gets enough CTAs for that, 32 channels per thread up to four CTAs per SM: the tensor of a
+// single image fills 4 CTAs, which took 65 us for the weights of a 3x3x512 -> 512 layer.
+static dim3 quantize_grid(unsigned per_image, int N, const QuantExtras& ex) {
+    if (ex.qw) {
+        const long long groups = (ex.words * 2 + QTHREADS - 1) / QTHREADS, want = groups < 148 * 4 ? groups : 148 * 4;
+        const unsigned share = (unsigned)((want + N - 1) / N);
+        if (per_image < share) per_image = share;
+    }
+    return dim3(per_image, (unsigned)N);
+}
+
 // BTN_W is cleared by a memset only where several CTAs add to an image's count; else the kernel writes it.
 static int clear_counts(int32_t* btn, int bits, dim3 grid, cudaStream_t stream) {
     if (!btn || bits == 1 || grid.x == 1) return TAB_OK;
@@ -398,7 +437,7 @@ static int launch_quantize_any(const void* x, const float* ths, uint64_t* q, int
     const FastDiv dPC = make_fastdiv((uint32_t)PC);
     const int V = load_width(x, C, IN16);
     const bool one = C <= 8;                                               // one lane per word
-    const dim3 grid(ctas_per_image(wpi, (long long)QTHREADS / (one ? 1 : 8) * QUNROLL, N), (unsigned)N);
+    const dim3 grid = quantize_grid(ctas_per_image(wpi, (long long)QTHREADS / (one ? 1 : 8) * QUNROLL, N), N, ex);
     const int rc = clear_counts(btn, BITS, grid, stream);
     if (rc != TAB_OK) return rc;
 #define TAB_QANY(VV) (one ? launch_pdl(quantize_any_kernel<BITS, IN16, VV, 1>, grid, dim3(QTHREADS), 0, stream, x, ths, q, btn, wpi, pixels * C, C, PC, dPC, ex) \
@@ -430,7 +469,7 @@ int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn
     const bool fast = (C % 64 == 0) && ((reinterpret_cast<uintptr_t>(x) & 31) == 0);
     uint64_t* q = reinterpret_cast<uint64_t*>(qx);
     if (fast) {
-        const dim3 grid(ctas_per_image(wpi, in16 ? 2 * QWORDS_PER_ITER : QWORDS_PER_ITER, N), (unsigned)N);
+        const dim3 grid = quantize_grid(ctas_per_image(wpi, in16 ? 2 * QWORDS_PER_ITER : QWORDS_PER_ITER, N), N, ex);
         const int rc = clear_counts(btn, bits, grid, stream);
         if (rc != TAB_OK) return rc;
         if (in16) {
@@ -615,6 +654,14 @@ int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* 
                            int N, int H, int W, int C, int* status, cudaStream_t stream) {
     return bits == 2 ? quantize_auto_by_width<2>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream)
                      : quantize_auto_by_width<1>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream);
+}
+
+int pack_weights_dispatch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, cudaStream_t stream) {
+    const long long halves = (long long)KN * KH * KW * packed_channels(C) * 2;
+    if (halves == 0) return TAB_OK;
+    if (halves >= (1LL << 31) * 256) return TAB_E_TOO_LARGE;
+    pack_weights_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, stream>>>(w8, w4, halves);
+    return check_launch();
 }
 
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream) {

@@ -60,8 +60,8 @@ inline int weight_bits(int type) { return (type == 1 || type == 3) ? 1 : 2; }   
 struct QuantExtras {
     double* zero_sums = nullptr;         // [N]: cleared
     unsigned* zero_counter = nullptr;    // cleared
-    const uint64_t* qw = nullptr;        // packed weights [KN][KH*KW*PC][wbits] to expand into w8 [KN][KH*KW*PC][64]
-    int8_t* w8 = nullptr;
+    const uint64_t* qw = nullptr;        // packed weights [KN][KH*KW*PC][wbits] to expand into w4 [KN][KH*KW*PC][32] (4-bit operands)
+    uint8_t* w4 = nullptr;
     long long words = 0;                 // KN*KH*KW*PC
     int wbits = 2, PC = 1, C = 64;       // of the weights
 };
@@ -70,6 +70,8 @@ struct QuantExtras {
 int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn, int bits,
                       int N, int H, int W, int C, cudaStream_t stream, const QuantExtras* extras = nullptr, bool in16 = false);
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream);
+// Byte weights {-1,0,+1} -> the 4-bit operands of the same words.
+int pack_weights_dispatch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, cudaStream_t stream);
 // Thresholds scale * mean|x[n]| and the bit-planes against them in one launch (sums: N doubles, bar: two words, all zero
 // before and after).
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,

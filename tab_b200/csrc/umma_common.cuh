@@ -57,7 +57,8 @@ inline FastDiv make_fastdiv(uint32_t d) {
 // Output (n, oh, ow) is virtual row (n*VH + oh)*VW + ow of any plane; rows with oh >= OH or ow >= OW are computed and dropped.
 struct TcConvParams {
     const uint64_t* qx;      // activation bit-planes
-    const int8_t* w8;        // byte weights
+    const int8_t* w8;        // weights: bytes, or (e2m1) nibbles, [KN][KH*KW*PC][64 or 32 bytes]
+    int e2m1;                // operands are 4-bit floats (see umma_e2m1) instead of bytes
     float* y;                // [M][KN]
     int16_t* y16;            // when not null the result goes here as int16 instead (no residual; |y| <= KH*KW*C must fit)
     const float* residual;   // [M][KN] added to the result, or null
@@ -164,6 +165,34 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
                  "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
                  :: "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate) : "memory");
 }
+// ---- 4-bit operands ----------------------------------------------------------------------------------------------------
+// kind::mxf4 multiplies e2m1 floats - {-1, 0, +1} are the nibbles 0xA, 0x0, 0x2 - with a power-of-two scale per 32 of them, here
+// always 1, into fp32: 128 x N x 64 in the cycles kind::i8 takes for 128 x N x 32 (measured on B200: 48 / 64 / 128 cycles at N = 64 /
+// 128 / 256 for both).  Products of {-1, 0, +1} accumulate exactly while the sum stays below 2^24 in magnitude, which
+// KH*KW*C < 2^24 guarantees; measured exact with running sums up to 15.4 million.
+// Order of the channels inside a word: the sum does not depend on it as long as both operands agree, so the order is the one
+// that needs no bit spreading - 32-bit word 4h + k of the eight holds channels 32h + 4i + k, i = 0..7 (channel 32h + 4i + k in
+// nibble i), a shift and a mask of plane bits.
+__host__ __device__ constexpr uint32_t umma_idesc_e2m1(int n, int m) {
+    return (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | (1u << 23) | ((uint32_t)(m >> 4) << 24);
+}
+// sf: tensor-memory columns that hold 0x7F (scale 1) everywhere.
+__device__ __forceinline__ void umma_e2m1(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t sf, uint32_t accumulate) {
+    asm volatile("{\n\t.reg .pred p;\n\t"
+                 "setp.ne.b32 p, %4, 0;\n\t"
+                 "tcgen05.mma.cta_group::1.kind::mxf4.block_scale.block32 [%0], %1, %2, %3, [%5], [%5], p;\n\t}"
+                 :: "r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(sf) : "memory");
+}
+// 16 columns x this warp's 32 lanes of tensor memory := v.
+__device__ __forceinline__ void tmem_fill16(uint32_t taddr, uint32_t v) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1,%1};" ::"r"(taddr), "r"(v) : "memory");
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+// 32 channels (32 bits of the magnitude plane and of the sign plane, sign only where magnitude) -> four words of nibbles.
+__device__ __forceinline__ uint4 nibbles32(uint32_t m, uint32_t s) {
+    return make_uint4(((m << 1) & 0x22222222u) | ((s << 3) & 0x88888888u), (m & 0x22222222u) | ((s << 2) & 0x88888888u),
+                      ((m >> 1) & 0x22222222u) | ((s << 1) & 0x88888888u), ((m >> 2) & 0x22222222u) | (s & 0x88888888u));
+}
 __device__ __forceinline__ void umma_commit(uint32_t mbar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(mbar) : "memory");
 }
@@ -247,8 +276,20 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t tmem_base, uint32_t c
     asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem_base), "r"(cols) : "memory");
 }
 
+// Four quantised values from the low four bits of a magnitude and a sign nibble: bytes 0x00 / 0x01 / 0xFF.
+__device__ __forceinline__ uint32_t expand4(uint32_t mnib, uint32_t snib) {
+    const uint32_t m01 = (mnib * 0x00204081u) & 0x01010101u;               // bit i -> byte i (the shifted copies do not overlap)
+    const uint32_t s01 = (snib * 0x00204081u) & 0x01010101u;
+    return m01 | (s01 * 0xFFu);
+}
+
 __device__ __forceinline__ void sts_v4(uint32_t a, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
     asm volatile("st.shared.v4.b32 [%0], {%1,%2,%3,%4};" ::"r"(a), "r"(x), "r"(y), "r"(z), "r"(w) : "memory");
+}
+__device__ __forceinline__ int lds_b32(uint32_t a) {
+    int r;
+    asm volatile("ld.shared.b32 %0, [%1];" : "=r"(r) : "r"(a) : "memory");
+    return r;
 }
 __device__ __forceinline__ int4 lds_v4(uint32_t a) {
     int4 r;

@@ -6,8 +6,8 @@ The reference's only interface is positional ``Conv2d(X, QW, thresholds, btn, ty
 types (cells 12, 17), which reads past the end of ``QW`` (``TAB_GEMM.cu:47-52``).  This module
 
   * quantises the fp32 weights once, at the bitwidth the type needs (``TAB_GEMM.cu:374-379``), keeps ``QW`` and
-    ``BTN_W`` (what ``Conv2d`` takes) and the byte-expanded form the tensor-core kernel multiplies, so that no call
-    re-expands weights;
+    ``BTN_W`` (what ``Conv2d`` takes), the byte-expanded form and the 4-bit form the tensor-core kernel multiplies, so that
+    no call re-expands weights;
   * refuses weights quantised at the wrong bitwidth instead of reading out of bounds;
   * computes the per-image activation thresholds ``scale * mean|x|`` when the caller does not pass them;
   * exposes the two stages separately (``quantize`` / ``conv_bits``) so that several convolutions of one input -
@@ -56,7 +56,25 @@ class TABConv2d(torch.nn.Module):
         self.register_buffer("QW", QW.contiguous())
         self.register_buffer("BTN_W", BTN_W.contiguous())
         self.register_buffer("W8", ops.expand_weights(self.QW, wb, self.KN, self.KH, self.KW, self.C))
+        self.register_buffer("W4", None, persistent=False)                  # W8 as the 4-bit operands the kernel multiplies
+        self._pack()
         self._state = None
+
+    def _pack(self):
+        self.W4 = None
+        if self.W8.is_cuda and self.KH * self.KW * self.C < 1 << 24:       # beyond that the byte form is multiplied
+            self.W4 = ops.pack_weights(self.W8, self.KN, self.KH, self.KW, self.C)
+
+    def _load_from_state_dict(self, *args, **kwargs):
+        super()._load_from_state_dict(*args, **kwargs)
+        self._pack()
+
+    def __setstate__(self, state):
+        super().__setstate__(state)
+        if "W4" not in self._buffers:                                      # pickled before there was one
+            self._non_persistent_buffers_set.add("W4")
+            self._buffers["W4"] = None
+            self._pack()
 
     @classmethod
     def from_float(cls, weight, conv_type, padding=(0, 0), stride=(1, 1), weight_thresholds=None, threshold_scale=0.7):
@@ -113,7 +131,7 @@ class TABConv2d(torch.nn.Module):
             raise ValueError("next_bitwidth needs next_threshold_scale")
         compact = out_int16 and residual is None and self.KH * self.KW * self.C <= 32767
         try:
-            return ops.conv2d_bits(QX, self.W8, self.conv_type, *self.geometry(N, H, W), residual=residual,
+            return ops.conv2d_bits(QX, self.W8 if self.W4 is None else self.W4, self.conv_type, *self.geometry(N, H, W), residual=residual,
                                    threshold_scale=next_threshold_scale, state=state, out_int16=compact, next_bitwidth=next_bitwidth)
         except _cabi.TabError as exc:
             if exc.code != -5:

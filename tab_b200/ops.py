@@ -163,6 +163,20 @@ def expand_weights(QW, bitwidth, KN, KH, KW, C):
     return w8
 
 
+def pack_weights(W8, KN, KH, KW, C):
+    """``expand_weights`` bytes -> uint8 ``{KN,KH,KW,Cp/2}``, the 4-bit operands ``conv2d_bits`` multiplies at twice the rate (in
+    the kernel's own channel order)."""
+    _check_input(W8, "W8", torch.int8)
+    Cp = (int(C) + 63) // 64 * 64
+    if W8.numel() != KN * KH * KW * Cp:
+        raise RuntimeError("W8 has %d bytes, expected KN*KH*KW*Cp = %d" % (W8.numel(), KN * KH * KW * Cp))
+    with torch.cuda.device(W8.device):
+        w4 = torch.empty((KN, KH, KW, Cp // 2), dtype=torch.uint8, device=W8.device)
+        rc = _cabi.lib().tab_pack_weights_launch(W8.data_ptr(), w4.data_ptr(), KN, KH, KW, C, _stream_ptr(W8.device))
+    _cabi.check(rc, "tab_pack_weights_launch")
+    return w4
+
+
 def new_state(N, device):
     """Zeroed state block for ``conv2d_bits(..., threshold_scale=...)``; one block serves any number of calls that are
     ordered on a stream (every call leaves it zeroed)."""
@@ -207,14 +221,16 @@ def quantize_i16(X16, thresholds, bitwidth, N, H, W, C):
 def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW,
                 residual=None, threshold_scale=None, state=None, out_int16=False, next_bitwidth=None):
     """The GEMM stage on the tensor cores: activations as ``Quantize`` wrote them (bitwidth 2 for types 0,1; 1 for
-    types 2,3), weights from ``expand_weights``.  Returns ``(Y, next_thresholds_or_None)``; ``Y = conv + residual``.
+    types 2,3), weights from ``expand_weights`` (int8) or ``pack_weights`` (uint8: twice the rate, KH*KW*C < 2**24).  Returns
+    ``(Y, next_thresholds_or_None)``; ``Y = conv + residual``.
     ``threshold_scale`` needs ``state`` (``new_state``).  ``out_int16``: ``Y`` as int16 (no residual; the values are
     integers of magnitude at most KH*KW*C) for ``quantize_i16``.  ``next_bitwidth`` (needs ``threshold_scale``): the same
     launch also quantises ``Y`` against the next thresholds at that bitwidth and a third value is returned, ``QX`` of the
     next convolution (``[N,OH,OW,ceil(KN/64),bits]`` int64, what ``Quantize(Y, next_thresholds, ...)`` gives).
     Raises ``TabError`` (TAB_E_TOO_LARGE) for shapes the tensor-core kernel does not cover."""
     _check_input(QX, "QX", torch.int64)
-    _check_input(W8, "W8", torch.int8)
+    packed4 = isinstance(W8, torch.Tensor) and W8.dtype == torch.uint8
+    _check_input(W8, "W8", torch.uint8 if packed4 else torch.int8)
     conv_type = int(type)
     p1, p2, s1, s2 = int(padding1), int(padding2), int(stride1), int(stride2)
     N, H, W, C, KN, KH, KW = (int(v) for v in (N, H, W, C, KN, KH, KW))
@@ -222,8 +238,8 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
     ab = 1 if conv_type in (2, 3) else 2
     if QX.numel() != N * H * W * PC * ab:
         raise RuntimeError("QX has %d words, type %d needs %d" % (QX.numel(), conv_type, N * H * W * PC * ab))
-    if W8.numel() != KN * KH * KW * PC * 64:
-        raise RuntimeError("W8 has %d bytes, expected KN*KH*KW*Cp = %d" % (W8.numel(), KN * KH * KW * PC * 64))
+    if W8.numel() != KN * KH * KW * PC * (32 if packed4 else 64):
+        raise RuntimeError("W8 has %d bytes, expected KN*KH*KW*Cp%s = %d" % (W8.numel(), "/2" if packed4 else "", KN * KH * KW * PC * (32 if packed4 else 64)))
     OH, OW = conv_out_size(H, W, KH, KW, p1, p2, s1, s2)
     if residual is not None:
         _check_input(residual, "residual", torch.float32)
@@ -238,6 +254,18 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
     with torch.cuda.device(QX.device):
         Y = torch.empty((N, KN, OH, OW), dtype=torch.int16 if out_int16 else torch.float32, device=QX.device)
         nxt = torch.empty((N,), dtype=torch.float32, device=QX.device) if threshold_scale is not None else None
+        if packed4:
+            nb = 0 if next_bitwidth is None else (1 if int(next_bitwidth) == 1 else 2)
+            QN = torch.empty((N, OH, OW, (KN + 63) // 64, nb), dtype=torch.int64, device=QX.device) if nb else None
+            rc = _cabi.lib().tab_conv2d_packed4_launch(QX.data_ptr(), W8.data_ptr(), Y.data_ptr(), 1 if out_int16 else 0, conv_type,
+                                                       p1, p2, s1, s2, N, H, W, C, KN, KH, KW,
+                                                       residual.data_ptr() if residual is not None else None,
+                                                       state.data_ptr() if nxt is not None else None,
+                                                       nxt.data_ptr() if nxt is not None else None,
+                                                       float(threshold_scale) if threshold_scale is not None else 0.0,
+                                                       QN.data_ptr() if nb else None, nb, _stream_ptr(QX.device))
+            _cabi.check(rc, "tab_conv2d_packed4_launch")
+            return (Y, nxt, QN) if nb else (Y, nxt)
         if next_bitwidth is not None:
             nb = 1 if int(next_bitwidth) == 1 else 2
             QN = torch.empty((N, OH, OW, (KN + 63) // 64, nb), dtype=torch.int64, device=QX.device)

@@ -673,3 +673,129 @@ def test_quantize_i16_any_channels(cuda, conv_path, C):
     for bw in (2, 1):
         q = ops.quantize_i16(dev_t(x, cuda), dev_t(ths, cuda), bw, 3, 9, 11, C)
         assert np.array_equal(q.cpu().numpy(), O.quantize(x.astype(np.float32), ths, bw, 3, 9, 11, C)[0])
+
+
+# ------------------------------------------------------------------- tiles whose width follows the filter count, ragged rows
+
+@pytest.mark.parametrize("geom", [
+    # p1 p2 s1 s2  N  H  W   C   KN KH KW       KN odd / even / multiple of 4; 1 to 4 K steps of the last channel word pair
+    (1, 1, 1, 1, 2, 9, 8, 3, 1, 3, 3),
+    (1, 1, 1, 1, 2, 9, 8, 33, 2, 3, 3),
+    (0, 0, 1, 1, 3, 9, 8, 96, 31, 1, 1),
+    (1, 1, 1, 1, 2, 20, 13, 97, 33, 3, 3),
+    (1, 1, 1, 1, 2, 20, 13, 160, 36, 3, 3),
+    (1, 1, 1, 1, 2, 20, 13, 161, 97, 3, 3),
+    (2, 2, 1, 1, 2, 20, 13, 70, 130, 5, 5),
+    (1, 1, 2, 2, 2, 20, 13, 64, 161, 3, 3),
+    (1, 1, 1, 1, 40, 3, 3, 64, 67, 3, 3),        # a 32-row slab spans three images: |y| sums row by row
+    (1, 1, 1, 1, 2, 14, 14, 256, 259, 3, 3),
+    (1, 1, 1, 1, 90, 14, 14, 130, 300, 3, 3),    # CTA pairs of 160-filter tiles
+    (1, 1, 1, 1, 60, 14, 14, 64, 450, 3, 3),
+    (0, 0, 1, 1, 30, 28, 28, 64, 384, 1, 1),     # two tiles of 192 filters; last round in halves of 96 or whole
+    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # 150 tiles: two halves of 128 filters, the last partial
+    (0, 0, 1, 1, 75, 16, 16, 64, 222, 1, 1),     # the same with 224-wide tiles, not split
+    (1, 1, 1, 1, 1, 12, 12, 64, 60, 3, 3),       # the TMA epilogue with a partial block
+    (1, 1, 1, 1, 1, 12, 12, 64, 28, 3, 3),
+])
+def test_filter_counts_and_channel_steps(cuda, geom, conv_path):
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    test_bits_stage_entry_point(cuda, geom)
+    p1, p2, s1, s2, N, H, W, C, KN, KH, KW = geom
+    x, ths = make_input(7, N, H, W, C)
+    w, wths = make_input(8, KN, KH, KW, C)
+    for t in (0, 3):
+        qw, btn = O.quantize(w, wths, O.weight_bits(t), KN, KH, KW, C)
+        assert np.array_equal(gpu_conv(cuda, x, qw, ths, btn, t, *geom), c_oracle.conv2d(x, qw, ths, btn, t, *geom))
+
+
+@pytest.mark.parametrize("C", [64, 70, 512])
+@pytest.mark.parametrize("N,KN,K", [(1, 5, 3), (1, 512, 3), (700, 16, 1)])
+def test_weight_expansion_inside_a_call(cuda, conv_path, N, KN, K, C):
+    """One-image calls (the launch has more CTAs than the tensor needs, for the weights) and many-image calls."""
+    if conv_path != "tensor":
+        pytest.skip("only the tensor-core path expands weights")
+    x, ths = make_input(5, N, 4, 5, C)
+    w, wths = make_input(6, KN, K, K, C)
+    for t in range(4):
+        qw, btn = O.quantize(w, wths, O.weight_bits(t), KN, K, K, C)
+        g = (K // 2, K // 2, 1, 1, N, 4, 5, C, KN, K, K)
+        assert np.array_equal(gpu_conv(cuda, x, qw, ths, btn, t, *g), c_oracle.conv2d(x, qw, ths, btn, t, *g))
+
+
+# ------------------------------------------------------------------- 4-bit operands
+
+@pytest.mark.parametrize("geom", [
+    # p1 p2 s1 s2  N  H  W   C   KN KH KW       1 to 5 words per pixel (1, 2, 4 taps per filter row), each tile and grid form
+    (1, 1, 1, 1, 2, 9, 8, 3, 1, 3, 3),
+    (1, 1, 1, 1, 2, 20, 13, 64, 64, 3, 3),
+    (2, 2, 1, 1, 2, 20, 13, 70, 130, 5, 5),
+    (1, 1, 1, 1, 3, 14, 14, 128, 128, 3, 3),
+    (1, 1, 1, 1, 2, 14, 14, 129, 97, 3, 3),
+    (1, 1, 1, 1, 2, 14, 14, 256, 259, 3, 3),
+    (1, 1, 1, 1, 2, 14, 14, 260, 36, 3, 3),
+    (1, 1, 2, 2, 2, 20, 13, 64, 161, 3, 3),
+    (1, 1, 2, 2, 64, 14, 14, 320, 256, 3, 3),
+    (1, 2, 3, 2, 3, 9, 8, 130, 70, 3, 3),
+    (1, 1, 1, 1, 40, 3, 3, 64, 67, 3, 3),        # a 32-row slab spans three images
+    (1, 1, 1, 1, 40, 3, 3, 64, 64, 3, 3),
+    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # halves
+    (1, 1, 1, 1, 200, 14, 14, 64, 256, 3, 3),    # several tiles per CTA: accumulators that overlap, one row block
+    (1, 1, 1, 1, 200, 14, 14, 64, 456, 3, 3),    # 256-filter tiles, the last block of the second one without filters
+    (1, 1, 1, 1, 60, 28, 28, 128, 128, 3, 3),    # the same with two row blocks
+    (1, 1, 1, 1, 48, 14, 14, 192, 320, 3, 3),
+    (1, 1, 2, 2, 200, 14, 14, 256, 512, 3, 3),
+    (1, 1, 1, 1, 8, 56, 56, 64, 60, 3, 3),       # the TMA epilogue, several tiles per CTA, a partial block
+    (1, 1, 1, 1, 1, 100, 150, 200, 40, 3, 3),    # long patches: several chunks of items
+    (3, 3, 2, 2, 2, 224, 224, 3, 64, 7, 7),
+])
+@pytest.mark.parametrize("t", [0, 1, 2, 3])
+def test_packed4_weights(cuda, geom, t, conv_path):
+    """The GEMM stage on 4-bit weights against the oracle - plain, with residual and thresholds (a residual that is no
+    integer included), 16-bit output, next layer's input - and against the byte form for what the oracle does not give."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    p1, p2, s1, s2, N, H, W, C, KN, KH, KW = geom
+    x, ths = make_input(91, N, H, W, C)
+    w, wths = make_input(92, KN, KH, KW, C)
+    ab, wb = O.act_bits(t), O.weight_bits(t)
+    qw, btn = O.quantize(w, wths, wb, KN, KH, KW, C)
+    qx, _ = TAB.Quantize(dev_t(x, cuda), dev_t(ths, cuda), ab, N, H, W, C)
+    w8 = TAB.ops.expand_weights(dev_t(qw, cuda), wb, KN, KH, KW, C)
+    w4 = TAB.ops.pack_weights(w8, KN, KH, KW, C)
+    state = TAB.ops.new_state(N, cuda)
+    y, _ = TAB.ops.conv2d_bits(qx, w4, t, *geom)
+    assert ",e2m1>" in _cabi.lib().tab_last_conv_kernel().decode()
+    some = sorted({0, N // 2, N - 1})                                   # images are independent
+    OH, OW = y.shape[2], y.shape[3]
+    for n in some:
+        yo = c_oracle.conv2d(x[n:n + 1], qw, ths[n:n + 1], btn, t, p1, p2, s1, s2, 1, H, W, C, KN, KH, KW)
+        assert np.array_equal(y.reshape(N, -1)[n].cpu().numpy(), yo.reshape(-1))
+    y8, _ = TAB.ops.conv2d_bits(qx, w8, t, *geom)
+    assert torch.equal(y, y8) and not torch.signbit(y[y == 0]).any().item()
+    r = torch.randn(*y.shape, device=cuda) * 5
+    for bw in (None, 2, 1):
+        for kw in (dict(residual=r), dict(residual=torch.round(r)), dict(out_int16=True), dict()):
+            a = TAB.ops.conv2d_bits(qx, w4, t, *geom, threshold_scale=0.7, state=state, next_bitwidth=bw, **kw)
+            b = TAB.ops.conv2d_bits(qx, w8, t, *geom, threshold_scale=0.7, state=state, next_bitwidth=bw, **kw)
+            assert len(a) == len(b) and all(torch.equal(u, v) for u, v in zip(a, b)) and not state.any().item()
+    y3, _ = TAB.ops.conv2d_bits(qx, w4, t, *geom, residual=r)
+    assert torch.equal(y3, y8 + r)
+    assert _cabi.lib().tab_device_status() == 0
+
+
+def test_packed4_sums_are_exact_at_large_magnitude(cuda, conv_path):
+    """All operands +1 but a few: sums near KH*KW*C = 401408 and differing in the last unit."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    N, H, W, C, KN, K = 1, 14, 14, 2048, 40, 14
+    x = torch.ones(N, H, W, C, device=cuda)
+    x[0, 3, 5, :7] = -1.0
+    w = torch.ones(KN, K, K, C, device=cuda)
+    for f in range(KN):
+        w[f].view(-1)[: 3 * f] = -1.0
+    one = torch.full((N,), 0.5, device=cuda)
+    q = TAB.Quantize(w, torch.full((KN,), 0.5, device=cuda), 2, KN, K, K, C)
+    y = TAB.Conv2d(x, q[0], one, q[1], 0, 0, 0, 1, 1, N, H, W, C, KN, K, K)
+    want = (x.double().reshape(1, -1) @ w.double().reshape(KN, -1).T).reshape(-1)
+    assert torch.equal(y.double().reshape(-1), want)
