@@ -34,6 +34,16 @@ setup(
             extra_compile_args=["-O2", "-std=c++17"],
             extra_link_args=["-Wl,-rpath,$ORIGIN/tab_b200"],
         ),
+        # the native bodies of tab_b200.ops, imported from inside the package
+        CppExtension(
+            name="tab_b200._host",
+            sources=[os.path.join("tab_b200", "csrc", "host_ops.cpp")],
+            include_dirs=[os.path.join(cuda_home, "include")],
+            library_dirs=[os.path.join(ROOT, "tab_b200"), os.path.join(cuda_home, "lib64")],
+            libraries=["tab_b200", "c10_cuda", "torch_cuda", "cudart"],
+            extra_compile_args=["-O2", "-std=c++17"],
+            extra_link_args=["-Wl,-rpath,$ORIGIN"],
+        ),
     ],
     cmdclass={"build_ext": BuildExtension},
 )

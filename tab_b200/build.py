@@ -4,8 +4,8 @@
     python -m tab_b200.build --lib      # libtab_b200.so only
 
 ``libtab_b200.so`` (the C ABI of ``include/tab_b200.h``) is compiled with nvcc directly;
-``TAB_CUDA`` (the reference-named PyTorch extension) is built by ``Setup_CUDA.py`` at the repository root
-and links against it.
+``TAB_CUDA`` (the reference-named PyTorch extension) and ``tab_b200._host`` (native bodies of ``tab_b200.ops``) are built by
+``Setup_CUDA.py`` at the repository root and link against it.
 """
 from __future__ import annotations
 
@@ -77,11 +77,17 @@ def module_path():
     return hits[0] if hits else None
 
 
+def host_module_path():
+    import glob
+    hits = glob.glob(os.path.join(HERE, "_host*.so"))
+    return hits[0] if hits else None
+
+
 def build_module(force=False):
-    """``python Setup_CUDA.py build_ext --inplace`` -> TAB_CUDA*.so at the repository root."""
-    deps = [os.path.join(CSRC, "tab_api.cpp"), os.path.join(ROOT, "include", "tab_b200.h"), os.path.join(ROOT, "Setup_CUDA.py")]
-    mp = module_path()
-    if not force and mp and not _stale(mp, deps):
+    """``python Setup_CUDA.py build_ext --inplace`` -> TAB_CUDA*.so at the repository root and tab_b200/_host*.so."""
+    deps = [os.path.join(CSRC, "tab_api.cpp"), os.path.join(CSRC, "host_ops.cpp"), os.path.join(ROOT, "include", "tab_b200.h"), os.path.join(ROOT, "Setup_CUDA.py")]
+    mp, hp = module_path(), host_module_path()
+    if not force and mp and hp and not _stale(mp, deps) and not _stale(hp, deps):
         return mp
     r = subprocess.run([sys.executable, "Setup_CUDA.py", "build_ext", "--inplace"], cwd=ROOT, capture_output=True, text=True)
     if r.returncode != 0:

@@ -1,0 +1,130 @@
+// tab_b200._host: the bodies of tab_b200.ops' operators - checks, output and scratch allocation, one C-ABI call - in native code.
+//
+// A small convolution takes the device less time than the interpreter needs to check sixteen arguments, allocate two tensors
+// and convert twenty values for a foreign call (about 20 us); here that is 2-3 us.  Every function returns None for arguments
+// that are anything but plainly valid (wrong device, dtype, size; an empty result; an error code of the C ABI): the caller
+// then runs its own body, which names what is wrong or does the rare case, so that there is one set of messages.
+#include <torch/extension.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <c10/cuda/CUDAGuard.h>
+#include "../../include/tab_b200.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = c10::optional<Tensor>;
+
+bool plain(const Tensor& t, at::ScalarType dtype) { return t.defined() && t.is_cuda() && t.is_contiguous() && t.scalar_type() == dtype; }
+tab_stream_t stream_of(const Tensor& t) { return reinterpret_cast<tab_stream_t>(at::cuda::getCurrentCUDAStream(t.get_device()).stream()); }
+Tensor make(const Tensor& like, at::IntArrayRef size, at::ScalarType dtype) { return at::empty(size, like.options().dtype(dtype)); }
+
+struct Conv {
+    int type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW;
+    int64_t OH = 0, OW = 0, PC = 0;
+    // Valid sizes with a result that is not empty.
+    bool good() {
+        if (type < 0 || type > 3 || N < 1 || H < 1 || W < 1 || C < 1 || KN < 1 || KH < 1 || KW < 1 || p1 < 0 || p2 < 0 || s1 < 1 || s2 < 1) return false;
+        OH = ((int64_t)H + 2 * (int64_t)p1 - KH + 1) / s1;
+        OW = ((int64_t)W + 2 * (int64_t)p2 - KW + 1) / s2;
+        PC = ((int64_t)C + 63) / 64;
+        return OH > 0 && OW > 0;
+    }
+    int64_t weight_words() const { return (int64_t)KN * KH * KW * PC; }
+    int64_t pixels() const { return (int64_t)N * H * W; }
+};
+
+py::object quantize(const Tensor& X, const Tensor& ths, int bitwidth, int N, int H, int W, int C) {
+    Tensor QX, BTN;
+    {
+        py::gil_scoped_release nogil;
+        if (plain(X, at::kFloat) && plain(ths, at::kFloat) && N >= 1 && H >= 1 && W >= 1 && C >= 1 && bitwidth >= 1 &&
+            X.numel() == (int64_t)N * H * W * C && ths.numel() == N) {
+            const c10::cuda::CUDAGuard guard(X.device());
+            QX = make(X, {N, H, W, ((int64_t)C + 63) / 64, bitwidth == 1 ? 1 : 2}, at::kLong);
+            BTN = make(X, {N}, at::kInt);
+            if (tab_quantize_launch(X.data_ptr<float>(), ths.data_ptr<float>(), QX.data_ptr<int64_t>(), BTN.data_ptr<int32_t>(),
+                                    bitwidth, N, H, W, C, stream_of(X)) != TAB_OK) QX.reset();
+        }
+    }
+    if (!QX.defined()) return py::none();
+    py::list out(2);
+    out[0] = QX; out[1] = BTN;
+    return out;
+}
+
+py::object conv2d(const Tensor& X, const Tensor& QW, const Tensor& ths, const Tensor& btn, int type, int p1, int p2, int s1, int s2,
+                  int N, int H, int W, int C, int KN, int KH, int KW) {
+    Tensor Y;
+    {
+        py::gil_scoped_release nogil;
+        Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
+        if (g.good() && plain(X, at::kFloat) && plain(QW, at::kLong) && plain(ths, at::kFloat) && plain(btn, at::kInt) &&
+            QW.numel() == g.weight_words() * (type == 1 || type == 3 ? 1 : 2) && (type != 2 || btn.numel() == KN) &&
+            X.numel() == g.pixels() * C && ths.numel() == N) {
+            const c10::cuda::CUDAGuard guard(X.device());
+            Y = make(X, {N, KN, g.OH, g.OW}, at::kFloat);
+            const size_t bytes = tab_conv2d_workspace_bytes(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW);
+            Tensor ws = make(X, {(int64_t)std::max<size_t>(bytes, 256)}, at::kByte);
+            if (tab_conv2d_launch(X.data_ptr<float>(), QW.data_ptr<int64_t>(), ths.data_ptr<float>(), btn.data_ptr<int32_t>(), Y.data_ptr<float>(),
+                                  ws.data_ptr(), (size_t)ws.numel(), type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, stream_of(X)) != TAB_OK) Y.reset();
+        }
+    }
+    return Y.defined() ? py::cast(Y) : py::none();
+}
+
+// state: zeroed, of tab_conv2d_state_bytes(N) bytes.
+py::object quantize_auto(const Tensor& X, double scale, int bitwidth, int N, int H, int W, int C, const Tensor& state) {
+    Tensor QX, ths;
+    {
+        py::gil_scoped_release nogil;
+        if (plain(X, at::kFloat) && N >= 1 && H >= 1 && W >= 1 && C >= 1 && bitwidth >= 1 && X.numel() == (int64_t)N * H * W * C &&
+            state.defined() && state.is_cuda()) {
+            const c10::cuda::CUDAGuard guard(X.device());
+            QX = make(X, {N, H, W, ((int64_t)C + 63) / 64, bitwidth == 1 ? 1 : 2}, at::kLong);
+            ths = make(X, {N}, at::kFloat);
+            if (tab_quantize_auto_launch(X.data_ptr<float>(), (float)scale, state.data_ptr(), ths.data_ptr<float>(), QX.data_ptr<int64_t>(), bitwidth,
+                                         N, H, W, C, stream_of(X)) != TAB_OK) QX.reset();
+        }
+    }
+    if (!QX.defined()) return py::none();
+    return py::make_tuple(QX, ths);
+}
+
+// The GEMM stage on 4-bit weights (ops.conv2d_bits with uint8 weights).
+py::object conv2d_packed4(const Tensor& QX, const Tensor& W4, int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW,
+                          const OptTensor& residual, c10::optional<double> threshold_scale, const OptTensor& state, bool out_int16,
+                          c10::optional<int> next_bitwidth) {
+    Tensor Y, nxt, QN;
+    {
+        py::gil_scoped_release nogil;
+        Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
+        const bool want = threshold_scale.has_value();
+        if (g.good() && plain(QX, at::kLong) && plain(W4, at::kByte) && QX.numel() == g.pixels() * g.PC * (type == 2 || type == 3 ? 1 : 2) &&
+            W4.numel() == g.weight_words() * 32 && !(out_int16 && residual.has_value()) &&
+            (!residual.has_value() || (plain(*residual, at::kFloat) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
+            (!want || (state.has_value() && state->defined() && state->is_cuda())) && (!next_bitwidth.has_value() || want)) {
+            const c10::cuda::CUDAGuard guard(QX.device());
+            const int nb = next_bitwidth.has_value() ? (*next_bitwidth == 1 ? 1 : 2) : 0;
+            Y = make(QX, {N, KN, g.OH, g.OW}, out_int16 ? at::kShort : at::kFloat);
+            if (want) nxt = make(QX, {N}, at::kFloat);
+            if (nb) QN = make(QX, {N, g.OH, g.OW, ((int64_t)KN + 63) / 64, nb}, at::kLong);
+            if (tab_conv2d_packed4_launch(QX.data_ptr<int64_t>(), W4.data_ptr<uint8_t>(), Y.data_ptr(), out_int16 ? 1 : 0, type, p1, p2, s1, s2,
+                                          N, H, W, C, KN, KH, KW, residual.has_value() ? residual->data_ptr<float>() : nullptr,
+                                          want ? state->data_ptr() : nullptr, want ? nxt.data_ptr<float>() : nullptr,
+                                          want ? (float)*threshold_scale : 0.f, nb ? QN.data_ptr<int64_t>() : nullptr, nb, stream_of(QX)) != TAB_OK) Y.reset();
+        }
+    }
+    if (!Y.defined()) return py::none();
+    py::object th = nxt.defined() ? py::cast(nxt) : py::none();
+    if (QN.defined()) return py::make_tuple(Y, th, QN);
+    return py::make_tuple(Y, th);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.def("quantize", &quantize);
+    m.def("conv2d", &conv2d);
+    m.def("quantize_auto", &quantize_auto);
+    m.def("conv2d_packed4", &conv2d_packed4);
+}

@@ -18,9 +18,13 @@ Results are those of ``Conv2d`` bit for bit.  Inference only: there is no backwa
 """
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from . import _cabi, ops
+
+_state_bytes = functools.lru_cache(maxsize=256)(lambda N: _cabi.lib().tab_conv2d_state_bytes(N))
 
 TYPE_NAMES = {0: "TNN", 1: "TBN", 2: "BTN", 3: "BNN"}
 
@@ -97,9 +101,10 @@ class TABConv2d(torch.nn.Module):
 
     def state(self, N, device):
         """The zeroed state block ``conv_bits`` needs for thresholds; kept, every call leaves it zeroed."""
-        if self._state is None or self._state.numel() < _cabi.lib().tab_conv2d_state_bytes(int(N)) or self._state.device != device:
-            self._state = ops.new_state(N, device)
-        return self._state
+        state = self._state
+        if state is None or state.numel() < _state_bytes(int(N)) or state.device != device:
+            state = self._state = ops.new_state(N, device)
+        return state
 
     # ---- the two stages -----------------------------------------------------------------------------------------
     def quantize(self, x, thresholds=None):

@@ -13,6 +13,35 @@ import torch
 from . import _cabi
 
 
+_native = None
+
+
+def _host():
+    """``tab_b200._host``, the same bodies in native code (a call costs the host microseconds there and tens of them here), or
+    ``False`` when only the C-ABI library has been built.  Its functions return ``None`` for anything they do not take - the
+    bodies below then run, and say what is wrong."""
+    global _native
+    if _native is None:
+        try:
+            from . import _host as module
+        except ImportError:
+            module = False
+        _native = module
+    return _native
+
+
+def _try(name, *args):
+    """Result of the native function, or ``None``.  A ``TypeError`` means a value the binding does not take as it is (a float
+    where an integer is expected, ...): the Python body converts or refuses it."""
+    host = _host()
+    if not host:
+        return None
+    try:
+        return getattr(host, name)(*args)
+    except TypeError:
+        return None
+
+
 def _check_input(t: torch.Tensor, name: str, dtype: torch.dtype) -> None:
     if not isinstance(t, torch.Tensor) or not t.is_cuda:
         raise RuntimeError("%s must be a CUDA tensor" % name)
@@ -36,6 +65,9 @@ def Quantize(X, thresholds, bitwidth, N, H, W, C):
 
     ``QX`` int64 ``{N,H,W,ceil(C/64),bits}``; ``BTN_W`` int32 ``{N}`` (zeros when ``bitwidth == 1``).
     """
+    done = _try("quantize", X, thresholds, bitwidth, N, H, W, C)
+    if done is not None:
+        return done
     _check_input(X, "X", torch.float32)
     _check_input(thresholds, "thresholds", torch.float32)
     N, H, W, C, bitwidth = int(N), int(H), int(W), int(C), int(bitwidth)
@@ -73,6 +105,9 @@ def _conv_checks(conv_type, QW, btn, N, H, W, C, KN, KH, KW, p1, p2, s1, s2):
 def Conv2d(X, QW, thresholds, btn, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW):
     """``TAB_Conv2d`` (``TAB_GPU.cpp:34-42``): float32 tensor of shape ``{N,KN,OH,OW}`` whose buffer is in
     ``[N][OH][OW][KN]`` order (``TAB_GEMM.cu:509,526``)."""
+    done = _try("conv2d", X, QW, thresholds, btn, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW)
+    if done is not None:
+        return done
     _check_input(X, "X", torch.float32)
     _check_input(QW, "QW", torch.int64)
     _check_input(thresholds, "thresholds", torch.float32)
@@ -186,6 +221,10 @@ def new_state(N, device):
 def quantize_auto(X, scale, bitwidth, N, H, W, C, state=None):
     """``Quantize`` with the thresholds computed on the way: ``thresholds[n] = scale * mean|X[n]|``.  One launch (sums, a
     grid-wide meeting point, quantisation).  Returns ``(QX, thresholds)``.  ``state``: a block from ``new_state(N, device)`` to reuse (zero before and after)."""
+    if state is not None:
+        done = _try("quantize_auto", X, scale, bitwidth, N, H, W, C, state)
+        if done is not None:
+            return done
     _check_input(X, "X", torch.float32)
     N, H, W, C = int(N), int(H), int(W), int(C)
     if X.numel() != N * H * W * C:
@@ -228,6 +267,11 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
     launch also quantises ``Y`` against the next thresholds at that bitwidth and a third value is returned, ``QX`` of the
     next convolution (``[N,OH,OW,ceil(KN/64),bits]`` int64, what ``Quantize(Y, next_thresholds, ...)`` gives).
     Raises ``TabError`` (TAB_E_TOO_LARGE) for shapes the tensor-core kernel does not cover."""
+    if isinstance(W8, torch.Tensor) and W8.dtype == torch.uint8:
+        done = _try("conv2d_packed4", QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW,
+                    residual, threshold_scale, state, out_int16, next_bitwidth)
+        if done is not None:
+            return done
     _check_input(QX, "QX", torch.int64)
     packed4 = isinstance(W8, torch.Tensor) and W8.dtype == torch.uint8
     _check_input(W8, "W8", torch.uint8 if packed4 else torch.int8)

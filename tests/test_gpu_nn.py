@@ -85,3 +85,58 @@ def test_prepared_chain_matches_oracle(cuda, t):
             assert (oh, ow, kn) == (7, 7, 512)
             assert np.array_equal(yd.cpu().numpy().reshape(-1), np.asarray(yo).reshape(-1)), (compact, fused_quant)
     assert _cabi.lib().tab_device_status() == 0
+
+
+def test_native_bodies_equal_the_python_ones(cuda):
+    """``tab_b200._host`` against the Python bodies of the same operators, including what it leaves to them (sizes that are no
+    plain integers, empty results, arguments that are refused)."""
+    from tab_b200 import ops
+    assert ops._host(), "tab_b200._host has not been built"
+
+    def both(fn):
+        native = fn()
+        saved, ops._native = ops._native, False
+        try:
+            python = fn()
+        finally:
+            ops._native = saved
+        flat = lambda r: [r] if isinstance(r, torch.Tensor) else list(r)
+        a, b = flat(native), flat(python)
+        assert type(native) is type(python) and len(a) == len(b)
+        for u, v in zip(a, b):
+            assert (u is None and v is None) or (u.dtype == v.dtype and u.shape == v.shape and u.device == v.device and torch.equal(u, v))
+        return native
+
+    N, H, W, C, KN, K = 3, 9, 8, 130, 70, 3
+    x, ths = make_input(1, N, H, W, C)
+    w, wths = make_input(2, KN, K, K, C)
+    xd, td, wd, wtd = (torch.from_numpy(a).to(cuda) for a in (x, ths, w, wths))
+    state = ops.new_state(N, cuda)
+    for t in range(4):
+        QW, btn = both(lambda: ops.Quantize(wd, wtd, O.weight_bits(t), KN, K, K, C))
+        for geom in ((1, 1, 1, 1, N, H, W, C, KN, K, K), (0, 2, 2, 1, np.int64(N), H, float(W), C, KN, K, K)):
+            both(lambda: ops.Conv2d(xd, QW, td, btn, t, *geom))
+        QX, _ = both(lambda: ops.quantize_auto(xd, 0.7, O.act_bits(t), N, H, W, C, state))
+        W4 = ops.pack_weights(ops.expand_weights(QW, O.weight_bits(t), KN, K, K, C), KN, K, K, C)
+        g = (1, 1, 1, 1, N, H, W, C, KN, K, K)
+        r = torch.randn(N, KN, H, W, device=cuda)
+        for kw in (dict(), dict(residual=r), dict(threshold_scale=0.7, state=state), dict(threshold_scale=0.7, state=state, out_int16=True, next_bitwidth=2),
+                   dict(residual=r, threshold_scale=0.7, state=state, next_bitwidth=1)):
+            both(lambda: ops.conv2d_bits(QX, W4, t, *g, **kw))
+    assert both(lambda: ops.Conv2d(xd, QW, td, btn, 3, 0, 0, 1, 1, N, H, W, C, KN, K, K)).numel() == N * KN * (H - 2) * (W - 2)
+    assert ops.Quantize(torch.empty(0, device=cuda), torch.empty(0, device=cuda), 2, 0, 4, 4, 64)[0].numel() == 0
+    with pytest.raises(RuntimeError, match="X has"):
+        ops.Quantize(xd, td, 2, N, H, W + 1, C)
+    with pytest.raises(RuntimeError, match="QX must have dtype"):
+        ops.conv2d_bits(xd, W4, 3, *g)
+
+
+def test_module_weights_follow_a_loaded_state(cuda):
+    """``load_state_dict`` replaces the weights, the 4-bit form among them; the state itself holds what it always held."""
+    N, H, W, C, KN = 2, 10, 9, 70, 40
+    x = torch.randn(N, H, W, C, device=cuda)
+    a = tab_nn.TABConv2d.from_float(torch.randn(KN, 3, 3, C, device=cuda), 0, 1, 1)
+    b = tab_nn.TABConv2d.from_float(torch.randn(KN, 3, 3, C, device=cuda), 0, 1, 1)
+    assert sorted(a.state_dict()) == ["BTN_W", "QW", "W8"] and not torch.equal(a(x), b(x))
+    b.load_state_dict(a.state_dict())
+    assert torch.equal(a(x), b(x))
