@@ -336,14 +336,19 @@ __device__ __forceinline__ void load_pair(const TcConvParams& p, RawPair& raw, i
     const int r = it >> two;
     if (r >= nrows) return;
     const int w0 = (it & two) * 2;
-    const uint32_t R = (uint32_t)(Rbase + r);
-    const uint32_t n = p.dVHW.div(R);
-    const uint32_t rem = R - n * (uint32_t)(p.VH * p.VW);
-    const uint32_t i = p.dVW.div(rem);
-    const uint32_t j = rem - i * (uint32_t)p.VW;
-    const int ih = (int)i * p.s1 + pa - p.p1, iw = (int)j * p.s2 + pb - p.p2;
-    if ((int)n >= p.N || (unsigned)ih >= (unsigned)p.H || (unsigned)iw >= (unsigned)p.W) return;
-    const long long widx = (((long long)n * p.H + ih) * p.W + iw) * p.PC + 4 * cq + w0;
+    uint32_t pix = (uint32_t)(Rbase + r);                                  // the grid is the image grid: a virtual row is a pixel
+    if (p.flat) {
+        if (pix >= (uint32_t)p.N * (uint32_t)(p.H * p.W)) return;
+    } else {
+        const uint32_t n = p.dVHW.div(pix);
+        const uint32_t rem = pix - n * (uint32_t)(p.VH * p.VW);
+        const uint32_t i = p.dVW.div(rem);
+        const uint32_t j = rem - i * (uint32_t)p.VW;
+        const int ih = (int)i * p.s1 + pa - p.p1, iw = (int)j * p.s2 + pb - p.p2;
+        if ((int)n >= p.N || (unsigned)ih >= (unsigned)p.H || (unsigned)iw >= (unsigned)p.W) return;
+        pix = (n * (uint32_t)p.H + (uint32_t)ih) * (uint32_t)p.W + (uint32_t)iw;   // N*H*W < 2^31 is checked on the host
+    }
+    const size_t widx = (size_t)pix * (uint32_t)p.PC + (uint32_t)(4 * cq + w0);
     const bool second = w0 + 1 < nw;
     if (p.abits == 2) {
         const ulonglong2* q = reinterpret_cast<const ulonglong2*>(p.qx + 2 * widx);
@@ -385,10 +390,14 @@ struct PatchIter {
 };
 
 // ---- epilogue ------------------------------------------------------------------------------------------------------------
-// tcgen05.ld hands lane r of a warp the 32 columns of accumulator row r; written straight out, one store instruction
-// would touch 32 different output rows.  The warp instead passes each 32x32 block through a private 4 KB shared-memory
-// buffer (16-byte chunks XOR-swizzled by row, so both directions are conflict-free) and stores it transposed: eight
-// lanes cover 128 contiguous bytes of one row, one instruction writes four full lines.  The residual is read the same way.
+// tcgen05.ld hands lane r of a warp 32 columns of accumulator row r.  Two ways out:
+//   16-bit results and layers with a residual whose rows start on 32-byte boundaries: lane r reads and writes its own row with 256-bit accesses - an instruction
+//     moves 32 whole 32-byte sectors, and no shared memory, no shuffles and few addresses are involved.  What bounds these
+//     epilogues is the instructions they issue (ncu: a 256 x 64 tile of a 3x3x64 layer took 8500 warp instructions, 0.39 a cycle
+//     and scheduler, more than half of them here).  ResNet-18-shaped network at batch 256: 1133 -> 1119 us.
+//   fp32 without a residual (KN % 4 == 0): bound by the stores; the warp transposes the block through shared memory so that every store is
+//     four whole lines.  Written row by row, 1x1 25088x1024x1024 took 71 us instead of 58, 3x3 64x56x56x64 29.3 instead of 27.6.
+// Other filter counts and partial blocks go through shared memory element by element (ragged_block).
 
 // |y| sums a warp has computed but not yet added to abs_sums: the global atomic is issued by the caller AFTER it has
 // released the accumulator buffer (an mbarrier arrive has release semantics and would otherwise wait for the atomic's
@@ -405,12 +414,9 @@ __device__ __forceinline__ void flush_pending(const TcConvParams& p, PendingSums
     ps.img0 = -1;
 }
 
-// Row data of a warp's 32-row slab (virtual rows Rw .. Rw + 31) in the transposed domain: lane (rsub = lane / 8,
-// chunk = lane % 8) handles rows 4i + rsub, i = 0..7, and four columns per row.  Computed before the accumulator
-// is waited for.
+// Row data of a warp's 32-row slab (virtual rows Rw .. Rw + 31).  Computed before the accumulator is waited for.
 struct SlabRows {
-    int mi[8];               // output row (index into [M][KN]) of row 4i + rsub, -1 = not an output position
-    int m_own;               // the same for row `lane` (the ragged path works row per lane)
+    int m_own;               // output row (index into [M][KN]) of row `lane`, -1 = not an output position
     int n_own;               // image of row `lane`
     int Rw, wimg0, split;    // first virtual row, its image, first slab row that belongs to the next image
     bool fast, slow;         // how |y| is summed, see slab_rows
@@ -432,8 +438,6 @@ __device__ __forceinline__ void slab_rows(const TcConvParams& p, int Rw, int lan
     const bool row_ok = n < p.N && oh < p.OH && ow < p.OW;
     sr.m_own = row_ok ? (n * p.OH + oh) * p.OW + ow : -1;                  // M < 2^31 is checked on the host
     sr.n_own = n;
-#pragma unroll
-    for (int i = 0; i < 8; i++) sr.mi[i] = __shfl_sync(0xFFFFFFFFu, sr.m_own, 4 * i + (lane >> 3));
     sr.Rw = Rw;
     sr.wimg0 = (int)p.dVHW.div((uint32_t)Rw);
     sr.split = (sr.wimg0 + 1) * VHW - Rw;
@@ -442,19 +446,24 @@ __device__ __forceinline__ void slab_rows(const TcConvParams& p, int Rw, int lan
     sr.slow = want_sum && !sr.fast;
 }
 
-// Streaming 128-bit load that leaves no line in L1 (the residual is read once).
-__device__ __forceinline__ float4 ld_stream_f4(const float4* ptr) {
-    float4 r;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(ptr));
-    return r;
+// 256-bit streaming load that leaves no line in L1 (the residual is read once), and store.
+__device__ __forceinline__ void ld_stream_8(const float* ptr, float* o) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=f"(o[0]), "=f"(o[1]), "=f"(o[2]), "=f"(o[3]), "=f"(o[4]), "=f"(o[5]), "=f"(o[6]), "=f"(o[7]) : "l"(ptr));
+}
+__device__ __forceinline__ void st_8(void* ptr, const uint32_t* o) {
+    asm volatile("st.global.v8.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8};" ::"l"(ptr), "r"(o[0]), "r"(o[1]), "r"(o[2]), "r"(o[3]),
+                 "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
 }
 
-// Residual values of the 32-column block at filter nbase, in the transposed layout (res[i] = row 4i + rsub, 4 columns).
-__device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const SlabRows& sr, int nbase, int lane, float4 (&res)[8]) {
+// Residual values of the lane's own row in the 32-column block at filter nbase.
+__device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const SlabRows& sr, int nbase, float (&res)[32]) {
 #pragma unroll
-    for (int i = 0; i < 8; i++) {
-        res[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (sr.mi[i] >= 0) res[i] = ld_stream_f4(reinterpret_cast<const float4*>(p.residual + (long long)sr.mi[i] * p.KN + nbase) + (lane & 7));
+    for (int i = 0; i < 32; i++) res[i] = 0.f;
+    if (sr.m_own >= 0) {
+        const float* row = p.residual + (long long)sr.m_own * p.KN + nbase;
+#pragma unroll
+        for (int q = 0; q < 4; q++) ld_stream_8(row + 8 * q, &res[8 * q]);
     }
 }
 
@@ -524,15 +533,13 @@ __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRo
 // E2M1: the accumulators are floats (integer-valued) instead of integers.
 template <int FUSED, bool E2M1>
 __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t taddr, const SlabRows& sr, int n0, int c0, int c1,
-                                             int lane, uint32_t stage, float4 (&res)[8], bool res_loaded, PendingSums& ps, bool down, uint32_t freed) {
-    const bool vec4 = (p.KN & 3) == 0;
-    const bool small_acc = p.Kw < (1 << 15);                               // |accumulator| <= 64 * Kw < 2^21: the bias conversion is exact
+                                             int lane, uint32_t stage, float (&res)[32], bool res_loaded, PendingSums& ps, bool down, uint32_t freed) {
     constexpr bool has_res = FUSED == 2;
+    const bool out16 = !has_res && p.y16 != nullptr;
+    const bool small_acc = p.Kw < (1 << 15);                               // |accumulator| <= 64 * Kw < 2^21: the bias conversion is exact
     const bool want_sum = FUSED && p.abs_sums != nullptr;
-    const int rsub = lane >> 3, chunk = lane & 7;
-    const int VHW = p.VH * p.VW;
-    unsigned isum_own = 0;                                                 // integer data: |y| total of the lane's own row
-    double dsum0 = 0.0, dsum1 = 0.0;                                       // float data: totals per image in the transposed domain
+    unsigned isum_own = 0;                                                 // whole numbers: |y| total of the lane's own row
+    double dsum0 = 0.0, dsum1 = 0.0;                                       // with a residual: totals per image
     if (n0 + c1 > p.KN) c1 = max(c0, (p.KN - n0 + 31) / 32 * 32);          // blocks without a real filter are left out
     if (E2M1 && freed != 0 && c0 >= c1 && lane == 0) mbar_arrive(freed);   // (this warp reads none)
     const int cstride = down ? -32 : 32;
@@ -548,157 +555,106 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
             if (lane == 0) mbar_arrive(freed);
             freed = 0;
         }
-        const int real = p.KN - nbase;                                     // filters of this block that exist (the others' accumulators are 0)
-        if (vec4 && real >= 32) {
-            // compact output whose rows start on 16-byte boundaries: the block is transposed as 16-bit values (half the
-            // shared-memory traffic; on the 64-filter layers that traffic, next to the MMAs' operand reads, is the bound)
-            const bool pack16 = !has_res && p.y16 != nullptr && (p.KN & 7) == 0;
-            if (E2M1 && !has_res && (sr.fast || p.y16 != nullptr)) {
-                // y is the accumulator itself.  |y| sums of the lane's own row: whole numbers below 2^23 add exactly in float
-                // (sr.fast bounds |y| by 2^18)
-                if (sr.fast) {
-                    float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
+        if (!has_res && want_sum) {                                        // y is the accumulator itself
+            unsigned row = 0;
+            if (E2M1 && sr.fast) {                                         // |y| < 2^18: 32 of them add exactly in float
+                float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
 #pragma unroll
-                    for (int j = 0; j < 32; j += 4) {
-                        f0 += fabsf(__uint_as_float(v[j])); f1 += fabsf(__uint_as_float(v[j + 1]));
-                        f2 += fabsf(__uint_as_float(v[j + 2])); f3 += fabsf(__uint_as_float(v[j + 3]));
-                    }
-                    isum_own += sr.m_own >= 0 ? __float2uint_rn((f0 + f1) + (f2 + f3)) : 0u;
+                for (int j = 0; j < 32; j += 4) {
+                    f0 += fabsf(__uint_as_float(v[j])); f1 += fabsf(__uint_as_float(v[j + 1]));
+                    f2 += fabsf(__uint_as_float(v[j + 2])); f3 += fabsf(__uint_as_float(v[j + 3]));
                 }
-                if (p.y16 != nullptr)                                      // the low 16 bits become the integer (|y| < 2^15)
+                row = __float2uint_rn((f0 + f1) + (f2 + f3));
+            } else {                                                       // |y| < 2^26: 32 of them fit 32 bits
+                unsigned r0 = 0, r1 = 0, r2 = 0, r3 = 0;                   // four independent |x| + acc chains (one SAD instruction each)
 #pragma unroll
-                    for (int j = 0; j < 32; j++) v[j] = __float_as_uint(__uint_as_float(v[j]) + 12582912.f);
+                for (int j = 0; j < 32; j += 4) {
+                    const int i0 = E2M1 ? __float2int_rn(__uint_as_float(v[j])) : (int)v[j], i1 = E2M1 ? __float2int_rn(__uint_as_float(v[j + 1])) : (int)v[j + 1];
+                    const int i2 = E2M1 ? __float2int_rn(__uint_as_float(v[j + 2])) : (int)v[j + 2], i3 = E2M1 ? __float2int_rn(__uint_as_float(v[j + 3])) : (int)v[j + 3];
+                    r0 = __sad(i0, 0, r0); r1 = __sad(i1, 0, r1); r2 = __sad(i2, 0, r2); r3 = __sad(i3, 0, r3);
+                }
+                row = (r0 + r1) + (r2 + r3);
             }
-            if (pack16) {
+            if (sr.m_own >= 0) {
+                if (sr.fast) isum_own += row;
+                else if (sr.n_own < p.N && row) atomicAdd(p.abs_sums + sr.n_own, (double)row);
+            }
+        }
+        if ((has_res || out16 ? p.wide : (p.KN & 3) == 0) && nbase + 32 <= p.KN) {
+            if (out16) {
+                uint32_t h[16];
 #pragma unroll
-                for (int q = 0; q < 4; q++)                                // row `lane`: 64 bytes, 16-byte chunk q at (q ^ (lane / 2 % 4))
-                    sts_v4(stage + lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4), __byte_perm(v[8 * q], v[8 * q + 1], 0x5410), __byte_perm(v[8 * q + 2], v[8 * q + 3], 0x5410),
-                           __byte_perm(v[8 * q + 4], v[8 * q + 5], 0x5410), __byte_perm(v[8 * q + 6], v[8 * q + 7], 0x5410));
-            } else {
+                for (int j = 0; j < 16; j++) {                             // float + 1.5 * 2^23: the low 16 bits are the integer (|y| < 2^15)
+                    const uint32_t lo = E2M1 ? __float_as_uint(__uint_as_float(v[2 * j]) + 12582912.f) : v[2 * j];
+                    const uint32_t hi = E2M1 ? __float_as_uint(__uint_as_float(v[2 * j + 1]) + 12582912.f) : v[2 * j + 1];
+                    h[j] = __byte_perm(lo, hi, 0x5410);
+                }
+                if (sr.m_own >= 0) {
+                    int16_t* row = p.y16 + (long long)sr.m_own * p.KN + nbase;
+                    st_8(row, h); st_8(row + 16, h + 8);
+                }
+                continue;
+            }
+            auto value = [&](uint32_t acc) -> float {
+                if (E2M1) return __uint_as_float(acc) + 0.f;               // + 0: a sum of products of zeros may be -0
+                return small_acc ? __int_as_float((int)acc + 0x4B400000) - 12582912.f : (float)(int)acc;   // the 1.5 * 2^23 bias, no I2F
+            };
+            if constexpr (!has_res) {                                      // transposed: eight lanes write 128 bytes of a row
 #pragma unroll
                 for (int q = 0; q < 8; q++)
                     sts_v4(stage + lane * 128 + ((q ^ (lane & 7)) << 4), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            }
-            if (!E2M1 && sr.fast && !has_res) {                            // y is the accumulator itself: sum |acc| of the lane's own row
-                unsigned r0 = 0, r1 = 0, r2 = 0, r3 = 0;                   // (row `lane` of the slab), in integers, before the transposition;
-#pragma unroll                                                             // four independent |x| + acc chains (one SAD instruction each)
-                for (int j = 0; j < 32; j += 4) {
-                    r0 = __sad((int)v[j], 0, r0); r1 = __sad((int)v[j + 1], 0, r1);
-                    r2 = __sad((int)v[j + 2], 0, r2); r3 = __sad((int)v[j + 3], 0, r3);
-                }
-                isum_own += sr.m_own >= 0 ? (r0 + r1) + (r2 + r3) : 0u;
-            }
-            if (has_res && !res_loaded) slab_load_residual(p, sr, nbase, lane, res);
-            __syncwarp();
-            if (pack16) {                                                  // four lanes store the 64 bytes of a row, eight rows per instruction
+                __syncwarp();
+                float* base = p.y + nbase + 4 * (lane & 7);
+                int4 raw[8];
+                int m[8];
 #pragma unroll
-                for (int i = 0; i < 4; i++) {
-                    const int r = 8 * i + (lane >> 2), c = lane & 3;
-                    const int4 raw = lds_v4(stage + r * 64 + ((c ^ ((r >> 1) & 3)) << 4));
-                    const int m = __shfl_sync(0xFFFFFFFFu, sr.m_own, r);
-                    if (m >= 0) {
-                        reinterpret_cast<int4*>(p.y16 + (long long)m * p.KN + nbase)[c] = raw;
-                        if (sr.slow) {
-                            const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
-                            const int q4[4] = {raw.x, raw.y, raw.z, raw.w};
-                            int tot = 0;
-#pragma unroll
-                            for (int j = 0; j < 4; j++) tot += abs((int)(int16_t)(q4[j] & 0xFFFF)) + abs(q4[j] >> 16);
-                            if (img < p.N) atomicAdd(p.abs_sums + img, (double)tot);
-                        }
-                    }
+                for (int i = 0; i < 8; i++) {                              // all reads before the first store: a store would wait for its own read
+                    const int r = 4 * i + (lane >> 3);
+                    raw[i] = lds_v4(stage + r * 128 + (((lane & 7) ^ (r & 7)) << 4));
+                    m[i] = __shfl_sync(0xFFFFFFFFu, sr.m_own, r);
                 }
+#pragma unroll
+                for (int i = 0; i < 8; i++)
+                    if (m[i] >= 0) *reinterpret_cast<float4*>(base + (long long)m[i] * p.KN) = make_float4(value(raw[i].x), value(raw[i].y), value(raw[i].z), value(raw[i].w));
                 __syncwarp();
                 continue;
             }
-            if (!has_res && p.y16 != nullptr) {                            // compact output: the integers themselves, 16 bits each
+            if (has_res && !res_loaded) slab_load_residual(p, sr, nbase, res);
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int r = 4 * i + rsub;
-                    const int4 raw = lds_v4(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
-                    if (sr.mi[i] >= 0) {
-                        reinterpret_cast<uint2*>(p.y16 + (long long)sr.mi[i] * p.KN + nbase)[chunk] =
-                            make_uint2(__byte_perm((uint32_t)raw.x, (uint32_t)raw.y, 0x5410), __byte_perm((uint32_t)raw.z, (uint32_t)raw.w, 0x5410));
-                        if (sr.slow) {
-                            const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
-                            if (img < p.N) {
-                                const int a4[4] = {raw.x, raw.y, raw.z, raw.w};
-                                double tot = 0.0;
-#pragma unroll
-                                for (int j = 0; j < 4; j++) tot += (double)(E2M1 ? abs((int)(int16_t)(a4[j] & 0xFFFF)) : abs(a4[j]));
-                                atomicAdd(p.abs_sums + img, tot);
-                            }
-                        }
-                    }
-                }
-                __syncwarp();
-                continue;
+            for (int j = 0; j < 32; j++) {
+                const float o = value(v[j]);
+                v[j] = __float_as_uint(has_res ? o + res[j] : o);
             }
-            float4 o[8];
-#pragma unroll
-            for (int i = 0; i < 8; i++) {
-                const int r = 4 * i + rsub;
-                const int4 raw = lds_v4(stage + r * 128 + ((chunk ^ (r & 7)) << 4));
-                if (E2M1) {                                                // + 0: a sum of products of zeros may be -0
-                    o[i].x = __int_as_float(raw.x) + 0.f; o[i].y = __int_as_float(raw.y) + 0.f;
-                    o[i].z = __int_as_float(raw.z) + 0.f; o[i].w = __int_as_float(raw.w) + 0.f;
-                } else if (small_acc) {                                    // int -> float by the 1.5 * 2^23 bias, no I2F
-                    o[i].x = __int_as_float(raw.x + 0x4B400000) - 12582912.f; o[i].y = __int_as_float(raw.y + 0x4B400000) - 12582912.f;
-                    o[i].z = __int_as_float(raw.z + 0x4B400000) - 12582912.f; o[i].w = __int_as_float(raw.w + 0x4B400000) - 12582912.f;
-                } else {
-                    o[i].x = (float)raw.x; o[i].y = (float)raw.y; o[i].z = (float)raw.z; o[i].w = (float)raw.w;
-                }
-            }
-            if (has_res) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) { o[i].x += res[i].x; o[i].y += res[i].y; o[i].z += res[i].z; o[i].w += res[i].w; }
-                // the next block's residual, in flight while this block is stored and summed
+            if (has_res) {                                                 // the next block's residual, in flight while this block is stored and summed
                 res_loaded = left > 1 && nbase + cstride + 32 <= p.KN;
-                if (res_loaded) slab_load_residual(p, sr, nbase + cstride, lane, res);
+                if (res_loaded) slab_load_residual(p, sr, nbase + cstride, res);
             }
+            if (sr.m_own >= 0) {
+                float* row = p.y + (long long)sr.m_own * p.KN + nbase;
 #pragma unroll
-            for (int i = 0; i < 8; i++)
-                if (sr.mi[i] >= 0) reinterpret_cast<float4*>(p.y + (long long)sr.mi[i] * p.KN + nbase)[chunk] = o[i];
-            if (sr.fast && has_res) {
-                // the residual need not be integer-valued: compensated (Kahan) float sums, two chains per image, whose value
-                // and compensation go to the double totals (good to about 1e-14 of the total)
-                float sa0 = 0.f, sa1 = 0.f, ca0 = 0.f, ca1 = 0.f, sb0 = 0.f, sb1 = 0.f, cb0 = 0.f, cb1 = 0.f;
-                auto kahan = [](float x, float& sv, float& cv) { const float yv = x - cv, tv = sv + yv; cv = (tv - sv) - yv; sv = tv; };
+                for (int q = 0; q < 4; q++) st_8(row + 8 * q, v + 8 * q);
+                if (has_res && want_sum) {
+                    // the residual need not be integer-valued: compensated (Kahan) float sums, four chains, whose value and
+                    // compensation go to the double totals (good to about 1e-14 of the total)
+                    float s4[4] = {0.f, 0.f, 0.f, 0.f}, c4[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    if (sr.mi[i] < 0) continue;
-                    if (4 * i + rsub < sr.split) {
-                        kahan(fabsf(o[i].x), sa0, ca0); kahan(fabsf(o[i].y), sa1, ca1); kahan(fabsf(o[i].z), sa0, ca0); kahan(fabsf(o[i].w), sa1, ca1);
-                    } else {
-                        kahan(fabsf(o[i].x), sb0, cb0); kahan(fabsf(o[i].y), sb1, cb1); kahan(fabsf(o[i].z), sb0, cb0); kahan(fabsf(o[i].w), sb1, cb1);
+                    for (int j = 0; j < 32; j++) {
+                        const int k = j & 3;
+                        const float yv = fabsf(__uint_as_float(v[j])) - c4[k], tv = s4[k] + yv;
+                        c4[k] = (tv - s4[k]) - yv;
+                        s4[k] = tv;
                     }
-                }
-                dsum0 += ((double)sa0 + (double)sa1) - ((double)ca0 + (double)ca1);
-                dsum1 += ((double)sb0 + (double)sb1) - ((double)cb0 + (double)cb1);
-            } else if (sr.slow) {
-#pragma unroll
-                for (int i = 0; i < 8; i++) {
-                    const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + 4 * i + rsub));
-                    if (sr.mi[i] >= 0 && img < p.N)
-                        atomicAdd(p.abs_sums + img, ((double)fabsf(o[i].x) + (double)fabsf(o[i].y)) + ((double)fabsf(o[i].z) + (double)fabsf(o[i].w)));
+                    const double a = (((double)s4[0] + (double)s4[1]) + ((double)s4[2] + (double)s4[3])) - (((double)c4[0] + (double)c4[1]) + ((double)c4[2] + (double)c4[3]));
+                    if (!sr.fast) { if (sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, a); }
+                    else if (lane < sr.split) dsum0 += a;
+                    else dsum1 += a;
                 }
             }
-            __syncwarp();
-        } else {                                                           // KN is no multiple of four, or a partial last block
+        } else {                                                           // rows that start anywhere, or a partial last block
             res_loaded = false;
 #pragma unroll
             for (int q = 0; q < 8; q++)
                 sts_v4(stage + lane * 128 + ((q ^ (lane & 7)) << 4), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
-            if (!has_res && want_sum && sr.m_own >= 0) {
-                unsigned r0 = 0, r1 = 0;
-#pragma unroll
-                for (int j = 0; j < 32; j += 2) {
-                    r0 = __sad(E2M1 ? __float2int_rn(__uint_as_float(v[j])) : (int)v[j], 0, r0);
-                    r1 = __sad(E2M1 ? __float2int_rn(__uint_as_float(v[j + 1])) : (int)v[j + 1], 0, r1);
-                }
-                if (sr.fast) isum_own += r0 + r1;
-                else if (sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, (double)r0 + (double)r1);
-            }
             __syncwarp();
             if (p.KN & 1) ragged_block<FUSED, 1, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
             else ragged_block<FUSED, 2, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
@@ -720,7 +676,6 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
         }
         ps.img0 = sr.wimg0;
     }
-    (void)VHW;
 }
 
 // ---- epilogue through TMA (TEPI) ---------------------------------------------------------------------------------------
@@ -809,8 +764,12 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     static_assert(SB <= 8, "eight ring barriers are laid out");
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
-    const uint32_t sbase = (raw + 1023u) & ~1023u;
-    unsigned char* smem = smem_raw + (sbase - raw);
+    const uint32_t sbase = raw;
+    unsigned char* smem = smem_raw;
+    if (raw & 1023u) {                                                     // never: see plan_shape
+        if (threadIdx.x == 0 && status) atomicExch(status, 19);
+        return;
+    }
     const uint32_t sPatch = sbase;                                         // [2][prow][128 B], prow % 8 == 0
     const uint32_t sRing = sbase + 2 * prow * IROW;                        // [nst][brows][128 B]
     const int tail = 2 * prow * IROW + nst * bstage;
@@ -891,22 +850,22 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         if constexpr (E2M1) {
             // The patches as one sequence of chunks of one item per thread.  Three chunks are loaded ahead, in registers that
             // are named and not rotated: a move of a register whose load is in flight would wait for it.
-            struct At { int t, cp, pl, base; };
+            struct At { int t, cp, pl, base, R0; };
             auto items_of = [&](int cp) { return nrows << (p.PC - 4 * cp > 2 ? 1 : 0); };
             auto advance = [&](At& a) {
                 a.base += NX;
                 if (a.base >= items_of(a.cp)) {
                     a.base = 0;
-                    if (++a.pl == planes) { a.pl = 0; if (++a.cp == ncp) { a.cp = 0; a.t += step; } }
+                    if (++a.pl == planes) { a.pl = 0; if (++a.cp == ncp) { a.cp = 0; a.t += step; a.R0 = tile_row0(a.t); } }
                 }
             };
             auto fetch = [&](RawPair& into, At& a) {
                 if (a.t >= ntiles) return;
                 const int pa = UNIT ? 0 : a.pl / PB;
-                load_pair(p, into, tile_row0(a.t), nrows, a.cp, pa, UNIT ? 0 : a.pl - pa * PB, a.base + xt);
+                load_pair(p, into, a.R0, nrows, a.cp, pa, UNIT ? 0 : a.pl - pa * PB, a.base + xt);
                 advance(a);
             };
-            At at = {cta0, 0, 0, 0}, ahead = at;
+            At at = {cta0, 0, 0, 0, tile_row0(cta0)}, ahead = at;
             auto stage = [&](const RawPair& mine) -> bool {
                 if (at.t >= ntiles || dead) return false;
                 const unsigned pb = q & 1;
@@ -1334,14 +1293,14 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             const int ec0 = MT == 2 || wg == 0 ? 0 : chalf, ec1 = MT == 2 || wg == 1 ? wcols : chalf;
             SlabRows sr;
             slab_rows<FUSED>(p, R0 + emb * UTM + (warp & 3) * 32, lane, sr);
-            float4 res[8];
+            float res[32];
             bool res_loaded = false;
             // the warp that reads the columns which overlap the other accumulator begins with them
             const bool first_in_line = E2M1 && overlap && wg == (buf ? 0 : 1), down = first_in_line && buf == 0;
             const int clast = n0 + ec1 <= p.KN ? ec1 : ec0 + max(0, (p.KN - n0 - ec0 + 31) / 32 * 32);     // end of the blocks with real filters
             const int cfirst = down ? clast - 32 : ec0;
-            if (FUSED == 2 && (p.KN & 3) == 0 && ec0 < clast && n0 + cfirst + 32 <= p.KN) {
-                slab_load_residual(p, sr, n0 + cfirst, lane, res);
+            if (FUSED == 2 && p.wide && ec0 < clast && n0 + cfirst + 32 <= p.KN) {
+                slab_load_residual(p, sr, n0 + cfirst, res);
                 res_loaded = true;
             }
             if (!mbar_wait_prof<6, PAIR>(prof_on, accFull + 8 * buf, (a >> 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 16); *deadp = 1; } break; }
@@ -1552,7 +1511,10 @@ static long long split_point(long long ntiles, int sms, bool capable) {
 static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, TcPlan* out, bool pair = false) {
     const long long halo = (long long)((p.KH - 1) / p.s1) * p.VW + (p.KW - 1) / p.s2;
     const long long nrows = 128LL * mt + halo, prow = (nrows + 7) / 8 * 8;
-    const long long fixed = 2 * prow * IROW + 1024 + 8 * (p.tepi ? 8192 : 4096) + 1024;   // patches, barriers, epilogue buffers, alignment
+    // patches, barriers, epilogue buffers (none where every block leaves straight from registers).  Dynamic shared memory starts
+    // on a 1024-byte boundary (no static shared memory in the kernel); the kernel checks that.
+    const bool staged = !(p.wide && p.KN % 32 == 0 && (p.residual || p.y16));
+    const long long fixed = 2 * prow * IROW + 1024 + 8 * (p.tepi ? 8192 : (staged ? 4096 : 0));
     const int tlog = resident_taps_log2(p.PC, p.e2m1 != 0), wpr = p.e2m1 ? 4 : 2;
     const long long taps = (long long)p.KH * p.KW;
     const long long nres = tlog ? (taps + (1 << tlog) - 1) >> tlog : taps * ((p.PC + wpr - 1) / wpr);   // slots of resident filters
@@ -1633,6 +1595,8 @@ static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
     if ((long long)p.N * p.H * p.W >= (1LL << 31) || (long long)p.M >= (1LL << 31) - 512) return false;
     if ((long long)p.KH * p.KW * p.PC >= (1LL << 20)) return false;
     if (p.e2m1 && (long long)p.KH * p.KW * p.C >= (1LL << 24)) return false;       // sums the fp32 accumulators may not hold exactly
+    const void* out = p.y16 ? static_cast<const void*>(p.y16) : static_cast<const void*>(p.y);
+    p.wide = p.KN % (p.y16 ? 16 : 8) == 0 && !(reinterpret_cast<uintptr_t>(out) & 31) && !(reinterpret_cast<uintptr_t>(p.residual) & 31);
     const bool tepi_ok = (p.KN & 3) == 0 && !(reinterpret_cast<uintptr_t>(p.y) & 15) && !(reinterpret_cast<uintptr_t>(p.residual) & 15) &&
                          (long long)p.KN * p.OW * p.OH * 4 < (1LL << 40);
     bool tepi_pays = p.residual != nullptr && p.y16 == nullptr && p.KN <= 64 && (long long)p.KH * p.KW * p.C <= 1024;
@@ -1648,6 +1612,7 @@ static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
         set_virtual_grid(p, false);
         if (!grid_in_range(p) || !tc_plan(p, sms, pl)) return false;
     }
+    p.flat = p.s1 == 1 && p.s2 == 1 && p.p1 == 0 && p.p2 == 0 && p.VH == p.H && p.VW == p.W;
     p.dVHW = make_fastdiv((uint32_t)(p.VH * p.VW));
     p.dVW = make_fastdiv((uint32_t)p.VW);
     return true;

@@ -67,6 +67,8 @@ struct TcConvParams {
     int M, Kw;
     int abits;               // planes of the activations: 2 ternary, 1 binary
     int VH, VW, PA, PB;      // virtual grid of one plane; planes
+    int flat;                // stride 1, no padding: virtual row = pixel
+    int wide;                // rows of the result and of the residual start on 32-byte boundaries
     int tepi;                // the grid is aligned for the TMA epilogue: a 32-row slab is one box of the output tensor
     FastDiv dVHW, dVW;
     // Optional tail: the CTA that finishes last turns the sums into the next layer's thresholds,
