@@ -260,23 +260,28 @@ class ClockSampler:
 def step_algorithmic_bytes(n_images):
     """Bytes every launch of one step must move, summed: per convolution input its elements read (4 B each; 2 B where the
     producer handed it over as int16) and 2 bits/element written by the quantiser; per convolution those bit-planes read, the
-    byte weights read, the output written (4 B/element; 2 B for a block's first convolution, whose only reader is the next
-    quantiser) and, where a shortcut is added, 4 B/element of residual read; the input statistics pass reads x once."""
+    4-bit weights read, the output written (4 B/element; 2 B for a block's first convolution, whose only reader is the next
+    quantiser) and, where a shortcut is added, 4 B/element of residual read; the input statistics pass reads x once.  From the
+    first strided shortcut on block results and shortcuts of more than 2^23 elements are 2 B/element too."""
     from tab_b200 import chain
     total = 4 * n_images * H0 * W0 * C0
     h = H0
-    for b in chain.resnet18_blocks():
+    x_bytes, blocks = 4, chain.resnet18_blocks()
+    for i, b in enumerate(blocks):
         a, bb, sc = b.conv_a, b.conv_b, b.shortcut
         oh = (h + 2 * a.pad - a.K + 1) // a.stride
+        small = i >= 2 and n_images * oh * oh * a.KN > 1 << 23
+        short_bytes = x_bytes if sc is None else (2 if small else 4)
+        out_bytes = 2 if small and i + 1 < len(blocks) else 4
         x_el, y_el = n_images * h * h * a.C, n_images * oh * oh * a.KN
         bits_in, bits_mid = x_el // 4, y_el // 4
-        total += 4 * x_el + bits_in                                        # quantise x
-        total += bits_in + a.KN * 9 * a.C + 2 * y_el                       # conv_a, int16 out
+        total += x_bytes * x_el + bits_in                                        # quantise x
+        total += bits_in + a.KN * 9 * a.C // 2 + 2 * y_el                       # conv_a, int16 out
         if sc is not None:
-            total += bits_in + sc.KN * sc.C + 4 * y_el                     # shortcut on the same bit-planes
+            total += bits_in + sc.KN * sc.C // 2 + short_bytes * y_el                     # shortcut on the same bit-planes
         total += 2 * y_el + bits_mid                                       # quantise y1 (int16)
-        total += bits_mid + bb.KN * 9 * bb.C + 4 * y_el + 4 * y_el         # conv_b + residual
-        h = oh
+        total += bits_mid + bb.KN * 9 * bb.C // 2 + (short_bytes + out_bytes) * y_el         # conv_b + residual
+        h, x_bytes = oh, out_bytes
     return total
 
 
@@ -684,15 +689,16 @@ def main():
             btn = torch.empty(n_local, dtype=torch.int32, device=dev)
             geom = conv.geometry(n_local, ih, ih)
             chained = cs.K == 3                                             # the 3x3 convolutions feed thresholds, the shortcuts do not
-            compact = chained and not has_res                               # a block's first convolution hands int16 to the next quantiser
-            if compact:
-                y16 = torch.empty(n_local * oh * oh * cs.KN, dtype=torch.int16, device=dev)
-                ms_gemm = time_launch(lambda: _cabi.check(lib.tab_conv2d_bits_i16_launch(
-                    qx.data_ptr(), conv.W8.data_ptr(), y16.data_ptr(), CONV_TYPE, *geom, state.data_ptr(), nxt.data_ptr(), 0.7, stream), "bits16"))
-            else:
-                ms_gemm = time_launch(lambda: _cabi.check(lib.tab_conv2d_bits_launch(
-                    qx.data_ptr(), conv.W8.data_ptr(), yb.data_ptr(), CONV_TYPE, *geom, res.data_ptr() if has_res else None,
-                    state.data_ptr() if chained else None, nxt.data_ptr() if chained else None, 0.7, stream), "bits"))
+            # int16 as in the chain: a block's first convolution, and from the first strided shortcut on large shortcuts,
+            # residuals and block results (the last one excepted)
+            small = not cs.name.startswith("s1") and n_local * oh * oh * cs.KN > 1 << 23
+            res16 = has_res and small
+            compact = (chained and not has_res) or (small and cs.name != "s4b1.b")
+            y = torch.empty(n_local * oh * oh * cs.KN, dtype=torch.int16, device=dev) if compact else yb
+            res = res.to(torch.int16) if res16 else res
+            ms_gemm = time_launch(lambda: _cabi.check(lib.tab_conv2d_packed4_launch(
+                qx.data_ptr(), conv.W4.data_ptr(), y.data_ptr(), int(compact), CONV_TYPE, *geom, res.data_ptr() if has_res else None, int(res16),
+                state.data_ptr() if chained else None, nxt.data_ptr() if chained else None, 0.7, None, 0, stream), "packed4"))
             kernel = lib.tab_last_conv_kernel().decode()
             if has_res:                                                     # a block's second convolution quantises the first one's int16 output
                 x16 = torch.round(xin * 8).to(torch.int16)
@@ -704,7 +710,7 @@ def main():
             ms_popc = time_launch(lambda: _cabi.check(lib.tab_conv2d_packed_launch(qx.data_ptr(), conv.QW.data_ptr(), conv.BTN_W.data_ptr(), yb.data_ptr(),
                                                                                     CONV_TYPE, *geom, stream), "popc"))
             lops = 2 * n_local * oh * oh * cs.KN * cs.K * cs.K * cs.C
-            gemm_bytes = qx.numel() * 8 + conv.W8.numel() + (2 * yb.numel() if compact else 4 * yb.numel() * (2 if has_res else 1))
+            gemm_bytes = qx.numel() * 8 + conv.W4.numel() + y.numel() * y.element_size() + (res.numel() * res.element_size() if has_res else 0)
             quant_bytes = (2 if has_res else 4) * xin.numel() + qx.numel() * 8
             sums["gemm_ms"] += ms_gemm; sums["popc_ms"] += ms_popc; sums["ops"] += lops; sums["gemm_bytes"] += gemm_bytes
             if cs.K == 3:                                                   # the shortcut reuses conv_a's bit-planes: no quantiser launch of its own
@@ -759,17 +765,17 @@ def main():
         "traffic": (L1_TRAFFIC_PER_IMAGE * l1_images) if L1_TRAFFIC_PER_IMAGE else None,
         "traffic_note": "ncu dram bytes read + written of the step's largest launch (conv_umma_persist_kernel<2,64,6,1,2,1>, 56x56x64 -> 64 with "
                         "residual), captured at 64 images and scaled to this rank's %d images - a lower bound: at 64 images four fifths of the "
-                        "output were still in the L2 when the launch ended; its algorithmic bytes are %.1fe6 (bit-planes + byte weights + fp32 "
+                        "output were still in the L2 when the launch ended; its algorithmic bytes are %.1fe6 (bit-planes + 4-bit weights + fp32 "
                         "residual read + fp32 output)"
-                        % (l1_images, (l1_images * 56 * 56 * 16 + 64 * 9 * 64 + 8 * l1_images * 56 * 56 * 64) / 1e6),
+                        % (l1_images, (l1_images * 56 * 56 * 16 + 64 * 9 * 32 + 8 * l1_images * 56 * 56 * 64) / 1e6),
         "gemm_stage": {
-            "kernel": "conv_umma_persist_kernel (persistent tcgen05.mma kind::i8 on bit-plane activations), %d launches per step, each timed alone" % len(layer_rows),
-            "bound": "tensor", "achieved": gemm_achieved, "peak": umma_tops, "unit": "TOP/s",
-            "frac": (gemm_achieved / umma_tops) if gemm_achieved else None,
+            "kernel": "conv_umma_persist_kernel (persistent tcgen05.mma kind::mxf4 on bit-plane activations), %d launches per step, each timed alone" % len(layer_rows),
+            "bound": "tensor", "achieved": gemm_achieved, "peak": 2.0 * umma_tops, "unit": "TOP/s",
+            "frac": (gemm_achieved / (2.0 * umma_tops)) if gemm_achieved else None,
             "frac_of_2x_bf16_measured": (gemm_achieved / (2.0 * bf16_peak)) if gemm_achieved else None,
             "hbm_GBps": (sums["gemm_bytes"] / (sums["gemm_ms"] * 1e-3) / 1e9) if sums["gemm_ms"] else None,
             "avg_launch_ms": sums["gemm_ms"] / max(len(layer_rows), 1),
-            "peak_source": "measured in this run: tcgen05.mma kind::i8 128x256x32 issued back to back from shared memory on every SM (no copies, "
+            "peak_source": "twice the rate measured in this run of tcgen05.mma kind::i8 128x256x32 (kind::mxf4 does 128x256x64 in the same cycles) issued back to back from shared memory on every SM (no copies, "
                            "no epilogue); 2 x MEASURED_PEAKS.json bf16_tflops would be %.0f TOP/s (%s); s8 mma.sync ceiling measured in this run: %.0f TOP/s"
                            % (2.0 * bf16_peak, peak_src, imma_sync_tops)},
         "quantize_in_step": {
@@ -788,7 +794,7 @@ def main():
     dom = [r for r in layer_rows if r["layer"] in ("s1b0.b", "s1b1.b")]
     if dom:
         dom_ms = sum(r["gemm_ms"] for r in dom) / len(dom)
-        dom_bytes = l1_images * 56 * 56 * 16 + 64 * 9 * 64 + 8 * l1_images * 56 * 56 * 64
+        dom_bytes = l1_images * 56 * 56 * 16 + 64 * 9 * 32 + 8 * l1_images * 56 * 56 * 64
         roofline["dominant_kernel"] = {
             "kernel": dom[0]["gemm_kernel"], "launches_per_step": len(dom), "bound": "hbm",
             "algorithmic_bytes_per_launch": dom_bytes, "avg_launch_ms": dom_ms,

@@ -149,7 +149,9 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
     a block's first convolution and its strided shortcut read the same bit-planes (same input, same thresholds).
     ``compact_mid``: a block's first convolution hands its result to the second one's quantiser as int16 (it is
     integer-valued and nothing else reads it), half the bytes of fp32; the convolution objects must accept
-    ``conv_bits(..., out_int16=True)`` and int16 input to ``quantize``.
+    ``conv_bits(..., out_int16=True)`` and int16 input to ``quantize``.  With ``fused_quant`` the block results of the later
+    stages travel the same way where the objects have a true ``int16_residual`` (``conv_bits`` then gets the int16 residual
+    another one returned, together with ``out_int16``).
     ``fused_quant``: every convolution that feeds another one also hands it its quantised input
     (``conv_bits(..., next_bitwidth=bits) -> (Y, next_ths, next_QX)``; the objects need a ``conv_type``), so that only the
     chain's input is quantised by a launch of its own; ``qx0``: that quantised input, when the caller already has it
@@ -160,13 +162,23 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
         blocks = resnet18_blocks()
         act_bits = lambda conv: 1 if conv.conv_type in (2, 3) else 2
         qx = qx0 if qx0 is not None else convs[blocks[0].conv_a.name].quantize(x, ths)
+        bound = None                                           # of |x|, None while x need not be whole numbers
         for i, b in enumerate(blocks):
             a, bb, sc = convs[b.conv_a.name], convs[b.conv_b.name], (convs[b.shortcut.name] if b.shortcut else None)
+            # From the first strided shortcut on the block results are whole numbers too: conv + conv, conv + conv + conv, ...
+            # They travel as int16 as well while their largest possible magnitude fits and the tensor is large enough for its
+            # bytes to matter (above the size up to which a convolution quantises its own result; 8 images 267 us with fp32
+            # results and 275 with int16 ones, 256 images 1071 and 983).
+            terms = b.conv_b.K * b.conv_b.K * b.conv_b.C
+            short_bound = bound if sc is None else b.shortcut.K * b.shortcut.K * b.shortcut.C
+            bound = None if short_bound is None else short_bound + terms
+            small = compact_mid and bound is not None and bound <= 32767 and N * oh * ow * b.conv_b.KN > 1 << 23 and all(getattr(c, "int16_residual", False) for c in (bb, sc or bb))
             oh, ow = (h + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride, (w + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride
-            short = x if sc is None else sc.conv_bits(qx, N, h, w, None, None)[0]
+            short = x if sc is None else (sc.conv_bits(qx, N, h, w, None, None, out_int16=True) if small else sc.conv_bits(qx, N, h, w, None, None))[0]
             _, _, q1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, out_int16=compact_mid, next_bitwidth=act_bits(bb))
             if i + 1 < len(blocks):
-                x, ths, qx = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE, next_bitwidth=act_bits(convs[blocks[i + 1].conv_a.name]))
+                out = dict(out_int16=True) if small else {}
+                x, ths, qx = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE, next_bitwidth=act_bits(convs[blocks[i + 1].conv_a.name]), **out)
             else:
                 x, ths = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE)
             h, w = oh, ow

@@ -234,7 +234,7 @@ size_t tab_conv2d_state_bytes(int N) { return N < 0 ? 0 : round256((size_t)N * 8
 static int bits_impl(const int64_t* qx, const int8_t* w8, float* y, int16_t* y16, int type, int p1, int p2, int s1, int s2,
                      int N, int H, int W, int C, int KN, int KH, int KW,
                      const float* residual, void* state, float* next_ths, float next_scale, tab_stream_t stream,
-                     int64_t* next_qx = nullptr, int next_bits = 0, bool e2m1 = false) {
+                     int64_t* next_qx = nullptr, int next_bits = 0, bool e2m1 = false, const int16_t* residual16 = nullptr) {
     int rc = conv_args_ok(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW);
     if (rc != TAB_OK) return rc;
     const long long oh = ((long long)H + 2LL * p1 - KH + 1) / s1, ow = ((long long)W + 2LL * p2 - KW + 1) / s2;
@@ -249,12 +249,12 @@ static int bits_impl(const int64_t* qx, const int8_t* w8, float* y, int16_t* y16
         return TAB_OK;
     }
     if (!qx || !w8 || (!y && !y16)) return TAB_E_NULL_POINTER;
-    if (misaligned(qx, 15) || misaligned(w8, 15) || misaligned(y, 15) || misaligned(y16, 15) || misaligned(residual, 15) || misaligned(state, 7) ||
+    if (misaligned(qx, 15) || misaligned(w8, 15) || misaligned(y, 15) || misaligned(y16, 15) || misaligned(residual, 15) || misaligned(residual16, 15) || misaligned(state, 7) ||
         misaligned(next_ths, 3) || misaligned(next_qx, 7))
         return TAB_E_ALIGNMENT;
     if (y16 && (long long)KH * KW * C > 32767) return TAB_E_TOO_LARGE;   // |y| <= KH*KW*C must fit 16 bits
     TcConvParams p = tc_geometry(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, oh, ow);
-    p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = w8; p.e2m1 = e2m1 ? 1 : 0; p.y = y; p.y16 = y16; p.residual = residual;
+    p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = w8; p.e2m1 = e2m1 ? 1 : 0; p.y = y; p.y16 = y16; p.residual = residual; p.residual16 = residual16;
     if (next_ths) {
         p.abs_sums = reinterpret_cast<double*>(state);
         p.done_counter = reinterpret_cast<unsigned*>(reinterpret_cast<double*>(state) + N);
@@ -310,11 +310,12 @@ int tab_pack_weights_launch(const int8_t* w8, uint8_t* w4, int KN, int KH, int K
 
 int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int y_is_int16, int type, int p1, int p2, int s1, int s2,
                               int N, int H, int W, int C, int KN, int KH, int KW,
-                              const float* residual, void* state, float* next_ths, float next_scale,
+                              const void* residual, int residual_is_int16, void* state, float* next_ths, float next_scale,
                               int64_t* next_qx, int next_bitwidth, tab_stream_t stream) {
-    if (y_is_int16 && residual) return TAB_E_BAD_ARGUMENT;
+    if (y_is_int16 && residual && !residual_is_int16) return TAB_E_BAD_ARGUMENT;
     return bits_impl(qx, reinterpret_cast<const int8_t*>(w4), y_is_int16 ? nullptr : static_cast<float*>(y), y_is_int16 ? static_cast<int16_t*>(y) : nullptr,
-                     type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, residual, state, next_ths, next_scale, stream, next_qx, next_bitwidth, true);
+                     type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, residual_is_int16 ? nullptr : static_cast<const float*>(residual),
+                     state, next_ths, next_scale, stream, next_qx, next_bitwidth, true, residual_is_int16 ? static_cast<const int16_t*>(residual) : nullptr);
 }
 
 int tab_quantize_auto_launch(const float* x, float scale, void* state, float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C,

@@ -456,15 +456,23 @@ __device__ __forceinline__ void st_8(void* ptr, const uint32_t* o) {
                  "r"(o[4]), "r"(o[5]), "r"(o[6]), "r"(o[7]) : "memory");
 }
 
-// Residual values of the lane's own row in the 32-column block at filter nbase.
-__device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const SlabRows& sr, int nbase, float (&res)[32]) {
+// Residual values of the lane's own row in the 32-column block at filter nbase, as they lie in memory: floats, or (FUSED 3)
+// pairs of 16-bit integers.
+template <int FUSED> __host__ __device__ constexpr int res_regs() { return FUSED == 3 ? 16 : 32; }
+template <int FUSED>
+__device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const SlabRows& sr, int nbase, float (&res)[res_regs<FUSED>()]) {
 #pragma unroll
-    for (int i = 0; i < 32; i++) res[i] = 0.f;
+    for (int i = 0; i < res_regs<FUSED>(); i++) res[i] = 0.f;
     if (sr.m_own >= 0) {
-        const float* row = p.residual + (long long)sr.m_own * p.KN + nbase;
+        const long long at = (long long)sr.m_own * p.KN + nbase;
+        const float* row = FUSED == 3 ? reinterpret_cast<const float*>(p.residual16 + at) : p.residual + at;
 #pragma unroll
-        for (int q = 0; q < 4; q++) ld_stream_8(row + 8 * q, &res[8 * q]);
+        for (int q = 0; q < res_regs<FUSED>() / 8; q++) ld_stream_8(row + 8 * q, &res[8 * q]);
     }
+}
+// Integer j (0 or 1) of a pair of 16-bit integers as a float: the biased integer becomes the low mantissa bits of 2^23.
+__device__ __forceinline__ float i16_float(uint32_t pair, int j) {
+    return __uint_as_float(__byte_perm(pair ^ 0x80008000u, 0x4B000000u, j ? 0x7632 : 0x7610)) - 8421376.f;   // 2^23 + 2^15
 }
 
 // A 32x32 block of integers staged row by row (row r: 128 bytes, 16-byte chunks XOR-swizzled by r % 8), written out for filter
@@ -474,9 +482,20 @@ __device__ __forceinline__ void slab_load_residual(const TcConvParams& p, const 
 template <int FUSED, int W, bool E2M1>
 __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRows& sr, int nbase, int lane, uint32_t stage, double& dsum0, double& dsum1) {
     constexpr int LPR = 32 / W, BATCH = 4;                                 // lanes per row; rows in flight per lane
-    constexpr bool has_res = FUSED == 2;
+    constexpr bool has_res = FUSED >= 2;
     const int sub = lane / LPR, c = (lane % LPR) * W;
     const bool col_ok = nbase + c < p.KN;
+    // |y| of W values of block row r: floats, or integers in the low halves
+    auto add_sum = [&](int, int r, const int (&q)[W], bool ints) {
+        double a = 0.0;
+#pragma unroll
+        for (int k = 0; k < W; k++) a += ints ? (double)abs((int)(int16_t)(q[k] & 0xFFFF)) : (double)fabsf(__int_as_float(q[k]));
+        if (sr.fast) { if (r < sr.split) dsum0 += a; else dsum1 += a; }
+        else {
+            const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
+            if (img < p.N) atomicAdd(p.abs_sums + img, a);
+        }
+    };
 #pragma unroll 1
     for (int i0 = 0; i0 < LPR; i0 += BATCH) {
         int m[BATCH];
@@ -486,7 +505,10 @@ __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRo
             m[b] = __shfl_sync(0xFFFFFFFFu, sr.m_own, (i0 + b) * W + sub);
             if (!col_ok) m[b] = -1;
 #pragma unroll
-            for (int k = 0; k < W; k++) res[b][k] = has_res && m[b] >= 0 ? __ldg(p.residual + (long long)m[b] * p.KN + nbase + c + k) : 0.f;
+            for (int k = 0; k < W; k++) {
+                const long long at = (long long)m[b] * p.KN + nbase + c + k;
+                res[b][k] = !has_res || m[b] < 0 ? 0.f : (FUSED == 3 ? (float)__ldg(p.residual16 + at) : __ldg(p.residual + at));
+            }
         }
 #pragma unroll
         for (int b = 0; b < BATCH; b++) {
@@ -497,10 +519,11 @@ __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRo
             for (int k = 0; k < W; k++) raw[k] = lds_b32(at + 4 * k);
             if (m[b] < 0) continue;
             const long long e = (long long)m[b] * p.KN + nbase + c;
-            if (!has_res && p.y16 != nullptr) {
+            if (FUSED != 2 && p.y16 != nullptr) {
                 if (E2M1)
 #pragma unroll
-                    for (int k = 0; k < W; k++) raw[k] = __float_as_int(__int_as_float(raw[k]) + 12582912.f);   // low half: the integer
+                    for (int k = 0; k < W; k++) raw[k] = __float_as_int(__int_as_float(raw[k]) + res[b][k] + 12582912.f);   // low half: the integer
+                if (has_res && p.abs_sums != nullptr) add_sum(b, r, raw, true);
                 if (W == 2) *reinterpret_cast<uint32_t*>(p.y16 + e) = __byte_perm((uint32_t)raw[0], (uint32_t)raw[W - 1], 0x5410);
                 else p.y16[e] = (int16_t)raw[0];
                 continue;
@@ -511,14 +534,10 @@ __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRo
             if (W == 2) *reinterpret_cast<float2*>(p.y + e) = make_float2(o[0], o[W - 1]);
             else p.y[e] = o[0];
             if (has_res && p.abs_sums != nullptr) {
-                double a = 0.0;
+                int bits[W];
 #pragma unroll
-                for (int k = 0; k < W; k++) a += (double)fabsf(o[k]);
-                if (sr.fast) { if (r < sr.split) dsum0 += a; else dsum1 += a; }
-                else {
-                    const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
-                    if (img < p.N) atomicAdd(p.abs_sums + img, a);
-                }
+                for (int k = 0; k < W; k++) bits[k] = __float_as_int(o[k]);
+                add_sum(b, r, bits, false);
             }
         }
     }
@@ -533,9 +552,9 @@ __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRo
 // E2M1: the accumulators are floats (integer-valued) instead of integers.
 template <int FUSED, bool E2M1>
 __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t taddr, const SlabRows& sr, int n0, int c0, int c1,
-                                             int lane, uint32_t stage, float (&res)[32], bool res_loaded, PendingSums& ps, bool down, uint32_t freed) {
-    constexpr bool has_res = FUSED == 2;
-    const bool out16 = !has_res && p.y16 != nullptr;
+                                             int lane, uint32_t stage, float (&res)[res_regs<FUSED>()], bool res_loaded, PendingSums& ps, bool down, uint32_t freed) {
+    constexpr bool has_res = FUSED >= 2, res16 = FUSED == 3;
+    const bool out16 = FUSED != 2 && p.y16 != nullptr;
     const bool small_acc = p.Kw < (1 << 15);                               // |accumulator| <= 64 * Kw < 2^21: the bias conversion is exact
     const bool want_sum = FUSED && p.abs_sums != nullptr;
     unsigned isum_own = 0;                                                 // whole numbers: |y| total of the lane's own row
@@ -580,8 +599,8 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                 else if (sr.n_own < p.N && row) atomicAdd(p.abs_sums + sr.n_own, (double)row);
             }
         }
-        if ((has_res || out16 ? p.wide : (p.KN & 3) == 0) && nbase + 32 <= p.KN) {
-            if (out16) {
+        if ((has_res || out16 ? (bool)p.wide : (p.KN & 3) == 0) && nbase + 32 <= p.KN) {
+            if (!has_res && out16) {
                 uint32_t h[16];
 #pragma unroll
                 for (int j = 0; j < 16; j++) {                             // float + 1.5 * 2^23: the low 16 bits are the integer (|y| < 2^15)
@@ -619,21 +638,38 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                 __syncwarp();
                 continue;
             }
-            if (has_res && !res_loaded) slab_load_residual(p, sr, nbase, res);
+            if (has_res && !res_loaded) slab_load_residual<FUSED>(p, sr, nbase, res);
 #pragma unroll
             for (int j = 0; j < 32; j++) {
                 const float o = value(v[j]);
-                v[j] = __float_as_uint(has_res ? o + res[j] : o);
+                v[j] = __float_as_uint(o + (res16 ? i16_float(__float_as_uint(res[j >> 1]), j & 1) : res[res16 ? 0 : j]));
             }
             if (has_res) {                                                 // the next block's residual, in flight while this block is stored and summed
                 res_loaded = left > 1 && nbase + cstride + 32 <= p.KN;
-                if (res_loaded) slab_load_residual(p, sr, nbase + cstride, res);
+                if (res_loaded) slab_load_residual<FUSED>(p, sr, nbase + cstride, res);
             }
             if (sr.m_own >= 0) {
-                float* row = p.y + (long long)sr.m_own * p.KN + nbase;
+                const long long at = (long long)sr.m_own * p.KN + nbase;
+                if (res16 && out16) {
+                    uint32_t h[16];
 #pragma unroll
-                for (int q = 0; q < 4; q++) st_8(row + 8 * q, v + 8 * q);
-                if (has_res && want_sum) {
+                    for (int j = 0; j < 16; j++)
+                        h[j] = __byte_perm(__float_as_uint(__uint_as_float(v[2 * j]) + 12582912.f), __float_as_uint(__uint_as_float(v[2 * j + 1]) + 12582912.f), 0x5410);
+                    st_8(p.y16 + at, h); st_8(p.y16 + at + 16, h + 8);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; q++) st_8(p.y + at + 8 * q, v + 8 * q);
+                }
+                if (res16 && want_sum && sr.fast) {                        // whole numbers below 2^18 + 2^15: 32 of them add exactly in float
+                    float f0 = 0.f, f1 = 0.f, f2 = 0.f, f3 = 0.f;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 4) {
+                        f0 += fabsf(__uint_as_float(v[j])); f1 += fabsf(__uint_as_float(v[j + 1]));
+                        f2 += fabsf(__uint_as_float(v[j + 2])); f3 += fabsf(__uint_as_float(v[j + 3]));
+                    }
+                    const double a = (double)((f0 + f1) + (f2 + f3));
+                    if (lane < sr.split) dsum0 += a; else dsum1 += a;
+                } else if (has_res && want_sum) {
                     // the residual need not be integer-valued: compensated (Kahan) float sums, four chains, whose value and
                     // compensation go to the double totals (good to about 1e-14 of the total)
                     float s4[4] = {0.f, 0.f, 0.f, 0.f}, c4[4] = {0.f, 0.f, 0.f, 0.f};
@@ -727,7 +763,8 @@ __device__ __forceinline__ void tepi_request_residual(const void* tmR, const Tep
 }
 
 // ---- the kernel ------------------------------------------------------------------------------------------------------------
-// FUSED: 0 plain; 1 per-image |y| sums and the threshold tail; 2 residual added (sums and tail when asked for).
+// FUSED: 0 plain; 1 per-image |y| sums and the threshold tail; 2 residual added (sums and tail when asked for); 3 the same
+// with a residual of 16-bit integers, the result as fp32 or 16-bit integers (4-bit operands only).
 // BRES: the filter block of the CTA (all taps, all channel pairs; needs KN <= TNI) is copied once and stays in shared
 // memory; otherwise it streams through a ring of SB stages, one stage per tap and channel pair.
 // TEPI: the epilogue moves the output (and the residual) with TMA boxes; needs the aligned virtual grid (p.tepi).
@@ -1293,14 +1330,14 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
             const int ec0 = MT == 2 || wg == 0 ? 0 : chalf, ec1 = MT == 2 || wg == 1 ? wcols : chalf;
             SlabRows sr;
             slab_rows<FUSED>(p, R0 + emb * UTM + (warp & 3) * 32, lane, sr);
-            float res[32];
+            float res[res_regs<FUSED>()];
             bool res_loaded = false;
             // the warp that reads the columns which overlap the other accumulator begins with them
             const bool first_in_line = E2M1 && overlap && wg == (buf ? 0 : 1), down = first_in_line && buf == 0;
             const int clast = n0 + ec1 <= p.KN ? ec1 : ec0 + max(0, (p.KN - n0 - ec0 + 31) / 32 * 32);     // end of the blocks with real filters
             const int cfirst = down ? clast - 32 : ec0;
-            if (FUSED == 2 && p.wide && ec0 < clast && n0 + cfirst + 32 <= p.KN) {
-                slab_load_residual(p, sr, n0 + cfirst, res);
+            if (FUSED >= 2 && p.wide && ec0 < clast && n0 + cfirst + 32 <= p.KN) {
+                slab_load_residual<FUSED>(p, sr, n0 + cfirst, res);
                 res_loaded = true;
             }
             if (!mbar_wait_prof<6, PAIR>(prof_on, accFull + 8 * buf, (a >> 1) & 1u)) { dead = true; if (lane == 0) { if (status) atomicExch(status, 16); *deadp = 1; } break; }
@@ -1513,7 +1550,7 @@ static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, T
     const long long nrows = 128LL * mt + halo, prow = (nrows + 7) / 8 * 8;
     // patches, barriers, epilogue buffers (none where every block leaves straight from registers).  Dynamic shared memory starts
     // on a 1024-byte boundary (no static shared memory in the kernel); the kernel checks that.
-    const bool staged = !(p.wide && p.KN % 32 == 0 && (p.residual || p.y16));
+    const bool staged = !(p.wide && p.KN % 32 == 0 && (p.residual || p.residual16 || p.y16));
     const long long fixed = 2 * prow * IROW + 1024 + 8 * (p.tepi ? 8192 : (staged ? 4096 : 0));
     const int tlog = resident_taps_log2(p.PC, p.e2m1 != 0), wpr = p.e2m1 ? 4 : 2;
     const long long taps = (long long)p.KH * p.KW;
@@ -1596,7 +1633,8 @@ static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
     if ((long long)p.KH * p.KW * p.PC >= (1LL << 20)) return false;
     if (p.e2m1 && (long long)p.KH * p.KW * p.C >= (1LL << 24)) return false;       // sums the fp32 accumulators may not hold exactly
     const void* out = p.y16 ? static_cast<const void*>(p.y16) : static_cast<const void*>(p.y);
-    p.wide = p.KN % (p.y16 ? 16 : 8) == 0 && !(reinterpret_cast<uintptr_t>(out) & 31) && !(reinterpret_cast<uintptr_t>(p.residual) & 31);
+    p.wide = p.KN % (p.y16 || p.residual16 ? 16 : 8) == 0 && !(reinterpret_cast<uintptr_t>(out) & 31) &&
+             !(reinterpret_cast<uintptr_t>(p.residual) & 31) && !(reinterpret_cast<uintptr_t>(p.residual16) & 31);
     const bool tepi_ok = (p.KN & 3) == 0 && !(reinterpret_cast<uintptr_t>(p.y) & 15) && !(reinterpret_cast<uintptr_t>(p.residual) & 15) &&
                          (long long)p.KN * p.OW * p.OH * 4 < (1LL << 40);
     bool tepi_pays = p.residual != nullptr && p.y16 == nullptr && p.KN <= 64 && (long long)p.KH * p.KW * p.C <= 1024;
@@ -1650,7 +1688,7 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
 template <int MT, int TNI, int SB, bool E2M1>
 static int launch_persist(const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcConvParams& p, const TcPlan& pl,
                           int sms, int* status, cudaStream_t stream) {
-    const int fused = p.residual ? 2 : (p.abs_sums ? 1 : 0);
+    const int fused = p.residual16 ? 3 : (p.residual ? 2 : (p.abs_sums ? 1 : 0));
     const bool tepi = p.tepi != 0;
     if (pl.pair) {
         if constexpr (MT == 1 && TNI == 256 && !E2M1) {
@@ -1671,7 +1709,7 @@ static int launch_persist(const CUtensorMap& tmB, const CUtensorMap& tmY, const 
             return TAB_E_TOO_LARGE;
         }
     }
-#define TAB_LAUNCH_F(BR) do { if (fused == 2) TAB_LAUNCH(BR, 2, false); if (fused == 1) TAB_LAUNCH(BR, 1, false); TAB_LAUNCH(BR, 0, false); } while (0)
+#define TAB_LAUNCH_F(BR) do { if constexpr (E2M1) { if (fused == 3) TAB_LAUNCH(BR, 3, false); } if (fused == 2) TAB_LAUNCH(BR, 2, false); if (fused == 1) TAB_LAUNCH(BR, 1, false); TAB_LAUNCH(BR, 0, false); } while (0)
     if (pl.resident) TAB_LAUNCH_F(true);
     TAB_LAUNCH_F(false);
 #undef TAB_LAUNCH_F
@@ -1751,7 +1789,7 @@ int tc_conv_dispatch(TcConvParams p, cudaStream_t stream) {
     int* status = umma_status_ptr();
     const bool halves = split_point(pl.tiles_m * pl.tiles_n, sms, half_box && !pl.pair && pl.tnw % 64 == 0) < pl.tiles_m * pl.tiles_n;
     snprintf(g_last_kernel, sizeof(g_last_kernel), "conv_umma_persist_kernel<%d,%d,%d,%d,%d,%d%s> grid %dx%d%s%s", pl.mt, pl.tn, pl.sb, (int)pl.resident,
-             p.residual ? 2 : (p.abs_sums ? 1 : 0), p.tepi, pl.pair ? ",pair" : (p.e2m1 ? ",e2m1" : ""), p.VH, p.VW, halves ? " halves" : "", p.next_qx ? " +next" : "");
+             p.residual16 ? 3 : (p.residual ? 2 : (p.abs_sums ? 1 : 0)), p.tepi, pl.pair ? ",pair" : (p.e2m1 ? ",e2m1" : ""), p.VH, p.VW, halves ? " halves" : "", p.next_qx ? " +next" : "");
     return p.e2m1 ? launch_plan<true>(tmB, tmY, tmR, p, pl, sms, status, stream) : launch_plan<false>(tmB, tmY, tmR, p, pl, sms, status, stream);
 }
 

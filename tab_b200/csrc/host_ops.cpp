@@ -100,8 +100,7 @@ py::object conv2d_packed4(const Tensor& QX, const Tensor& W4, int type, int p1, 
         Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
         const bool want = threshold_scale.has_value();
         if (g.good() && plain(QX, at::kLong) && plain(W4, at::kByte) && QX.numel() == g.pixels() * g.PC * (type == 2 || type == 3 ? 1 : 2) &&
-            W4.numel() == g.weight_words() * 32 && !(out_int16 && residual.has_value()) &&
-            (!residual.has_value() || (plain(*residual, at::kFloat) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
+            W4.numel() == g.weight_words() * 32 && (!residual.has_value() || ((plain(*residual, at::kShort) || (!out_int16 && plain(*residual, at::kFloat))) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
             (!want || (state.has_value() && state->defined() && state->is_cuda())) && (!next_bitwidth.has_value() || want)) {
             const c10::cuda::CUDAGuard guard(QX.device());
             const int nb = next_bitwidth.has_value() ? (*next_bitwidth == 1 ? 1 : 2) : 0;
@@ -109,7 +108,7 @@ py::object conv2d_packed4(const Tensor& QX, const Tensor& W4, int type, int p1, 
             if (want) nxt = make(QX, {N}, at::kFloat);
             if (nb) QN = make(QX, {N, g.OH, g.OW, ((int64_t)KN + 63) / 64, nb}, at::kLong);
             if (tab_conv2d_packed4_launch(QX.data_ptr<int64_t>(), W4.data_ptr<uint8_t>(), Y.data_ptr(), out_int16 ? 1 : 0, type, p1, p2, s1, s2,
-                                          N, H, W, C, KN, KH, KW, residual.has_value() ? residual->data_ptr<float>() : nullptr,
+                                          N, H, W, C, KN, KH, KW, residual.has_value() ? residual->data_ptr() : nullptr, residual.has_value() && residual->scalar_type() == at::kShort ? 1 : 0,
                                           want ? state->data_ptr() : nullptr, want ? nxt.data_ptr<float>() : nullptr,
                                           want ? (float)*threshold_scale : 0.f, nb ? QN.data_ptr<int64_t>() : nullptr, nb, stream_of(QX)) != TAB_OK) Y.reset();
         }

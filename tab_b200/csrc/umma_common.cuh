@@ -60,8 +60,9 @@ struct TcConvParams {
     const int8_t* w8;        // weights: bytes, or (e2m1) nibbles, [KN][KH*KW*PC][64 or 32 bytes]
     int e2m1;                // operands are 4-bit floats (see umma_e2m1) instead of bytes
     float* y;                // [M][KN]
-    int16_t* y16;            // when not null the result goes here as int16 instead (no residual; |y| <= KH*KW*C must fit)
+    int16_t* y16;            // when not null the result goes here as int16 instead (no fp32 residual; the values must fit)
     const float* residual;   // [M][KN] added to the result, or null
+    const int16_t* residual16;   // the same as 16-bit integers (one of the two at most), or null
     double* abs_sums;        // [N]: += sum |y| per image, or null
     int N, H, W, C, PC, KN, KH, KW, OH, OW, p1, p2, s1, s2;
     int M, Kw;

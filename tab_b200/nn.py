@@ -41,6 +41,8 @@ class TABConv2d(torch.nn.Module):
     """One TAB convolution with prepared weights.  ``forward(x)`` takes fp32 NHWC activations ``[N,H,W,C]`` and returns
     what ``Conv2d`` returns: float32 ``{N,KN,OH,OW}`` over a ``[N][OH][OW][KN]`` buffer (``TAB_GEMM.cu:509,526``)."""
 
+    int16_residual = True                                                  # conv_bits takes an int16 residual, with out_int16 too
+
     def __init__(self, QW, BTN_W, conv_type, KN, KH, KW, C, padding=(0, 0), stride=(1, 1), threshold_scale=0.7):
         super().__init__()
         conv_type = int(conv_type)
@@ -127,14 +129,17 @@ class TABConv2d(torch.nn.Module):
 
     def conv_bits(self, QX, N, H, W, residual=None, next_threshold_scale=None, state=None, out_int16=False, next_bitwidth=None):
         """GEMM stage on quantised activations.  Returns ``(Y, next_thresholds_or_None)``.  ``out_int16``: ``Y`` as int16
-        where that is possible (no residual, KH*KW*C <= 32767, a shape the tensor-core kernel covers), else fp32 as usual:
-        look at ``Y.dtype``.  ``next_bitwidth`` (with ``next_threshold_scale``): a third value is returned, ``Y`` quantised
+        where that is possible (no residual, or one of int16 with which the caller knows the sum to fit; KH*KW*C <= 32767, a
+        shape the tensor-core kernel covers), else fp32 as usual: look at ``Y.dtype``.  ``next_bitwidth`` (with ``next_threshold_scale``): a third value is returned, ``Y`` quantised
         against the next thresholds at that bitwidth - the next convolution's ``QX`` - from the same launch."""
         if next_threshold_scale is not None and state is None:
             state = self.state(N, QX.device)
         if next_bitwidth is not None and next_threshold_scale is None:
             raise ValueError("next_bitwidth needs next_threshold_scale")
-        compact = out_int16 and residual is None and self.KH * self.KW * self.C <= 32767
+        res16 = residual is not None and residual.dtype == torch.int16
+        if res16 and self.W4 is None:
+            residual, res16 = residual.float(), False
+        compact = out_int16 and (residual is None or res16) and self.KH * self.KW * self.C <= 32767
         try:
             return ops.conv2d_bits(QX, self.W8 if self.W4 is None else self.W4, self.conv_type, *self.geometry(N, H, W), residual=residual,
                                    threshold_scale=next_threshold_scale, state=state, out_int16=compact, next_bitwidth=next_bitwidth)
@@ -144,6 +149,8 @@ class TABConv2d(torch.nn.Module):
         # shapes the tensor-core kernel does not cover: the bit-packed popcount kernel, then the chaining in one pass
         Y = ops.conv2d_packed(QX, self.QW, self.BTN_W, self.conv_type, *self.geometry(N, H, W))
         nxt = None
+        if res16:
+            residual = residual.float()
         if residual is not None or next_threshold_scale is not None:
             nxt = ops.residual_threshold(Y, residual, next_threshold_scale if next_threshold_scale is not None else 0.0)
             if next_threshold_scale is None:

@@ -263,7 +263,8 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
     types 2,3), weights from ``expand_weights`` (int8) or ``pack_weights`` (uint8: twice the rate, KH*KW*C < 2**24).  Returns
     ``(Y, next_thresholds_or_None)``; ``Y = conv + residual``.
     ``threshold_scale`` needs ``state`` (``new_state``).  ``out_int16``: ``Y`` as int16 (no residual; the values are
-    integers of magnitude at most KH*KW*C) for ``quantize_i16``.  ``next_bitwidth`` (needs ``threshold_scale``): the same
+    integers of magnitude at most KH*KW*C) for ``quantize_i16``.  With uint8 weights the residual may be int16 too, and then so
+    may ``Y``, where the caller knows that the sum fits.  ``next_bitwidth`` (needs ``threshold_scale``): the same
     launch also quantises ``Y`` against the next thresholds at that bitwidth and a third value is returned, ``QX`` of the
     next convolution (``[N,OH,OW,ceil(KN/64),bits]`` int64, what ``Quantize(Y, next_thresholds, ...)`` gives).
     Raises ``TabError`` (TAB_E_TOO_LARGE) for shapes the tensor-core kernel does not cover."""
@@ -286,12 +287,15 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
         raise RuntimeError("W8 has %d bytes, expected KN*KH*KW*Cp%s = %d" % (W8.numel(), "/2" if packed4 else "", KN * KH * KW * PC * (32 if packed4 else 64)))
     OH, OW = conv_out_size(H, W, KH, KW, p1, p2, s1, s2)
     if residual is not None:
-        _check_input(residual, "residual", torch.float32)
+        res16 = packed4 and isinstance(residual, torch.Tensor) and residual.dtype == torch.int16
+        _check_input(residual, "residual", torch.int16 if res16 else torch.float32)
         if residual.numel() != N * KN * OH * OW:
             raise RuntimeError("residual has %d elements, expected %d" % (residual.numel(), N * KN * OH * OW))
+    else:
+        res16 = False
     if threshold_scale is not None and state is None:
         raise RuntimeError("threshold_scale needs a state block (new_state)")
-    if out_int16 and residual is not None:
+    if out_int16 and residual is not None and not res16:
         raise RuntimeError("out_int16 cannot be combined with a residual")
     if next_bitwidth is not None and threshold_scale is None:
         raise RuntimeError("next_bitwidth needs threshold_scale (the thresholds the result is quantised against)")
@@ -303,7 +307,7 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
             QN = torch.empty((N, OH, OW, (KN + 63) // 64, nb), dtype=torch.int64, device=QX.device) if nb else None
             rc = _cabi.lib().tab_conv2d_packed4_launch(QX.data_ptr(), W8.data_ptr(), Y.data_ptr(), 1 if out_int16 else 0, conv_type,
                                                        p1, p2, s1, s2, N, H, W, C, KN, KH, KW,
-                                                       residual.data_ptr() if residual is not None else None,
+                                                       residual.data_ptr() if residual is not None else None, 1 if res16 else 0,
                                                        state.data_ptr() if nxt is not None else None,
                                                        nxt.data_ptr() if nxt is not None else None,
                                                        float(threshold_scale) if threshold_scale is not None else 0.0,

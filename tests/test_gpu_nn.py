@@ -84,6 +84,19 @@ def test_prepared_chain_matches_oracle(cuda, t):
             yd, oh, ow, kn = chain.forward_prepared({k: Nhwc(v) for k, v in convs.items()}, xd, thd, N, compact_mid=compact, fused_quant=fused_quant)
             assert (oh, ow, kn) == (7, 7, 512)
             assert np.array_equal(yd.cpu().numpy().reshape(-1), np.asarray(yo).reshape(-1)), (compact, fused_quant)
+    # the modules themselves: 16-bit block results from the first strided shortcut on
+    yd, _, _, _ = chain.forward_prepared(convs, xd, thd, N, compact_mid=True, fused_quant=True)
+    assert yd.dtype == torch.float32 and np.array_equal(yd.cpu().numpy().reshape(-1), np.asarray(yo).reshape(-1))
+    reps = 85                                                          # enough images for them to be used, against the fp32 hand-over
+    xl, tl = xd.repeat(reps, 1, 1, 1).contiguous(), thd.repeat(reps).contiguous()
+    seen = []
+    plain = tab_nn.TABConv2d.conv_bits
+    try:
+        tab_nn.TABConv2d.conv_bits = lambda self, *a, **k: (seen.append(a[4] is not None and a[4].dtype == torch.int16 if len(a) > 4 else False), plain(self, *a, **k))[1]
+        yl, _, _, _ = chain.forward_prepared(convs, xl, tl, N * reps, compact_mid=True, fused_quant=True)
+    finally:
+        tab_nn.TABConv2d.conv_bits = plain
+    assert any(seen) and torch.equal(yl.reshape(reps, -1), yd.reshape(1, -1).expand(reps, -1))
     assert _cabi.lib().tab_device_status() == 0
 
 

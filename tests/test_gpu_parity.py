@@ -779,6 +779,15 @@ def test_packed4_weights(cuda, geom, t, conv_path):
             a = TAB.ops.conv2d_bits(qx, w4, t, *geom, threshold_scale=0.7, state=state, next_bitwidth=bw, **kw)
             b = TAB.ops.conv2d_bits(qx, w8, t, *geom, threshold_scale=0.7, state=state, next_bitwidth=bw, **kw)
             assert len(a) == len(b) and all(torch.equal(u, v) for u, v in zip(a, b)) and not state.any().item()
+    # a 16-bit residual, the result as fp32 and as 16-bit integers
+    r16 = torch.round(r).to(torch.int16)
+    for bw in (None, 2, 1):
+        b = TAB.ops.conv2d_bits(qx, w8, t, *geom, residual=r16.float(), threshold_scale=0.7, state=state, next_bitwidth=bw)
+        for out16 in (False, True):
+            a = TAB.ops.conv2d_bits(qx, w4, t, *geom, residual=r16, threshold_scale=0.7, state=state, next_bitwidth=bw, out_int16=out16)
+            assert a[0].dtype == (torch.int16 if out16 else torch.float32) and torch.equal(a[0].float(), b[0])
+            assert all(torch.equal(u, v) for u, v in zip(a[1:], b[1:]) if u is not None) and not state.any().item()
+    assert torch.equal(TAB.ops.conv2d_bits(qx, w4, t, *geom, residual=r16, out_int16=True)[0].float(), b[0])
     y3, _ = TAB.ops.conv2d_bits(qx, w4, t, *geom, residual=r)
     assert torch.equal(y3, y8 + r)
     assert _cabi.lib().tab_device_status() == 0
