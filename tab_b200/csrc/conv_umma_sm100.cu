@@ -1544,8 +1544,9 @@ static long long split_point(long long ntiles, int sms, bool capable) {
     return capable && ntiles > grid && rest != 0 && 2 * rest <= grid ? ntiles - rest : ntiles;
 }
 
+// most: filters of a tile, where that is to be fewer than the shape's tn.
 // pair: clusters of two CTAs; a tile is 256 rows (128 per CTA) x tn filters, a ring stage holds tn/2 filters per CTA.
-static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, TcPlan* out, bool pair = false) {
+static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, TcPlan* out, bool pair = false, int most = 0) {
     const long long halo = (long long)((p.KH - 1) / p.s1) * p.VW + (p.KW - 1) / p.s2;
     const long long nrows = 128LL * mt + halo, prow = (nrows + 7) / 8 * 8;
     // patches, barriers, epilogue buffers (none where every block leaves straight from registers).  Dynamic shared memory starts
@@ -1559,10 +1560,11 @@ static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, T
     pl.mt = mt; pl.tn = tn; pl.sb = sb; pl.pair = pair;
     // The filters are shared out evenly over as few tiles of at most tn as hold them, in whole 32-column blocks of the
     // epilogue: 130 filters are multiplied as 160 columns and not as 256, 300 as twice 160 and not as 256 + 256.
-    pl.tiles_n = (p.KN + tn - 1) / tn;
+    if (most <= 0) most = tn;
+    pl.tiles_n = (p.KN + most - 1) / most;
     pl.tnw = (int)((p.KN + pl.tiles_n - 1) / pl.tiles_n + 31) / 32 * 32;
     const long long tnw = pl.tnw;
-    pl.resident = !pair && p.KN <= tn && fixed + nres * tnw * IROW <= UMMA_SMEM_MAX;
+    pl.resident = !pair && p.KN <= most && fixed + nres * tnw * IROW <= UMMA_SMEM_MAX;
     const long long smem = pl.resident ? fixed + nres * tnw * IROW : fixed + (long long)sb * (pair ? tnw / 2 : tnw) * IROW;
     if (smem > UMMA_SMEM_MAX) return false;
     pl.prow = (int)prow; pl.nrows = (int)nrows; pl.nst = pl.resident ? (int)nres : sb; pl.smem = (int)smem;
@@ -1615,8 +1617,15 @@ static bool tc_plan(const TcConvParams& p, int sms, TcPlan* best) {
         if (!plan_shape(p, sms, c[0], c[1], c[2], &pl)) continue;
         if (!found) { *best = pl; found = true; }
         if (pl.tiles_m * pl.tiles_n * 2 > sms) { *best = pl; break; }      // enough tiles: take it; else keep looking for more tiles
-        if (pl.tiles_m * pl.tiles_n > best->tiles_m * best->tiles_n) *best = pl;
+        // fewer: the most tiles, and of equals the later (fewer filters, then one row block: an image of 49 positions leaves the
+        // second one empty and waits for its expansion all the same)
+        if (pl.tiles_m * pl.tiles_n >= best->tiles_m * best->tiles_n) *best = pl;
     }
+    // A single small image: tiles of 32 filters where even those leave half of the SMs without one and the sum is long (short
+    // ones are done before the second CTA's set-up is: 32x32x64 6.7 us with 64 filters per tile, 7.1 with 32).  With the rule
+    // above, 7x7x512 -> 512: 16.9 -> 15.2 us.
+    TcPlan half;
+    if (found && best->tn == 64 && p.KN > 32 && p.Kw >= 32 && best->tiles_m * best->tiles_n * 4 <= sms && plan_shape(p, sms, 1, 64, 6, &half, false, 32)) *best = half;
     return found;
 }
 
