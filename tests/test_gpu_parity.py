@@ -747,6 +747,8 @@ def test_weight_expansion_inside_a_call(cuda, conv_path, N, KN, K, C):
     (1, 1, 2, 2, 200, 14, 14, 256, 512, 3, 3),
     (1, 1, 1, 1, 8, 56, 56, 64, 60, 3, 3),       # the TMA epilogue, several tiles per CTA, a partial block
     (1, 1, 1, 1, 1, 100, 150, 200, 40, 3, 3),    # long patches: several chunks of items
+    (1, 1, 1, 1, 1, 7, 7, 512, 512, 3, 3),       # one small image, a long sum: tiles of 32 filters
+    (1, 1, 1, 1, 1, 7, 7, 300, 72, 3, 3),
     (3, 3, 2, 2, 2, 224, 224, 3, 64, 7, 7),
 ])
 @pytest.mark.parametrize("t", [0, 1, 2, 3])
