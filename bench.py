@@ -262,7 +262,7 @@ def step_algorithmic_bytes(n_images):
     producer handed it over as int16) and 2 bits/element written by the quantiser; per convolution those bit-planes read, the
     4-bit weights read, the output written (4 B/element; 2 B for a block's first convolution, whose only reader is the next
     quantiser) and, where a shortcut is added, 4 B/element of residual read; the input statistics pass reads x once.  From the
-    first strided shortcut on block results and shortcuts of more than 2^23 elements are 2 B/element too."""
+    first strided shortcut on large block results and shortcuts are 2 B/element too."""
     from tab_b200 import chain
     total = 4 * n_images * H0 * W0 * C0
     h = H0
@@ -270,7 +270,7 @@ def step_algorithmic_bytes(n_images):
     for i, b in enumerate(blocks):
         a, bb, sc = b.conv_a, b.conv_b, b.shortcut
         oh = (h + 2 * a.pad - a.K + 1) // a.stride
-        small = i >= 2 and n_images * oh * oh * a.KN > 1 << 23
+        small = i >= 2 and n_images * oh * oh * a.KN > chain.INT16_RESULTS_FROM
         short_bytes = x_bytes if sc is None else (2 if small else 4)
         out_bytes = 2 if small and i + 1 < len(blocks) else 4
         x_el, y_el = n_images * h * h * a.C, n_images * oh * oh * a.KN
@@ -691,7 +691,7 @@ def main():
             chained = cs.K == 3                                             # the 3x3 convolutions feed thresholds, the shortcuts do not
             # int16 as in the chain: a block's first convolution, and from the first strided shortcut on large shortcuts,
             # residuals and block results (the last one excepted)
-            small = not cs.name.startswith("s1") and n_local * oh * oh * cs.KN > 1 << 23
+            small = not cs.name.startswith("s1") and n_local * oh * oh * cs.KN > chain.INT16_RESULTS_FROM
             res16 = has_res and small
             compact = (chained and not has_res) or (small and cs.name != "s4b1.b")
             y = torch.empty(n_local * oh * oh * cs.KN, dtype=torch.int16, device=dev) if compact else yb

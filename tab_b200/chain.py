@@ -26,6 +26,7 @@ from typing import List, Optional
 import numpy as np
 
 THRESHOLD_SCALE = 0.7
+INT16_RESULTS_FROM = 1 << 22           # elements of a block result above which it travels as int16, see forward_prepared
 
 
 @dataclass
@@ -165,15 +166,15 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
         bound = None                                           # of |x|, None while x need not be whole numbers
         for i, b in enumerate(blocks):
             a, bb, sc = convs[b.conv_a.name], convs[b.conv_b.name], (convs[b.shortcut.name] if b.shortcut else None)
+            oh, ow = (h + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride, (w + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride
             # From the first strided shortcut on the block results are whole numbers too: conv + conv, conv + conv + conv, ...
             # They travel as int16 as well while their largest possible magnitude fits and the tensor is large enough for its
-            # bytes to matter (above the size up to which a convolution quantises its own result; 8 images 267 us with fp32
-            # results and 275 with int16 ones, 256 images 1071 and 983).
+            # bytes to matter (0.8M values, 8 images: 267 us with fp32 results and 275 with int16 ones; 6.4M and more, 256
+            # images: 1071 and 983).
             terms = b.conv_b.K * b.conv_b.K * b.conv_b.C
             short_bound = bound if sc is None else b.shortcut.K * b.shortcut.K * b.shortcut.C
             bound = None if short_bound is None else short_bound + terms
-            small = compact_mid and bound is not None and bound <= 32767 and N * oh * ow * b.conv_b.KN > 1 << 23 and all(getattr(c, "int16_residual", False) for c in (bb, sc or bb))
-            oh, ow = (h + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride, (w + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride
+            small = compact_mid and bound is not None and bound <= 32767 and N * oh * ow * b.conv_b.KN > INT16_RESULTS_FROM and all(getattr(c, "int16_residual", False) for c in (bb, sc or bb))
             short = x if sc is None else (sc.conv_bits(qx, N, h, w, None, None, out_int16=True) if small else sc.conv_bits(qx, N, h, w, None, None))[0]
             _, _, q1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, out_int16=compact_mid, next_bitwidth=act_bits(bb))
             if i + 1 < len(blocks):
