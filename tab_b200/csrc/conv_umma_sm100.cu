@@ -46,7 +46,14 @@ constexpr int PTHREADS = 512;                                              // 16
 // The epilogue of these variants fits 96 registers, so up to 21 warps fit the register file.  Measured per filter-block
 // width on the ResNet-18-shaped layers: 2 / 4 / 3 extra warps; one more each changed nothing, and on residual layers the
 // epilogue is the bound and needs the registers.
-__host__ __device__ constexpr int extra_warps(int fused, bool tepi, int tn) { return (fused <= 1 && !tepi) ? (tn == 64 ? 2 : (tn == 128 ? 4 : 3)) : 0; }
+// 4-bit operands (an item is two words, so patches have fewer): the 316-318 items of a 128- or 256-filter tile's patch at 28x28
+// and 14x14 are one round of ten warps and two of nine; 64-filter tiles gain from two warps more, and lose what is gained on
+// small problems with five more (3x3 16x112x112x256->64 69.6 us with 2, 65.2 with 4, 64.0 with 7; the network at 8 images 265,
+// 263, 270).  With a residual four more showed no gain (network at 256 images 988 us against 986).
+__host__ __device__ constexpr int extra_warps(int fused, bool tepi, int tn, bool e2m1) {
+    if (e2m1) return (fused <= 1 && !tepi) ? (tn == 64 ? 4 : (tn == 128 ? 5 : 4)) : 0;
+    return (fused <= 1 && !tepi) ? (tn == 64 ? 2 : (tn == 128 ? 4 : 3)) : 0;
+}
 // Kernels that can work a tile as two halves of tn/2 filters (their filter boxes hold tn/2 filters): one row block, the
 // widest tile, streamed filters, transposing epilogue, single CTAs.
 __host__ __device__ constexpr bool split_capable(int mt, int tn, bool resident, bool tepi, bool pair) { return mt == 1 && tn == 256 && !resident && !tepi && !pair; }
@@ -781,7 +788,7 @@ __device__ __forceinline__ void tepi_request_residual(const void* tmR, const Tep
 // columns of scales do not fit beside two 256-column accumulators: those overlap by 16 columns, which the epilogue reads
 // first, and the next tile's MMAs wait for that ("freed") instead of only for the tile before last.
 template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false, bool E2M1 = false>
-__global__ void __launch_bounds__(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI), 1)
+__global__ void __launch_bounds__(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1), 1)
 conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
                          const TcConvParams p, int* __restrict__ status,
                          const int prow, const int nrows, const int nst, const int tiles_m, const int tiles_n, const int split_from, const int tnw) {
@@ -795,7 +802,7 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     constexpr int SFCOL = ABUF + ACOLS;                                    // E2M1: 16 columns of scales behind them
     constexpr int TCOLS = !E2M1 ? 2 * ACOLS : (SFCOL + 16 <= 256 ? 256 : 512);
     static_assert(!E2M1 || !PAIR, "CTA pairs multiply bytes");
-    constexpr int NXW = 5 + extra_warps(FUSED, TEPI, TNI) + (MT == 1 ? 1 : 0);   // expander warps: 0, 12 and up, and warp 3 when it has no MMAs to issue
+    constexpr int NXW = 5 + extra_warps(FUSED, TEPI, TNI, E2M1) + (MT == 1 ? 1 : 0);   // expander warps: 0, 12 and up, and warp 3 when it has no MMAs to issue
     constexpr int NX = 32 * NXW;
     static_assert(2 * ACOLS <= 512, "two accumulator buffers must fit the 512 TMEM columns");
     static_assert(SB <= 8, "eight ring barriers are laid out");
@@ -1685,12 +1692,12 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
     if (PAIR) {
         const long long pairs = std::min<long long>(sms / 2, pair_clusters());
         const unsigned grid = 2u * (unsigned)(ntiles < pairs ? ntiles : pairs);
-        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream, 2u,
+        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)pl.smem, stream, 2u,
                                   tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles, pl.tnw);
     }
     const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);
     const long long split_from = split_point(ntiles, sms, split_capable(MT, TNI, BRES, TEPI, PAIR) && pl.tnw % 64 == 0);
-    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI)), (size_t)pl.smem, stream,
+    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)pl.smem, stream,
                       tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)split_from, pl.tnw);
 }
 
@@ -1735,7 +1742,7 @@ static int pair_clusters() {
         auto kernel = conv_umma_persist_kernel<1, 256, 8, false, 0, false, true>;
         int clusters = 0;
         cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2); cfg.blockDim = dim3(PTHREADS + 32 * extra_warps(0, false, 256)); cfg.dynamicSmemBytes = UMMA_SMEM_MAX;
+        cfg.gridDim = dim3(2); cfg.blockDim = dim3(PTHREADS + 32 * extra_warps(0, false, 256, false)); cfg.dynamicSmemBytes = UMMA_SMEM_MAX;
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
