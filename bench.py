@@ -688,6 +688,7 @@ def main():
             nxt = torch.empty(n_local, dtype=torch.float32, device=dev)
             btn = torch.empty(n_local, dtype=torch.int32, device=dev)
             geom = conv.geometry(n_local, ih, ih)
+            w4 = tab_ops.pack_weights(conv.W8, conv.KN, conv.KH, conv.KW, conv.C)
             chained = cs.K == 3                                             # the 3x3 convolutions feed thresholds, the shortcuts do not
             # int16 as in the chain: a block's first convolution, and from the first strided shortcut on large shortcuts,
             # residuals and block results (the last one excepted)
@@ -697,7 +698,7 @@ def main():
             y = torch.empty(n_local * oh * oh * cs.KN, dtype=torch.int16, device=dev) if compact else yb
             res = res.to(torch.int16) if res16 else res
             ms_gemm = time_launch(lambda: _cabi.check(lib.tab_conv2d_packed4_launch(
-                qx.data_ptr(), conv.W4.data_ptr(), y.data_ptr(), int(compact), CONV_TYPE, *geom, res.data_ptr() if has_res else None, int(res16),
+                qx.data_ptr(), w4.data_ptr(), y.data_ptr(), int(compact), CONV_TYPE, *geom, res.data_ptr() if has_res else None, int(res16),
                 state.data_ptr() if chained else None, nxt.data_ptr() if chained else None, 0.7, None, 0, stream), "packed4"))
             kernel = lib.tab_last_conv_kernel().decode()
             if has_res:                                                     # a block's second convolution quantises the first one's int16 output
@@ -710,7 +711,7 @@ def main():
             ms_popc = time_launch(lambda: _cabi.check(lib.tab_conv2d_packed_launch(qx.data_ptr(), conv.QW.data_ptr(), conv.BTN_W.data_ptr(), yb.data_ptr(),
                                                                                     CONV_TYPE, *geom, stream), "popc"))
             lops = 2 * n_local * oh * oh * cs.KN * cs.K * cs.K * cs.C
-            gemm_bytes = qx.numel() * 8 + conv.W4.numel() + y.numel() * y.element_size() + (res.numel() * res.element_size() if has_res else 0)
+            gemm_bytes = qx.numel() * 8 + w4.numel() + y.numel() * y.element_size() + (res.numel() * res.element_size() if has_res else 0)
             quant_bytes = (2 if has_res else 4) * xin.numel() + qx.numel() * 8
             sums["gemm_ms"] += ms_gemm; sums["popc_ms"] += ms_popc; sums["ops"] += lops; sums["gemm_bytes"] += gemm_bytes
             if cs.K == 3:                                                   # the shortcut reuses conv_a's bit-planes: no quantiser launch of its own

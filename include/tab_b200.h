@@ -192,12 +192,15 @@ int tab_quantize_i16_launch(const int16_t* x, const float* ths, int64_t* qx, int
  * that keep byte weights.
  *   tab_pack_weights_launch     tab_expand_weights_launch's bytes -> 32 bytes per 64-channel word, [KN][KH][KW][Cp/2], in the
  *                               kernel's own channel order (opaque to the caller); both pointers 16-byte aligned
+ *   tab_pack_weights_many_launch  the same for `count` layers in one launch per 32 of them: words[i] = KN*KH*KW*ceil(C/64) of
+ *                               layer i (host arrays, read before the call returns)
  *   tab_conv2d_packed4_launch   tab_conv2d_bits_launch / _i16_launch / _next_launch in one entry point: y is float or, with
  *                               y_is_int16, int16; residual (float, or int16 with residual_is_int16), state with next_ths,
  *                               and next_qx with next_bitwidth are optional as there.  An int16 y takes an int16 residual or
  *                               none, and the caller knows that conv + residual fits 16 bits.  TAB_E_TOO_LARGE also when KH*KW*C >= 2^24.
  */
 int tab_pack_weights_launch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, tab_stream_t stream);
+int tab_pack_weights_many_launch(int count, const int8_t* const* w8, uint8_t* const* w4, const long long* words, tab_stream_t stream);
 int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int y_is_int16, int type, int p1, int p2, int s1, int s2,
                               int N, int H, int W, int C, int KN, int KH, int KW,
                               const void* residual, int residual_is_int16, void* state, float* next_ths, float next_scale,

@@ -157,8 +157,13 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
     (``conv_bits(..., next_bitwidth=bits) -> (Y, next_ths, next_QX)``; the objects need a ``conv_type``), so that only the
     chain's input is quantised by a launch of its own; ``qx0``: that quantised input, when the caller already has it
     (``quantize_auto`` gives it together with ``ths``).
+    Objects with a ``pack_together`` get the keywords it returns for them with every ``conv_bits``: what they derive from their
+    weights is then derived once per pass for all layers.
     Returns ``(y, OH, OW, KN)`` like ``forward``; the results are identical."""
     h, w = H, W
+    together = getattr(next(iter(convs.values()), None), "pack_together", None)
+    packed = together(convs) if together is not None else {}
+    extra = lambda spec: packed.get(spec.name, {})
     if fused_quant:
         blocks = resnet18_blocks()
         act_bits = lambda conv: 1 if conv.conv_type in (2, 3) else 2
@@ -175,21 +180,21 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
             short_bound = bound if sc is None else b.shortcut.K * b.shortcut.K * b.shortcut.C
             bound = None if short_bound is None else short_bound + terms
             small = compact_mid and bound is not None and bound <= 32767 and N * oh * ow * b.conv_b.KN > INT16_RESULTS_FROM and all(getattr(c, "int16_residual", False) for c in (bb, sc or bb))
-            short = x if sc is None else (sc.conv_bits(qx, N, h, w, None, None, out_int16=True) if small else sc.conv_bits(qx, N, h, w, None, None))[0]
-            _, _, q1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, out_int16=compact_mid, next_bitwidth=act_bits(bb))
+            short = x if sc is None else (sc.conv_bits(qx, N, h, w, None, None, **extra(b.shortcut), **(dict(out_int16=True) if small else {})))[0]
+            _, _, q1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, out_int16=compact_mid, next_bitwidth=act_bits(bb), **extra(b.conv_a))
             if i + 1 < len(blocks):
                 out = dict(out_int16=True) if small else {}
-                x, ths, qx = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE, next_bitwidth=act_bits(convs[blocks[i + 1].conv_a.name]), **out)
+                x, ths, qx = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE, next_bitwidth=act_bits(convs[blocks[i + 1].conv_a.name]), **out, **extra(b.conv_b))
             else:
-                x, ths = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE)
+                x, ths = bb.conv_bits(q1, N, oh, ow, short, THRESHOLD_SCALE, **extra(b.conv_b))
             h, w = oh, ow
         return x, h, w, blocks[-1].conv_b.KN
     for b in resnet18_blocks():
         a, bb, sc = convs[b.conv_a.name], convs[b.conv_b.name], (convs[b.shortcut.name] if b.shortcut else None)
         oh, ow = (h + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride, (w + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride
         qx = a.quantize(x, ths)
-        short = x if sc is None else sc.conv_bits(qx, N, h, w, None, None)[0]
-        y1, t1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, out_int16=True) if compact_mid else a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE)
-        y2, ths = bb.conv_bits(bb.quantize(y1, t1), N, oh, ow, short, THRESHOLD_SCALE)     # y2 = conv + shortcut
+        short = x if sc is None else sc.conv_bits(qx, N, h, w, None, None, **extra(b.shortcut))[0]
+        y1, t1 = a.conv_bits(qx, N, h, w, None, THRESHOLD_SCALE, **extra(b.conv_a), **(dict(out_int16=True) if compact_mid else {}))
+        y2, ths = bb.conv_bits(bb.quantize(y1, t1), N, oh, ow, short, THRESHOLD_SCALE, **extra(b.conv_b))     # y2 = conv + shortcut
         x, h, w = y2, oh, ow
     return x, h, w, resnet18_blocks()[-1].conv_b.KN

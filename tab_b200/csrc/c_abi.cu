@@ -305,7 +305,20 @@ int tab_pack_weights_launch(const int8_t* w8, uint8_t* w4, int KN, int KH, int K
     if (KN == 0) return TAB_OK;
     if (!w8 || !w4) return TAB_E_NULL_POINTER;
     if (misaligned(w8, 15) || misaligned(w4, 15)) return TAB_E_ALIGNMENT;
-    return pack_weights_dispatch(w8, w4, KN, KH, KW, C, reinterpret_cast<cudaStream_t>(stream));
+    const long long words = (long long)KN * KH * KW * packed_channels(C);
+    return pack_weights_dispatch(1, &w8, &w4, &words, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int tab_pack_weights_many_launch(int count, const int8_t* const* w8, uint8_t* const* w4, const long long* words, tab_stream_t stream) {
+    if (count < 0) return TAB_E_BAD_ARGUMENT;
+    if (count == 0) return TAB_OK;
+    if (!w8 || !w4 || !words) return TAB_E_NULL_POINTER;
+    for (int i = 0; i < count; i++) {
+        if (words[i] < 0) return TAB_E_BAD_ARGUMENT;
+        if (words[i] > 0 && (!w8[i] || !w4[i])) return TAB_E_NULL_POINTER;
+        if (misaligned(w8[i], 15) || misaligned(w4[i], 15)) return TAB_E_ALIGNMENT;
+    }
+    return pack_weights_dispatch(count, w8, w4, words, reinterpret_cast<cudaStream_t>(stream));
 }
 
 int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int y_is_int16, int type, int p1, int p2, int s1, int s2,

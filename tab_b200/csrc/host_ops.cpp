@@ -90,29 +90,67 @@ py::object quantize_auto(const Tensor& X, double scale, int bitwidth, int N, int
     return py::make_tuple(QX, ths);
 }
 
-// The GEMM stage on 4-bit weights (ops.conv2d_bits with uint8 weights).
-py::object conv2d_packed4(const Tensor& QX, const Tensor& W4, int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW,
+// Byte weights of several layers -> their 4-bit operands, parts of one allocation.
+py::object pack_weights(const std::vector<Tensor>& W8) {
+    std::vector<Tensor> W4;
+    {
+        py::gil_scoped_release nogil;
+        std::vector<int64_t> sizes;
+        int64_t total = 0;
+        for (const Tensor& w : W8) {
+            if (!plain(w, at::kChar) || w.numel() == 0 || w.numel() % 64 != 0 || w.device() != W8[0].device()) break;
+            sizes.push_back(w.numel() / 2);
+            total += w.numel() / 2;
+        }
+        if (!W8.empty() && sizes.size() == W8.size()) {
+            const c10::cuda::CUDAGuard guard(W8[0].device());
+            W4 = make(W8[0], {total}, at::kByte).split_with_sizes(sizes);
+            std::vector<const int8_t*> from;
+            std::vector<uint8_t*> to;
+            std::vector<long long> words;
+            for (size_t i = 0; i < W8.size(); i++) {
+                from.push_back(W8[i].data_ptr<int8_t>());
+                to.push_back(W4[i].data_ptr<uint8_t>());
+                words.push_back(sizes[i] / 32);
+            }
+            if (tab_pack_weights_many_launch((int)W8.size(), from.data(), to.data(), words.data(), stream_of(W8[0])) != TAB_OK) W4.clear();
+        }
+    }
+    if (W4.empty()) return py::none();
+    return py::cast(W4);
+}
+
+// The GEMM stage on 4-bit weights (ops.conv2d_bits with uint8 weights), or on byte weights that the call packs first.
+py::object conv2d_packed4(const Tensor& QX, const Tensor& weights, int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW,
                           const OptTensor& residual, c10::optional<double> threshold_scale, const OptTensor& state, bool out_int16,
                           c10::optional<int> next_bitwidth) {
     Tensor Y, nxt, QN;
+    int rc = TAB_OK;
     {
         py::gil_scoped_release nogil;
         Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
         const bool want = threshold_scale.has_value();
-        if (g.good() && plain(QX, at::kLong) && plain(W4, at::kByte) && QX.numel() == g.pixels() * g.PC * (type == 2 || type == 3 ? 1 : 2) &&
-            W4.numel() == g.weight_words() * 32 && (!residual.has_value() || ((plain(*residual, at::kShort) || (!out_int16 && plain(*residual, at::kFloat))) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
+        if (g.good() && plain(QX, at::kLong) && (plain(weights, at::kByte) || (plain(weights, at::kChar) && weights.device() == QX.device())) && QX.numel() == g.pixels() * g.PC * (type == 2 || type == 3 ? 1 : 2) &&
+            weights.numel() == g.weight_words() * (weights.scalar_type() == at::kByte ? 32 : 64) && (!residual.has_value() || ((plain(*residual, at::kShort) || (!out_int16 && plain(*residual, at::kFloat))) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
             (!want || (state.has_value() && state->defined() && state->is_cuda())) && (!next_bitwidth.has_value() || want)) {
             const c10::cuda::CUDAGuard guard(QX.device());
             const int nb = next_bitwidth.has_value() ? (*next_bitwidth == 1 ? 1 : 2) : 0;
             Y = make(QX, {N, KN, g.OH, g.OW}, out_int16 ? at::kShort : at::kFloat);
             if (want) nxt = make(QX, {N}, at::kFloat);
             if (nb) QN = make(QX, {N, g.OH, g.OW, ((int64_t)KN + 63) / 64, nb}, at::kLong);
-            if (tab_conv2d_packed4_launch(QX.data_ptr<int64_t>(), W4.data_ptr<uint8_t>(), Y.data_ptr(), out_int16 ? 1 : 0, type, p1, p2, s1, s2,
+            Tensor W4 = weights;
+            if (weights.scalar_type() == at::kChar) {
+                W4 = make(weights, {weights.numel() / 2}, at::kByte);
+                rc = tab_pack_weights_launch(weights.data_ptr<int8_t>(), W4.data_ptr<uint8_t>(), KN, KH, KW, C, stream_of(QX));
+            }
+            if (rc == TAB_OK) rc = tab_conv2d_packed4_launch(QX.data_ptr<int64_t>(), W4.data_ptr<uint8_t>(), Y.data_ptr(), out_int16 ? 1 : 0, type, p1, p2, s1, s2,
                                           N, H, W, C, KN, KH, KW, residual.has_value() ? residual->data_ptr() : nullptr, residual.has_value() && residual->scalar_type() == at::kShort ? 1 : 0,
                                           want ? state->data_ptr() : nullptr, want ? nxt.data_ptr<float>() : nullptr,
-                                          want ? (float)*threshold_scale : 0.f, nb ? QN.data_ptr<int64_t>() : nullptr, nb, stream_of(QX)) != TAB_OK) Y.reset();
+                                          want ? (float)*threshold_scale : 0.f, nb ? QN.data_ptr<int64_t>() : nullptr, nb, stream_of(QX));
+            if (rc != TAB_OK) Y.reset();
         }
     }
+    if (rc == TAB_E_TOO_LARGE) return py::int_(rc);                         // the caller need not find that out again
     if (!Y.defined()) return py::none();
     py::object th = nxt.defined() ? py::cast(nxt) : py::none();
     if (QN.defined()) return py::make_tuple(Y, th, QN);
@@ -125,5 +163,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("quantize", &quantize);
     m.def("conv2d", &conv2d);
     m.def("quantize_auto", &quantize_auto);
+    m.def("pack_weights", &pack_weights);
     m.def("conv2d_packed4", &conv2d_packed4);
 }

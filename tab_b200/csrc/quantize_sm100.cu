@@ -70,22 +70,40 @@ __device__ __forceinline__ void expand_half(const uint64_t* __restrict__ qw, uin
     *reinterpret_cast<uint4*>(w4 + word * 32 + h * 16) = nibbles32(m, s & m);
 }
 
-__global__ void pack_weights_kernel(const int8_t* __restrict__ w8, uint8_t* __restrict__ w4, long long halves) {
-    const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= halves) return;
-    uint32_t m = 0, s = 0;
+// Byte weights -> 4-bit operands, several layers in one launch: a CTA takes 256 halves (32 channels: 32 bytes in, 16 out) of the
+// layer whose range of CTAs it lies in.  Bound by the launch: a prepared layer's bytes are the registered weights and are
+// packed again by every pass, so that whoever writes them is followed; a network does that once per pass for all its layers.
+// B200, GPU time of a call with / without it: 3x3 64x14x14x256->256 19.4 / 18.1 us, the ResNet-18-shaped network's 19 layers
+// (11 MB) in one launch 268 / 265 us at 8 images (one launch per layer adds about 1.2 us each).
+constexpr int PACK_LAYERS = 32;
+struct PackList {
+    const int8_t* w8[PACK_LAYERS];
+    uint8_t* w4[PACK_LAYERS];
+    long long halves[PACK_LAYERS];
+    unsigned first[PACK_LAYERS + 1];     // first CTA of each layer
+    int count;
+};
+__global__ void __launch_bounds__(256) pack_weights_kernel(const __grid_constant__ PackList list) {
+    pdl_wait();                                                            // the bytes may be the previous launch's, the nibbles its operands
+    int l = 0;
+    while (l + 1 < list.count && blockIdx.x >= list.first[l + 1]) l++;
+    const long long idx = (long long)(blockIdx.x - list.first[l]) * 256 + threadIdx.x;
+    if (idx < list.halves[l]) {
+        uint32_t m = 0, s = 0;
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const uint4 v = __ldg(reinterpret_cast<const uint4*>(w8 + idx * 32) + k);
-        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+        for (int k = 0; k < 2; k++) {
+            const uint4 v = __ldg(reinterpret_cast<const uint4*>(list.w8[l] + idx * 32) + k);
+            const uint32_t q[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int i = 0; i < 16; i++) {
-            const uint32_t b = (q[i >> 2] >> (8 * (i & 3))) & 0xFFu;
-            m |= (b & 1u) << (16 * k + i);
-            s |= (b >> 7) << (16 * k + i);
+            for (int i = 0; i < 16; i++) {
+                const uint32_t b = (q[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+                m |= (b & 1u) << (16 * k + i);
+                s |= (b >> 7) << (16 * k + i);
+            }
         }
+        *reinterpret_cast<uint4*>(list.w4[l] + idx * 16) = nibbles32(m, s & m);
     }
-    *reinterpret_cast<uint4*>(w4 + idx * 16) = nibbles32(m, s & m);
+    pdl_launch_dependents();
 }
 
 template <int WB>
@@ -656,12 +674,25 @@ int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* 
                      : quantize_auto_by_width<1>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream);
 }
 
-int pack_weights_dispatch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, cudaStream_t stream) {
-    const long long halves = (long long)KN * KH * KW * packed_channels(C) * 2;
-    if (halves == 0) return TAB_OK;
-    if (halves >= (1LL << 31) * 256) return TAB_E_TOO_LARGE;
-    pack_weights_kernel<<<(unsigned)((halves + 255) / 256), 256, 0, stream>>>(w8, w4, halves);
-    return check_launch();
+int pack_weights_dispatch(int count, const int8_t* const* w8, uint8_t* const* w4, const long long* words, cudaStream_t stream) {
+    for (int done = 0; done < count;) {
+        PackList list = {};
+        long long blocks = 0;
+        for (; done < count && list.count < PACK_LAYERS; done++) {
+            const long long more = (words[done] * 2 + 255) / 256;
+            if (more >= (1LL << 31)) return TAB_E_TOO_LARGE;
+            if (more == 0) continue;
+            if (blocks + more >= (1LL << 31)) break;                       // the rest goes into another launch
+            const int l = list.count++;
+            list.w8[l] = w8[done]; list.w4[l] = w4[done]; list.halves[l] = words[done] * 2;
+            list.first[l] = (unsigned)blocks;
+            blocks += more;
+        }
+        if (list.count == 0) continue;
+        const int rc = launch_pdl(pack_weights_kernel, dim3((unsigned)blocks), dim3(256), 0, stream, list);
+        if (rc != TAB_OK) return rc;
+    }
+    return TAB_OK;
 }
 
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream) {

@@ -70,8 +70,8 @@ struct QuantExtras {
 int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn, int bits,
                       int N, int H, int W, int C, cudaStream_t stream, const QuantExtras* extras = nullptr, bool in16 = false);
 int expand_weights_dispatch(const int64_t* qw, int8_t* w8, int wbits, int KN, int KH, int KW, int C, cudaStream_t stream);
-// Byte weights {-1,0,+1} -> the 4-bit operands of the same words.
-int pack_weights_dispatch(const int8_t* w8, uint8_t* w4, int KN, int KH, int KW, int C, cudaStream_t stream);
+// Byte weights {-1,0,+1} of `count` layers -> the 4-bit operands of the same words (words[i] = KN*KH*KW*PC of layer i).
+int pack_weights_dispatch(int count, const int8_t* const* w8, uint8_t* const* w4, const long long* words, cudaStream_t stream);
 // Thresholds scale * mean|x[n]| and the bit-planes against them in one launch (sums: N doubles, bar: two words, all zero
 // before and after).
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,

@@ -6,8 +6,8 @@ The reference's only interface is positional ``Conv2d(X, QW, thresholds, btn, ty
 types (cells 12, 17), which reads past the end of ``QW`` (``TAB_GEMM.cu:47-52``).  This module
 
   * quantises the fp32 weights once, at the bitwidth the type needs (``TAB_GEMM.cu:374-379``), keeps ``QW`` and
-    ``BTN_W`` (what ``Conv2d`` takes), the byte-expanded form and the 4-bit form the tensor-core kernel multiplies, so that
-    no call re-expands weights;
+    ``BTN_W`` (what ``Conv2d`` takes) and the byte-expanded form, whose values - as they are at the time of the call, whoever
+    wrote them - every call multiplies;
   * refuses weights quantised at the wrong bitwidth instead of reading out of bounds;
   * computes the per-image activation thresholds ``scale * mean|x|`` when the caller does not pass them;
   * exposes the two stages separately (``quantize`` / ``conv_bits``) so that several convolutions of one input -
@@ -62,25 +62,25 @@ class TABConv2d(torch.nn.Module):
         self.register_buffer("QW", QW.contiguous())
         self.register_buffer("BTN_W", BTN_W.contiguous())
         self.register_buffer("W8", ops.expand_weights(self.QW, wb, self.KN, self.KH, self.KW, self.C))
-        self.register_buffer("W4", None, persistent=False)                  # W8 as the 4-bit operands the kernel multiplies
-        self._pack()
         self._state = None
-
-    def _pack(self):
-        self.W4 = None
-        if self.W8.is_cuda and self.KH * self.KW * self.C < 1 << 24:       # beyond that the byte form is multiplied
-            self.W4 = ops.pack_weights(self.W8, self.KN, self.KH, self.KW, self.C)
-
-    def _load_from_state_dict(self, *args, **kwargs):
-        super()._load_from_state_dict(*args, **kwargs)
-        self._pack()
 
     def __setstate__(self, state):
         super().__setstate__(state)
-        if "W4" not in self._buffers:                                      # pickled before there was one
-            self._non_persistent_buffers_set.add("W4")
-            self._buffers["W4"] = None
-            self._pack()
+        self._buffers.pop("W4", None)                                      # a derived form that pickles of older versions hold
+        self._non_persistent_buffers_set.discard("W4")
+
+    def _four_bit(self):
+        """Whether the bytes are multiplied as 4-bit operands (else, for very long sums, as they are)."""
+        return self.KH * self.KW * self.C < 1 << 24
+
+    @staticmethod
+    def pack_together(convs):
+        """For a pass through several layers, name -> layer: name -> keywords for its ``conv_bits``, which then need not pack
+        the weights by itself.  One launch for all of them instead of one per layer; the packed forms are of ``W8`` as it is
+        now and serve this pass only."""
+        own = [(k, c._buffers["W8"]) for k, c in convs.items() if isinstance(c, TABConv2d) and type(c).conv_bits is TABConv2d.conv_bits and c._four_bit()]
+        packed = ops.pack_weights_many([w for _, w in own])
+        return {} if packed is None else {k: {"packed": p} for (k, _), p in zip(own, packed)}
 
     @classmethod
     def from_float(cls, weight, conv_type, padding=(0, 0), stride=(1, 1), weight_thresholds=None, threshold_scale=0.7):
@@ -127,22 +127,24 @@ class TABConv2d(torch.nn.Module):
         N, H, W = (int(v) for v in x.shape[:3])
         return ops.quantize_auto(x, self.threshold_scale, act_bitwidth(self.conv_type), N, H, W, self.C, self.state(N, x.device))
 
-    def conv_bits(self, QX, N, H, W, residual=None, next_threshold_scale=None, state=None, out_int16=False, next_bitwidth=None):
+    def conv_bits(self, QX, N, H, W, residual=None, next_threshold_scale=None, state=None, out_int16=False, next_bitwidth=None, packed=None):
         """GEMM stage on quantised activations.  Returns ``(Y, next_thresholds_or_None)``.  ``out_int16``: ``Y`` as int16
         where that is possible (no residual, or one of int16 with which the caller knows the sum to fit; KH*KW*C <= 32767, a
         shape the tensor-core kernel covers), else fp32 as usual: look at ``Y.dtype``.  ``next_bitwidth`` (with ``next_threshold_scale``): a third value is returned, ``Y`` quantised
-        against the next thresholds at that bitwidth - the next convolution's ``QX`` - from the same launch."""
+        against the next thresholds at that bitwidth - the next convolution's ``QX`` - from the same launch.  ``packed``: the
+        current weights as ``pack_together`` gave them (the call then saves the launch that packs them)."""
         if next_threshold_scale is not None and state is None:
             state = self.state(N, QX.device)
         if next_bitwidth is not None and next_threshold_scale is None:
             raise ValueError("next_bitwidth needs next_threshold_scale")
         res16 = residual is not None and residual.dtype == torch.int16
-        if res16 and self.W4 is None:
+        four = self._four_bit()
+        if res16 and not four:
             residual, res16 = residual.float(), False
         compact = out_int16 and (residual is None or res16) and self.KH * self.KW * self.C <= 32767
         try:
-            return ops.conv2d_bits(QX, self.W8 if self.W4 is None else self.W4, self.conv_type, *self.geometry(N, H, W), residual=residual,
-                                   threshold_scale=next_threshold_scale, state=state, out_int16=compact, next_bitwidth=next_bitwidth)
+            return ops.conv2d_bits(QX, self.W8 if packed is None or not four else packed, self.conv_type, *self.geometry(N, H, W), residual=residual,
+                                   threshold_scale=next_threshold_scale, state=state, out_int16=compact, next_bitwidth=next_bitwidth, pack=four)
         except _cabi.TabError as exc:
             if exc.code != -5:
                 raise

@@ -8,6 +8,8 @@ raise instead of returning a partially written tensor (``TAB_GEMM.cu:292-321``).
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from . import _cabi
@@ -19,7 +21,7 @@ _native = None
 def _host():
     """``tab_b200._host``, the same bodies in native code (a call costs the host microseconds there and tens of them here), or
     ``False`` when only the C-ABI library has been built.  Its functions return ``None`` for anything they do not take - the
-    bodies below then run, and say what is wrong."""
+    bodies below then run, and say what is wrong (``conv2d_packed4`` also the code of a shape that is not covered)."""
     global _native
     if _native is None:
         try:
@@ -212,6 +214,26 @@ def pack_weights(W8, KN, KH, KW, C):
     return w4
 
 
+def pack_weights_many(W8s):
+    """``pack_weights`` of several layers' bytes in one launch: flat uint8 tensors, parts of one allocation - or ``None`` where
+    they are anything but contiguous int8 tensors of whole 64-channel words on one CUDA device."""
+    W8s = list(W8s)
+    done = _try("pack_weights", W8s)
+    if done is not None:
+        return done
+    if not W8s or not all(isinstance(w, torch.Tensor) and w.is_cuda and w.is_contiguous() and w.dtype == torch.int8 and w.numel() and
+                          w.numel() % 64 == 0 and w.device == W8s[0].device and w.data_ptr() % 16 == 0 for w in W8s):
+        return None
+    with torch.cuda.device(W8s[0].device):
+        sizes = [w.numel() // 2 for w in W8s]
+        w4 = torch.empty((sum(sizes),), dtype=torch.uint8, device=W8s[0].device).split(sizes)
+        pointers = lambda ts: (ctypes.c_void_p * len(ts))(*(t.data_ptr() for t in ts))
+        rc = _cabi.lib().tab_pack_weights_many_launch(len(W8s), pointers(W8s), pointers(w4), (ctypes.c_longlong * len(W8s))(*(n // 32 for n in sizes)),
+                                                      _stream_ptr(W8s[0].device))
+    _cabi.check(rc, "tab_pack_weights_many_launch")
+    return list(w4)
+
+
 def new_state(N, device):
     """Zeroed state block for ``conv2d_bits(..., threshold_scale=...)``; one block serves any number of calls that are
     ordered on a stream (every call leaves it zeroed)."""
@@ -258,9 +280,10 @@ def quantize_i16(X16, thresholds, bitwidth, N, H, W, C):
 
 
 def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW,
-                residual=None, threshold_scale=None, state=None, out_int16=False, next_bitwidth=None):
+                residual=None, threshold_scale=None, state=None, out_int16=False, next_bitwidth=None, pack=False):
     """The GEMM stage on the tensor cores: activations as ``Quantize`` wrote them (bitwidth 2 for types 0,1; 1 for
-    types 2,3), weights from ``expand_weights`` (int8) or ``pack_weights`` (uint8: twice the rate, KH*KW*C < 2**24).  Returns
+    types 2,3), weights from ``expand_weights`` (int8) or ``pack_weights`` (uint8: twice the rate, KH*KW*C < 2**24); with
+    ``pack`` int8 weights are packed by a launch of this call and multiplied like uint8 ones.  Returns
     ``(Y, next_thresholds_or_None)``; ``Y = conv + residual``.
     ``threshold_scale`` needs ``state`` (``new_state``).  ``out_int16``: ``Y`` as int16 (no residual; the values are
     integers of magnitude at most KH*KW*C) for ``quantize_i16``.  With uint8 weights the residual may be int16 too, and then so
@@ -268,12 +291,16 @@ def conv2d_bits(QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, 
     launch also quantises ``Y`` against the next thresholds at that bitwidth and a third value is returned, ``QX`` of the
     next convolution (``[N,OH,OW,ceil(KN/64),bits]`` int64, what ``Quantize(Y, next_thresholds, ...)`` gives).
     Raises ``TabError`` (TAB_E_TOO_LARGE) for shapes the tensor-core kernel does not cover."""
-    if isinstance(W8, torch.Tensor) and W8.dtype == torch.uint8:
+    if isinstance(W8, torch.Tensor) and (W8.dtype == torch.uint8 or (pack and W8.dtype == torch.int8)):
         done = _try("conv2d_packed4", QX, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW,
                     residual, threshold_scale, state, out_int16, next_bitwidth)
+        if isinstance(done, int):                                          # valid arguments the tensor-core kernel does not cover
+            _cabi.check(done, "tab_conv2d_packed4_launch")
         if done is not None:
             return done
     _check_input(QX, "QX", torch.int64)
+    if pack and isinstance(W8, torch.Tensor) and W8.dtype == torch.int8:
+        W8 = pack_weights(W8, int(KN), int(KH), int(KW), C)
     packed4 = isinstance(W8, torch.Tensor) and W8.dtype == torch.uint8
     _check_input(W8, "W8", torch.uint8 if packed4 else torch.int8)
     conv_type = int(type)

@@ -153,3 +153,76 @@ def test_module_weights_follow_a_loaded_state(cuda):
     assert sorted(a.state_dict()) == ["BTN_W", "QW", "W8"] and not torch.equal(a(x), b(x))
     b.load_state_dict(a.state_dict())
     assert torch.equal(a(x), b(x))
+
+
+def _pair(cuda, N=2, H=10, W=9, C=70, KN=40):
+    """An input and two layers of one geometry with different weights."""
+    make = lambda: tab_nn.TABConv2d.from_float(torch.randn(KN, 3, 3, C, device=cuda), 0, 1, 1)
+    return torch.randn(N, H, W, C, device=cuda), make(), make()
+
+
+@pytest.mark.parametrize("write", [
+    lambda a, b: a.W8.copy_(b.W8),
+    lambda a, b: a.state_dict()["W8"].copy_(b.W8),
+    lambda a, b: a.W8.data.copy_(b.W8),                                    # no version counter sees this one
+    lambda a, b: a.W8.data.view(torch.int64).copy_(b.W8.view(torch.int64)),
+    lambda a, b: setattr(a, "W8", b.W8.clone()),
+    lambda a, b: a._buffers.__setitem__("W8", b.W8),
+], ids=["copy_", "state_dict", "data", "reinterpreted", "assigned", "buffers"])
+def test_module_multiplies_the_registered_weights(cuda, write):
+    """``W8`` is what a call multiplies, whoever wrote it and however; also the one pass that packs all layers at once."""
+    x, a, b = _pair(cuda)
+    old, want = a(x), b(x)
+    assert not torch.equal(old, want)
+    write(a, b)
+    assert torch.equal(a(x), want)
+    assert "e2m1" in _cabi.lib().tab_last_conv_kernel().decode()
+    kw = tab_nn.TABConv2d.pack_together({"a": a, "b": b})
+    qx = a.quantize(x)
+    assert sorted(kw) == ["a", "b"]
+    for k in kw:
+        assert torch.equal(a.conv_bits(qx, 2, 10, 9, **kw[k])[0], want)
+    from tab_b200 import ops
+    saved, ops._native = ops._native, False
+    try:                                                                   # the Python body of the same
+        for w, k in zip(ops.pack_weights_many([a.W8, b.W8]), kw):
+            assert torch.equal(w, kw[k]["packed"])
+        assert torch.equal(a(x), want)
+    finally:
+        ops._native = saved
+    assert ops.pack_weights_many([a.W8, b.W8.cpu()]) is None and ops.pack_weights_many([]) is None
+
+
+def test_captured_module_follows_its_weights(cuda):
+    """A captured pass multiplies what ``W8`` holds when it is replayed, as it did when ``W8`` itself was the operand."""
+    x, a, b = _pair(cuda)
+    want = b(x)
+    a(x)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        y = a(x)
+    a.W8.copy_(b.W8)
+    g.replay()
+    assert torch.equal(y, want)
+    a.load_state_dict(tab_nn.TABConv2d.from_float(torch.randn(40, 3, 3, 70, device=cuda), 0, 1, 1).state_dict())
+    g.replay()
+    assert torch.equal(y, a(x)) and not torch.equal(y, want)
+
+
+def test_module_copies_and_moves(cuda):
+    """Deep copies, pickles (also ones that hold the derived form older versions kept) and weights that were loaded while the
+    module was on the CPU give the same results on the same kernel."""
+    import copy
+    import pickle
+    x, a, b = _pair(cuda)
+    want = a(x)
+    old = pickle.loads(pickle.dumps(a))
+    old._buffers["W4"] = torch.zeros(8, dtype=torch.uint8, device=cuda)
+    old._non_persistent_buffers_set.add("W4")
+    b.cpu()
+    b.load_state_dict(a.state_dict())
+    b.to(cuda)
+    for m in (copy.deepcopy(a), pickle.loads(pickle.dumps(old)), b):
+        assert torch.equal(m(x), want) and "e2m1" in _cabi.lib().tab_last_conv_kernel().decode()
+        assert [n for n, _ in m.named_buffers()] == ["QW", "BTN_W", "W8"]
