@@ -1199,7 +1199,9 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
         unsigned a = 0, blk = 0;
         bool dead = false;
         PendingSums pending;
-        if (has_res && lane == 0) {                                        // the residual of the warp's first block
+        // The residual of the warp's first block.  A warp without columns (tiles of 32 filters: the second of the two that share a
+        // row block) has none: nothing would wait for the copy, and the CTA could exit with it under way.
+        if (has_res && lane == 0 && ec0 < ec1) {
             TepiIter first = {cta0, ec0};
             first.settle(ec0, step, ntiles, tiles_n, tnw, p.KN);
             if (first.t < ntiles) tepi_request_residual(&tmR, tepi_box(p, slab_row(first.t), (first.t % tiles_n) * tnw + first.cb), sbuf, mres);

@@ -8,7 +8,7 @@ import pytest
 import torch
 
 import tab_b200 as TAB
-from tab_b200 import _cabi, chain
+from tab_b200 import _cabi, chain, nn as tab_nn
 from oracle import c_oracle, tab_oracle as O
 from oracle.oracle_ops import OracleOps
 from util import make_input
@@ -810,3 +810,32 @@ def test_packed4_sums_are_exact_at_large_magnitude(cuda, conv_path):
     y = TAB.Conv2d(x, q[0], one, q[1], 0, 0, 0, 1, 1, N, H, W, C, KN, K, K)
     want = (x.double().reshape(1, -1) @ w.double().reshape(KN, -1).T).reshape(-1)
     assert torch.equal(y.double().reshape(-1), want)
+
+
+@pytest.mark.parametrize("geom", [
+    # p1 p2 s1 s2  N  H  W   C   KN KH KW       two tiles of 32 filters (a small image, 33 to 64 filters, 32 words or more per sum)
+    (3, 3, 1, 1, 1, 16, 16, 20, 64, 7, 7),
+    (3, 3, 1, 1, 1, 16, 16, 20, 36, 7, 7),
+    (3, 3, 1, 1, 1, 28, 28, 16, 64, 7, 7),
+    (3, 3, 1, 1, 1, 9, 13, 3, 60, 7, 7),
+])
+@pytest.mark.parametrize("t", [0, 3])
+def test_tma_epilogue_on_tiles_of_32_filters(cuda, geom, t, conv_path):
+    """The TMA epilogue where only half of its warps have columns: fp32 residuals, next thresholds, the next layer's input, and
+    the same without a residual (the other epilogue)."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    test_packed4_weights(cuda, geom, t, conv_path)
+    p1, p2, s1, s2, N, H, W, C, KN, KH, KW = geom
+    x, ths = make_input(93, N, H, W, C)
+    w, wths = make_input(94, KN, KH, KW, C)
+    qw, btn = O.quantize(w, wths, O.weight_bits(t), KN, KH, KW, C)
+    m = tab_nn.TABConv2d(dev_t(qw, cuda), dev_t(btn, cuda), t, KN, KH, KW, C, (p1, p2), (s1, s2))
+    yo = c_oracle.conv2d(x, qw, ths, btn, t, *geom)
+    r = np.random.default_rng(3).standard_normal(yo.shape).astype(np.float32)
+    for _ in range(3):
+        y, nxt = m.conv_bits(m.quantize(dev_t(x, cuda), dev_t(ths, cuda)), N, H, W, residual=dev_t(r, cuda), next_threshold_scale=0.7)
+        assert np.array_equal(y.cpu().numpy(), yo + r)
+        want = np.float32(np.float64(np.float32(0.7)) * np.abs((yo + r).astype(np.float64)).sum() / yo.size)
+        assert abs(nxt.item() - want) <= 2 * np.spacing(want)              # compensated sums: good to far less than the last place
+    assert ",2,1" in _cabi.lib().tab_last_conv_kernel().decode()           # residual, TMA epilogue
