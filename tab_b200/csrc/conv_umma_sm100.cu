@@ -791,7 +791,7 @@ template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = 
 __global__ void __launch_bounds__(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1), 1)
 conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_constant__ CUtensorMap tmY, const __grid_constant__ CUtensorMap tmR,
                          const TcConvParams p, int* __restrict__ status,
-                         const int prow, const int nrows, const int nst, const int tiles_m, const int tiles_n, const int split_from, const int tnw) {
+                         const int prow, const int nrows, const int nst, const int tiles_m, const int tiles_n, const int split_from, const int tnw, const int base_slack) {
     static_assert(!PAIR || (MT == 1 && !BRES && !TEPI), "CTA pairs: one row block per CTA, streamed filters, transposing epilogue");
     constexpr bool SPLIT = split_capable(MT, TNI, BRES, TEPI, PAIR);
     const int brows = PAIR ? tnw / 2 : tnw;                                // filters of a slice this CTA holds
@@ -808,10 +808,13 @@ conv_umma_persist_kernel(const __grid_constant__ CUtensorMap tmB, const __grid_c
     static_assert(SB <= 8, "eight ring barriers are laid out");
     extern __shared__ unsigned char smem_raw[];
     const uint32_t raw = (uint32_t)__cvta_generic_to_shared(smem_raw);
-    const uint32_t sbase = raw;
-    unsigned char* smem = smem_raw;
-    if (raw & 1023u) {                                                     // never: see plan_shape
+    // The swizzled tiles need a 1024-byte boundary.  Dynamic shared memory starts on one as long as nothing lies before it; where
+    // something does, the tiles move up by what the launch has to spare (base_slack, see dynamic_smem).
+    const uint32_t sbase = (raw + 1023u) & ~1023u;
+    unsigned char* smem = smem_raw + (sbase - raw);
+    if (sbase - raw > (uint32_t)base_slack) {                              // (only a plan without a spare kilobyte can get here)
         if (threadIdx.x == 0 && status) atomicExch(status, 19);
+        pdl_wait();                                                        // what follows in the stream may rely on what came before
         return;
     }
     const uint32_t sPatch = sbase;                                         // [2][prow][128 B], prow % 8 == 0
@@ -1558,8 +1561,7 @@ static long long split_point(long long ntiles, int sms, bool capable) {
 static bool plan_shape(const TcConvParams& p, int sms, int mt, int tn, int sb, TcPlan* out, bool pair = false, int most = 0) {
     const long long halo = (long long)((p.KH - 1) / p.s1) * p.VW + (p.KW - 1) / p.s2;
     const long long nrows = 128LL * mt + halo, prow = (nrows + 7) / 8 * 8;
-    // patches, barriers, epilogue buffers (none where every block leaves straight from registers).  Dynamic shared memory starts
-    // on a 1024-byte boundary (no static shared memory in the kernel); the kernel checks that.
+    // patches, barriers, epilogue buffers (none where every block leaves straight from registers)
     const bool staged = !(p.wide && p.KN % 32 == 0 && (p.residual || p.residual16 || p.y16));
     const long long fixed = 2 * prow * IROW + 1024 + 8 * (p.tepi ? 8192 : (staged ? 4096 : 0));
     const int tlog = resident_taps_log2(p.PC, p.e2m1 != 0), wpr = p.e2m1 ? 4 : 2;
@@ -1674,6 +1676,12 @@ static bool tc_prepare(TcConvParams& p, int sms, TcPlan* pl) {
     return true;
 }
 
+// Dynamic shared memory of a launch: the plan's, and up to a kilobyte for the kernel to round its base up with where the SM has
+// it left.  A plan that fills the SM to the last kilobyte (16x112x112x256 -> 64 keeps its filters resident that way, 65 us; with
+// a reserved kilobyte they would have to stream) relies on the base being aligned already, which holds while the kernel has no
+// static shared memory - and with any, cudaFuncSetAttribute refuses UMMA_SMEM_MAX.
+static int dynamic_smem(const TcPlan& pl) { return std::min(pl.smem + 1024, UMMA_SMEM_MAX); }
+
 template <int MT, int TNI, int SB, bool BRES, int FUSED, bool TEPI, bool PAIR = false, bool E2M1 = false>
 static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, const CUtensorMap& tmR, const TcConvParams& p, const TcPlan& pl,
                             int sms, int* status, cudaStream_t stream) {
@@ -1694,13 +1702,13 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
     if (PAIR) {
         const long long pairs = std::min<long long>(sms / 2, pair_clusters());
         const unsigned grid = 2u * (unsigned)(ntiles < pairs ? ntiles : pairs);
-        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)pl.smem, stream, 2u,
-                                  tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles, pl.tnw);
+        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)dynamic_smem(pl), stream, 2u,
+                                  tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles, pl.tnw, dynamic_smem(pl) - pl.smem);
     }
     const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);
     const long long split_from = split_point(ntiles, sms, split_capable(MT, TNI, BRES, TEPI, PAIR) && pl.tnw % 64 == 0);
-    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)pl.smem, stream,
-                      tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)split_from, pl.tnw);
+    return launch_pdl(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)dynamic_smem(pl), stream,
+                      tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)split_from, pl.tnw, dynamic_smem(pl) - pl.smem);
 }
 
 template <int MT, int TNI, int SB, bool E2M1>
