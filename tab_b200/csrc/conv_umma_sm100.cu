@@ -676,6 +676,11 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                     }
                     const double a = (double)((f0 + f1) + (f2 + f3));
                     if (lane < sr.split) dsum0 += a; else dsum1 += a;
+                } else if (has_res && want_sum && !sr.fast) {              // term by term in double: infinite or huge residuals too
+                    double a0 = 0.0, a1 = 0.0;
+#pragma unroll
+                    for (int j = 0; j < 32; j += 2) { a0 += (double)fabsf(__uint_as_float(v[j])); a1 += (double)fabsf(__uint_as_float(v[j + 1])); }
+                    if (sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, a0 + a1);
                 } else if (has_res && want_sum) {
                     // the residual need not be integer-valued: compensated (Kahan) float sums, four chains, whose value and
                     // compensation go to the double totals (good to about 1e-14 of the total)
@@ -688,8 +693,7 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                         s4[k] = tv;
                     }
                     const double a = (((double)s4[0] + (double)s4[1]) + ((double)s4[2] + (double)s4[3])) - (((double)c4[0] + (double)c4[1]) + ((double)c4[2] + (double)c4[3]));
-                    if (!sr.fast) { if (sr.n_own < p.N) atomicAdd(p.abs_sums + sr.n_own, a); }
-                    else if (lane < sr.split) dsum0 += a;
+                    if (lane < sr.split) dsum0 += a;
                     else dsum1 += a;
                 }
             }

@@ -839,3 +839,28 @@ def test_tma_epilogue_on_tiles_of_32_filters(cuda, geom, t, conv_path):
         want = np.float32(np.float64(np.float32(0.7)) * np.abs((yo + r).astype(np.float64)).sum() / yo.size)
         assert abs(nxt.item() - want) <= 2 * np.spacing(want)              # compensated sums: good to far less than the last place
     assert ",2,1" in _cabi.lib().tab_last_conv_kernel().decode()           # residual, TMA epilogue
+
+
+@pytest.mark.parametrize("H,KN", [(2, 128), (2, 33), (2, 72), (1, 100)])
+def test_thresholds_of_small_images_with_extreme_residuals(cuda, H, KN, conv_path):
+    """Images of so few positions that 32 rows of the grid span three, residuals that are infinite or whose sum leaves the range of
+    float: the sums of |y| are taken in double, so the next thresholds are infinite there and finite here."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    N, C, K = 40, 64, 3
+    x, ths = make_input(5, N, H, H, C)
+    w, wths = make_input(6, KN, K, K, C)
+    qw, btn = O.quantize(w, wths, 2, KN, K, K, C)
+    geom = (1, 1, 1, 1, N, H, H, C, KN, K, K)
+    yo = c_oracle.conv2d(x, qw, ths, btn, 0, *geom).reshape(N, -1)
+    r = np.random.default_rng(1).standard_normal(yo.shape).astype(np.float32)
+    r[1, 5] = np.inf
+    r[2, :] = 3e38
+    r[3, 0], r[3, 1] = -np.inf, np.inf
+    want = (np.float64(np.float32(0.7)) * np.abs((yo + r).astype(np.float64)).sum(axis=1) / yo.shape[1]).astype(np.float32)
+    qx = TAB.Quantize(dev_t(x, cuda), dev_t(ths, cuda), 2, N, H, H, C)[0]
+    w8 = TAB.ops.expand_weights(dev_t(qw, cuda), 2, KN, K, K, C)
+    for weights in (w8, TAB.ops.pack_weights(w8, KN, K, K, C)):
+        y, nxt = TAB.ops.conv2d_bits(qx, weights, 0, *geom, residual=dev_t(r, cuda), threshold_scale=0.7, state=TAB.ops.new_state(N, cuda))
+        assert np.array_equal(y.cpu().numpy().reshape(N, -1), yo + r)
+        assert np.array_equal(np.isinf(nxt.cpu().numpy()), np.isinf(want)) and np.allclose(nxt.cpu().numpy(), want, rtol=2e-7, atol=0)
