@@ -37,7 +37,8 @@ enum {
     TAB_E_WORKSPACE = -3,      /* workspace smaller than tab_conv2d_workspace_bytes() or misaligned */
     TAB_E_CUDA = -4,           /* the CUDA runtime reported an error; see tab_last_cuda_error() */
     TAB_E_TOO_LARGE = -5,      /* a size exceeds what an entry point supports */
-    TAB_E_ALIGNMENT = -6       /* a pointer is not aligned to its element type */
+    TAB_E_ALIGNMENT = -6,      /* a pointer is not aligned to its element type */
+    TAB_E_STALLED = -7         /* a bounded wait of an earlier launch on the device ran out; see tab_device_status() */
 };
 
 /* Human-readable text for a TAB_E_* code (static storage). */
@@ -85,11 +86,12 @@ int tab_conv2d_set_path(int path);
 const char* tab_last_conv_kernel(void);
 /*
  * Every wait inside the tensor-core kernel and inside tab_quantize_auto_launch's kernel is bounded; a wait that ran out makes
- * the kernel record a code and return early, leaving its outputs incomplete.  This call synchronises the current device,
- * returns that code (0 = none; 11-19: a role of the tensor-core kernel gave up on an mbarrier; 21, 22: the grid-wide
- * meeting point of tab_conv2d_bits_next_launch / tab_quantize_auto_launch, which needs the launch's CTAs resident together -
- * other work occupying the device for tenths of a second can cause it) and clears it.  A non-zero code invalidates the
- * outputs of every launch on the device since the previous call.
+ * the kernel record a code and return early, leaving its outputs incomplete (a state block is zero again all the same).  From
+ * then on the entry points that launch these kernels return TAB_E_STALLED, until this call: it synchronises the current device,
+ * returns the code and clears it (0 = none; 11-19: a role of the tensor-core kernel gave up on an mbarrier; 21: the grid-wide
+ * meeting point of tab_conv2d_bits_next_launch, whose CTAs - one per SM at most - wait for one another: other work that occupies
+ * SMs for a second can cause it; 22: that of tab_quantize_auto_launch, a cooperative launch, whose CTAs run at the same time
+ * whatever other streams do).  A non-zero code invalidates the outputs of every launch on the device since the previous call.
  */
 int tab_device_status(void);
 

@@ -65,6 +65,7 @@ const char* tab_error_string(int code) {
         case TAB_E_CUDA: return "CUDA runtime error (see tab_last_cuda_error)";
         case TAB_E_TOO_LARGE: return "problem size exceeds the supported range";
         case TAB_E_ALIGNMENT: return "pointer not aligned as the entry point requires";
+        case TAB_E_STALLED: return "a bounded wait of an earlier launch ran out and its outputs are void (tab_device_status tells which and clears this)";
         default: return "unknown error code";
     }
 }
@@ -347,7 +348,9 @@ int tab_quantize_auto_launch(const float* x, float scale, void* state, float* th
     if ((long long)H * W >= (1LL << 31)) return TAB_E_TOO_LARGE;
     double* sums = reinterpret_cast<double*>(state);
     unsigned* bar = reinterpret_cast<unsigned*>(sums + N) + 1;
-    return quantize_auto_dispatch(x, scale, sums, bar, ths, qx, bitwidth == 1 ? 1 : 2, N, H, W, C, device_status_word(), s);
+    int* status = device_status_word();
+    if (stalled(status)) return TAB_E_STALLED;
+    return quantize_auto_dispatch(x, scale, sums, bar, ths, qx, bitwidth == 1 ? 1 : 2, N, H, W, C, status, s);
 }
 
 int tab_quantize_i16_launch(const int16_t* x, const float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C, tab_stream_t stream) {

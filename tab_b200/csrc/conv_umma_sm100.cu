@@ -107,11 +107,13 @@ __device__ __forceinline__ void fused_finish(const TcConvParams& p) {
 // ---- second phase: the grid quantises its own result for the next convolution ------------------------------------------
 // Replaces, for a chained layer, the quantiser launch of the next convolution (TerOnlyKernel / BinOnlyKernel,
 // TAB_GEMM.cu:163-247, same encoding).  Every CTA first reports in at a grid-wide counter - all CTAs of the launch are
-// resident (one per SM at most), so the wait is for CTAs that are running; it is bounded all the same - then computes the
+// resident (one per SM at most), so the wait is for CTAs that are running or will as soon as what holds their SM ends; it is
+// bounded all the same (as cooperative launches, which would guarantee it, these cost the host 2.4 us more each: the
+// ResNet-18-shaped network at 8 images 282 -> 315 us) - then computes the
 // thresholds of all images from the complete |y| sums (the arithmetic of fused_finish), and the CTAs share the words of
 // the result, last word first (the end of the tensor is what was written last).  Data written by other SMs in this
 // launch is read with L2-coherent loads.
-constexpr uint32_t GRID_WAIT_LIMIT = 1u << 22;                             // x ~100 ns
+constexpr uint32_t GRID_WAIT_LIMIT = 1u << 21;                             // a second or two
 
 __device__ __forceinline__ float4 ld_cg_f4(const float* ptr) {
     float4 r;
@@ -184,8 +186,8 @@ __device__ __noinline__ void quantize_tail(const QuantTailArgs p, float* ths_sme
         if (!ok && status) atomicExch(status, 21);
         flag = ok ? 1 : 0;
     }
-    if (!__syncthreads_or(flag)) return;                                   // the result of the launch is void; the status says so
-    for (int n = tid; n < p.N; n += (int)blockDim.x) {
+    const bool met = __syncthreads_or(flag);                               // else the result of the launch is void; the status says so
+    for (int n = tid; met && n < p.N; n += (int)blockDim.x) {
         const double sum = __ldcg(p.abs_sums + n);
         const float t = (float)((double)p.ths_scale * (sum / p.per_image));
         ths_smem[n] = t;
@@ -202,7 +204,7 @@ __device__ __noinline__ void quantize_tail(const QuantTailArgs p, float* ths_sme
     // words of the result: word w = 64 consecutive channels = elements [64 w, 64 w + 64) of y; 8 lanes per word, 64 words
     // per pass of the CTA, UN passes per step with all loads of a step issued before the first is used (addresses are one
     // base register plus constants)
-    if (tid >= 512) return;                                                // 64 words per pass: 512 threads (kernels with extra warps have more)
+    if (!met || tid >= 512) return;                                        // 64 words per pass: 512 threads (kernels with extra warps have more)
     const int PC2 = p.KN >> 6, bits = p.next_bits, byte = tid & 7;
     const uint32_t grp = (uint32_t)tid >> 3;
     const uint32_t words = (uint32_t)((long long)p.M * PC2);               // < 2^31, checked on the host
@@ -1484,9 +1486,8 @@ static bool make_map_4d(CUtensorMap* m, const void* base, int KN, int OW, int OH
     return true;
 }
 
-// Where an expired wait is recorded (0 = never).  In host code the name is only a symbol handle; the device
-// address is looked up once per device, under a lock.
-static __device__ int g_umma_status;
+// Where an expired wait is recorded (0 = never): a word of pinned host memory per device, which kernels write in place and the
+// next launch looks at.  Allocated by the first call on a device, under a lock.
 static int* umma_status_ptr() {
     static std::mutex mu;
     static int* addr[64] = {};
@@ -1494,8 +1495,12 @@ static int* umma_status_ptr() {
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return nullptr;
     std::lock_guard<std::mutex> lock(mu);
     if (!addr[dev]) {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;         // the allocation has nothing to do with what a thread may be capturing
         void* ptr = nullptr;
-        if (cudaGetSymbolAddress(&ptr, g_umma_status) != cudaSuccess) return nullptr;
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (cudaHostAlloc(&ptr, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable) != cudaSuccess) { cudaGetLastError(); ptr = nullptr; }
+        cudaThreadExchangeStreamCaptureMode(&mode);
+        if (ptr) *static_cast<volatile int*>(ptr) = 0;
         addr[dev] = static_cast<int*>(ptr);
     }
     return addr[dev];
@@ -1505,9 +1510,11 @@ int* device_status_word() { return umma_status_ptr(); }
 
 // Reads (and clears) the record of expired waits on the current device; synchronises the device.
 int umma_status_read_and_clear() {
-    int v = -1, zero = 0;
-    if (cudaMemcpyFromSymbol(&v, g_umma_status, sizeof(int)) != cudaSuccess) return -1;
-    cudaMemcpyToSymbol(g_umma_status, &zero, sizeof(int));
+    if (cudaDeviceSynchronize() != cudaSuccess) return -1;
+    volatile int* word = umma_status_ptr();
+    if (!word) return -1;
+    const int v = *word;
+    *word = 0;
     return v;
 }
 
@@ -1706,7 +1713,7 @@ static int launch_persist_u(const CUtensorMap& tmB, const CUtensorMap& tmY, cons
     if (PAIR) {
         const long long pairs = std::min<long long>(sms / 2, pair_clusters());
         const unsigned grid = 2u * (unsigned)(ntiles < pairs ? ntiles : pairs);
-        return launch_pdl_cluster(conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)dynamic_smem(pl), stream, 2u,
+        return launch_pdl_as(false, 2u, conv_umma_persist_kernel<MT, TNI, SB, BRES, FUSED, TEPI, PAIR, E2M1>, dim3(grid), dim3(PTHREADS + 32 * extra_warps(FUSED, TEPI, TNI, E2M1)), (size_t)dynamic_smem(pl), stream,
                                   tmB, tmY, tmR, p, status, pl.prow, pl.nrows, pl.nst, (int)pl.tiles_m, (int)pl.tiles_n, (int)ntiles, pl.tnw, dynamic_smem(pl) - pl.smem);
     }
     const unsigned grid = (unsigned)(ntiles < sms ? ntiles : sms);
@@ -1817,6 +1824,7 @@ int tc_conv_dispatch(TcConvParams p, cudaStream_t stream) {
         if (p.residual && !make_map_4d(&tmR, p.residual, p.KN, p.OW, p.OH, p.N, bw, bh)) return TAB_E_TOO_LARGE;
     }
     int* status = umma_status_ptr();
+    if (stalled(status)) return TAB_E_STALLED;
     const bool halves = split_point(pl.tiles_m * pl.tiles_n, sms, half_box && !pl.pair && pl.tnw % 64 == 0) < pl.tiles_m * pl.tiles_n;
     snprintf(g_last_kernel, sizeof(g_last_kernel), "conv_umma_persist_kernel<%d,%d,%d,%d,%d,%d%s> grid %dx%d%s%s", pl.mt, pl.tn, pl.sb, (int)pl.resident,
              p.residual16 ? 3 : (p.residual ? 2 : (p.abs_sums ? 1 : 0)), p.tepi, pl.pair ? ",pair" : (p.e2m1 ? ",e2m1" : ""), p.VH, p.VW, halves ? " halves" : "", p.next_qx ? " +next" : "");

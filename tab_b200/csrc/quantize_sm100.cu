@@ -504,12 +504,12 @@ int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn
 // ---- thresholds and bit-planes of a tensor in one launch ----------------------------------------------------------------
 // What every caller of Quantize does first - thresholds[n] = scale * mean|x[n]| (the reference leaves it to framework ops) -
 // and the quantisation against them, as two phases of one persistent grid: per-image sums of |x| (double atomics), a
-// grid-wide counter (all CTAs are resident: the grid is sized by the occupancy calculator; the wait is bounded and
-// reports in *status), then every CTA quantises, last unit first, the units it has just summed - the end of its share is
+// grid-wide counter (all CTAs are resident: the grid is sized by the occupancy calculator and launched cooperatively; the wait is
+// bounded and reports in *status), then every CTA quantises, last unit first, the units it has just summed - the end of its share is
 // what the L2 still holds, and its last unit is still in registers.  A unit is one CTA step (QUNROLL passes) of one image; a
 // CTA owns consecutive units, so that its sum leaves the registers once per image and not once per unit.
 // FULL: C % 64 == 0 and 32-byte rows (every lane has eight real channels); else V and L as in quantize_any_kernel.
-constexpr uint32_t QA_WAIT_LIMIT = 1u << 22;
+constexpr uint32_t QA_WAIT_LIMIT = 1u << 21;                               // a second or two; the slowest CTA of 180 GB of input needs 30 ms
 
 template <int BITS, int V, int L, bool FULL>
 __global__ void __launch_bounds__(QTHREADS, 4)
@@ -584,13 +584,13 @@ quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restric
         if (!ok && status) atomicExch(status, 22);
         flag = ok ? 1 : 0;
     }
-    if (!__syncthreads_or(flag)) return;
-    if (blockIdx.x == 0 && ths_out)
+    const bool met = __syncthreads_or(flag);                               // else the result of the launch is void; the status says so
+    if (met && blockIdx.x == 0 && ths_out)
         for (int m = threadIdx.x; m < N; m += QTHREADS) ths_out[m] = (float)((double)scale * (__ldcg(sums + m) / per_image));
     // phase 2: the CTA's units again, last first (v still holds the last one)
     long long tn = -1;
     float t = 0.f;
-    for (long long u = ue - 1; u >= ub; u--) {
+    for (long long u = ue - 1; met && u >= ub; u--) {
         if (u != ue - 1) {
             if (st == 0) { n--; st = steps_per_image - 1; } else st--;
             load_unit(n, st);
@@ -645,7 +645,7 @@ static int launch_quantize_auto(const float* x, float scale, double* sums, unsig
         }
     }
     const unsigned grid = (unsigned)(units < cap ? units : cap);
-    return launch_pdl(quantize_auto_kernel<BITS, V, L, FULL>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out,
+    return launch_pdl_as(true, 1, quantize_auto_kernel<BITS, V, L, FULL>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out,
                       reinterpret_cast<uint64_t*>(qx), wpi, pixels * C, C, PC, make_fastdiv((uint32_t)PC), spi, units, N, status);
 }
 

@@ -19,31 +19,32 @@ inline int check_launch() {
 // still draining (the predecessor executed griddepcontrol.launch_dependents in every CTA); it must execute
 // griddepcontrol.wait before it touches anything a predecessor wrote or may still read.  Works under stream capture
 // (the dependency becomes a programmatic edge of the graph).
+// resident: every CTA of the grid runs at the same time or the launch fails (cooperative launch) - for kernels whose CTAs wait for
+// one another, which other streams' work must not keep from being placed.
+// cluster: CTAs per thread-block cluster along x (grid.x a multiple of it).
 template <typename... KArgs, typename... Args>
-inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+inline int launch_pdl_as(bool resident, unsigned cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
+    cudaLaunchAttribute attr[3];
+    unsigned n = 0;
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    if (resident) {
+        attr[n].id = cudaLaunchAttributeCooperative;
+        attr[n++].val.cooperative = 1;
+    }
+    if (cluster > 1) {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = cluster; attr[n].val.clusterDim.y = 1; attr[n++].val.clusterDim.z = 1;
+    }
+    cfg.attrs = attr; cfg.numAttrs = n;
     cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
     return e == cudaSuccess ? TAB_OK : record_cuda_error(e);
 }
-
-// The same for a kernel that runs as thread-block clusters of `cluster` CTAs along x (grid.x a multiple of it).
 template <typename... KArgs, typename... Args>
-inline int launch_pdl_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, unsigned cluster, Args... args) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = cluster; attr[1].val.clusterDim.y = 1; attr[1].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 2;
-    cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
-    return e == cudaSuccess ? TAB_OK : record_cuda_error(e);
+inline int launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_pdl_as(false, 1, kernel, grid, block, smem, stream, args...);
 }
 
 #ifdef __CUDACC__
@@ -76,8 +77,10 @@ int pack_weights_dispatch(int count, const int8_t* const* w8, uint8_t* const* w4
 // before and after).
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
                            int N, int H, int W, int C, int* status, cudaStream_t stream);
-// Device word that records a bounded wait that ran out (shared with the tensor-core kernel); null if unavailable.
+// Word of the current device that records a bounded wait that ran out (shared with the tensor-core kernel); null if unavailable.
+// It lies in pinned host memory, so that the launches that follow see it without synchronising.
 int* device_status_word();
+inline bool stalled(const int* status) { return status && *static_cast<const volatile int*>(status) != 0; }
 
 // conv_sm100.cu: implicit-im2col popcount GEMM on packed activations.  csa: carry-save popcount tree (else one POPC per word).
 int conv_packed_dispatch(const int64_t* qx, const int64_t* qw, const int32_t* btn, float* y, int type,

@@ -864,3 +864,66 @@ def test_thresholds_of_small_images_with_extreme_residuals(cuda, H, KN, conv_pat
         y, nxt = TAB.ops.conv2d_bits(qx, weights, 0, *geom, residual=dev_t(r, cuda), threshold_scale=0.7, state=TAB.ops.new_state(N, cuda))
         assert np.array_equal(y.cpu().numpy().reshape(N, -1), yo + r)
         assert np.array_equal(np.isinf(nxt.cpu().numpy()), np.isinf(want)) and np.allclose(nxt.cpu().numpy(), want, rtol=2e-7, atol=0)
+
+
+@pytest.mark.parametrize("C", [64, 70])
+def test_meeting_point_whose_wait_runs_out(cuda, conv_path, C):
+    """A counter that can never reach the number of CTAs: the wait ends by itself, the next calls say so until the status is read,
+    and the state block is zero again, so that a caller who keeps it goes on with right results."""
+    if conv_path != "tensor":
+        pytest.skip("no convolution in this test")
+    N, H, W, KN = 2, 4, 4, 64
+    lib = _cabi.lib()
+    assert lib.tab_device_status() == 0
+    m = tab_nn.TABConv2d.from_float(torch.randn(KN, 3, 3, C, device=cuda), 0, 1, 1)
+    x = torch.randn(N, H, W, C, device=cuda)
+    want, qwant = m(x), m.quantize(x)
+    state = m.state(N, cuda)
+    try:
+        state.view(torch.int32)[2 * N + 1] = -1                             # the meeting point, behind the sums and the completion counter: two CTAs take it to 1
+        m.quantize_auto(x)
+        torch.cuda.synchronize()
+        with pytest.raises(_cabi.TabError, match="bounded wait") as stop:
+            m(x)
+        assert stop.value.code == -7
+        with pytest.raises(_cabi.TabError, match="bounded wait"):
+            m.conv_bits(qwant, N, H, W)
+    finally:
+        assert lib.tab_device_status() == 22
+    assert lib.tab_device_status() == 0 and not state.any().item()
+    assert torch.equal(m(x), want) and torch.equal(m.quantize(x), qwant)
+
+
+def test_meeting_points_on_several_streams(cuda, conv_path):
+    """The quantiser that finds its thresholds, whose CTAs wait for one another, on four streams at once and behind work that holds
+    SMs: its launches are placed whole (cooperative ones), captured ones too."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    N, H, W, C = 16, 28, 28, 130
+    layers = [tab_nn.TABConv2d.from_float(torch.randn(128, 3, 3, C, device=cuda), 0, 1, 1) for _ in range(4)]
+    x = torch.randn(N, H, W, C, device=cuda)
+    a = torch.randn(2048, 2048, device=cuda)
+
+    def one(m):
+        qx, ths = m.quantize_auto(x)
+        return m.conv_bits(qx, N, H, W)[0], qx, ths
+
+    want = [one(m) for m in layers]
+    streams = [torch.cuda.Stream() for _ in layers]
+    torch.cuda.synchronize()
+    got = [[] for _ in layers]
+    for _ in range(20):
+        for m, s, g in zip(layers, streams, got):
+            with torch.cuda.stream(s):
+                a @ a
+                g.append(one(m))
+    torch.cuda.synchronize()
+    for w, g in zip(want, got):
+        assert all(torch.equal(u, v) for r in g for u, v in zip(r, w))
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        out = one(layers[0])
+    for _ in range(3):
+        graph.replay()
+    assert all(torch.equal(u, v) for u, v in zip(out, want[0]))
+    assert _cabi.lib().tab_device_status() == 0
