@@ -18,6 +18,15 @@ bool plain(const Tensor& t, at::ScalarType dtype) { return t.defined() && t.is_c
 tab_stream_t stream_of(const Tensor& t) { return reinterpret_cast<tab_stream_t>(at::cuda::getCurrentCUDAStream(t.get_device()).stream()); }
 Tensor make(const Tensor& like, at::IntArrayRef size, at::ScalarType dtype) { return at::empty(size, like.options().dtype(dtype)); }
 
+// n elements are the product of the sizes.  Sizes come from the caller one by one: their product may leave 64 bits, and a wrapped
+// one must not pass for the size of a small tensor.
+bool holds(int64_t n, std::initializer_list<int64_t> sizes) {
+    int64_t product = 1;
+    for (const int64_t s : sizes)
+        if (__builtin_mul_overflow(product, s, &product)) return false;
+    return n == product;
+}
+
 struct Conv {
     int type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW;
     int64_t OH = 0, OW = 0, PC = 0;
@@ -29,8 +38,10 @@ struct Conv {
         PC = ((int64_t)C + 63) / 64;
         return OH > 0 && OW > 0;
     }
-    int64_t weight_words() const { return (int64_t)KN * KH * KW * PC; }
-    int64_t pixels() const { return (int64_t)N * H * W; }
+    // n elements are `per_word` for each packed word of the weights, `per_pixel` for each pixel of the activations, the results.
+    bool weights(int64_t n, int64_t per_word) const { return holds(n, {KN, KH, KW, PC, per_word}); }
+    bool activations(int64_t n, int64_t per_pixel) const { return holds(n, {N, H, W, per_pixel}); }
+    bool results(int64_t n) const { return holds(n, {N, KN, OH, OW}); }
 };
 
 py::object quantize(const Tensor& X, const Tensor& ths, int bitwidth, int N, int H, int W, int C) {
@@ -38,7 +49,7 @@ py::object quantize(const Tensor& X, const Tensor& ths, int bitwidth, int N, int
     {
         py::gil_scoped_release nogil;
         if (plain(X, at::kFloat) && plain(ths, at::kFloat) && N >= 1 && H >= 1 && W >= 1 && C >= 1 && bitwidth >= 1 &&
-            X.numel() == (int64_t)N * H * W * C && ths.numel() == N) {
+            holds(X.numel(), {N, H, W, C}) && ths.numel() == N) {
             const c10::cuda::CUDAGuard guard(X.device());
             QX = make(X, {N, H, W, ((int64_t)C + 63) / 64, bitwidth == 1 ? 1 : 2}, at::kLong);
             BTN = make(X, {N}, at::kInt);
@@ -59,8 +70,8 @@ py::object conv2d(const Tensor& X, const Tensor& QW, const Tensor& ths, const Te
         py::gil_scoped_release nogil;
         Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
         if (g.good() && plain(X, at::kFloat) && plain(QW, at::kLong) && plain(ths, at::kFloat) && plain(btn, at::kInt) &&
-            QW.numel() == g.weight_words() * (type == 1 || type == 3 ? 1 : 2) && (type != 2 || btn.numel() == KN) &&
-            X.numel() == g.pixels() * C && ths.numel() == N) {
+            g.weights(QW.numel(), type == 1 || type == 3 ? 1 : 2) && (type != 2 || btn.numel() == KN) &&
+            g.activations(X.numel(), C) && ths.numel() == N) {
             const c10::cuda::CUDAGuard guard(X.device());
             Y = make(X, {N, KN, g.OH, g.OW}, at::kFloat);
             const size_t bytes = tab_conv2d_workspace_bytes(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW);
@@ -77,7 +88,7 @@ py::object quantize_auto(const Tensor& X, double scale, int bitwidth, int N, int
     Tensor QX, ths;
     {
         py::gil_scoped_release nogil;
-        if (plain(X, at::kFloat) && N >= 1 && H >= 1 && W >= 1 && C >= 1 && bitwidth >= 1 && X.numel() == (int64_t)N * H * W * C &&
+        if (plain(X, at::kFloat) && N >= 1 && H >= 1 && W >= 1 && C >= 1 && bitwidth >= 1 && holds(X.numel(), {N, H, W, C}) &&
             state.defined() && state.is_cuda()) {
             const c10::cuda::CUDAGuard guard(X.device());
             QX = make(X, {N, H, W, ((int64_t)C + 63) / 64, bitwidth == 1 ? 1 : 2}, at::kLong);
@@ -130,8 +141,8 @@ py::object conv2d_packed4(const Tensor& QX, const Tensor& weights, int type, int
         py::gil_scoped_release nogil;
         Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
         const bool want = threshold_scale.has_value();
-        if (g.good() && plain(QX, at::kLong) && (plain(weights, at::kByte) || (plain(weights, at::kChar) && weights.device() == QX.device())) && QX.numel() == g.pixels() * g.PC * (type == 2 || type == 3 ? 1 : 2) &&
-            weights.numel() == g.weight_words() * (weights.scalar_type() == at::kByte ? 32 : 64) && (!residual.has_value() || ((plain(*residual, at::kShort) || (!out_int16 && plain(*residual, at::kFloat))) && residual->numel() == (int64_t)N * KN * g.OH * g.OW)) &&
+        if (g.good() && plain(QX, at::kLong) && (plain(weights, at::kByte) || (plain(weights, at::kChar) && weights.device() == QX.device())) && g.activations(QX.numel(), g.PC * (type == 2 || type == 3 ? 1 : 2)) &&
+            g.weights(weights.numel(), weights.scalar_type() == at::kByte ? 32 : 64) && (!residual.has_value() || ((plain(*residual, at::kShort) || (!out_int16 && plain(*residual, at::kFloat))) && g.results(residual->numel()))) &&
             (!want || (state.has_value() && state->defined() && state->is_cuda())) && (!next_bitwidth.has_value() || want)) {
             const c10::cuda::CUDAGuard guard(QX.device());
             const int nb = next_bitwidth.has_value() ? (*next_bitwidth == 1 ? 1 : 2) : 0;

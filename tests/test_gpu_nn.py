@@ -226,3 +226,17 @@ def test_module_copies_and_moves(cuda):
     for m in (copy.deepcopy(a), pickle.loads(pickle.dumps(old)), b):
         assert torch.equal(m(x), want) and "e2m1" in _cabi.lib().tab_last_conv_kernel().decode()
         assert [n for n, _ in m.named_buffers()] == ["QW", "BTN_W", "W8"]
+
+
+def test_sizes_whose_product_leaves_64_bits_are_refused(cuda):
+    """N*H*W*C = 2**64 + 96, and the bytes of its bit-planes are small modulo 2**64 too: a tensor of 96 elements is not taken for
+    that.  (The checks are made on exact products; the call ends on the host, before anything is launched.)"""
+    from tab_b200 import ops
+    N, H, W, C = 1117667411, 5531, 373004, 8
+    assert N * H * W * C - 2 ** 64 == 96
+    ths = torch.empty(N, device=cuda)
+    QW = torch.zeros(1, 1, 1, 1, 2, dtype=torch.int64, device=cuda)
+    with pytest.raises(RuntimeError, match="X has 96 elements"):
+        ops.Conv2d(torch.zeros(96, device=cuda), QW, ths, torch.zeros(1, dtype=torch.int32, device=cuda), 0, 0, 0, H, W, N, H, W, C, 1, 1, 1)
+    with pytest.raises(RuntimeError, match="X has 96 elements"):
+        ops.Quantize(torch.zeros(96, device=cuda), ths, 2, N, H, W, C)
