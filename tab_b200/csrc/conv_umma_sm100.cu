@@ -484,69 +484,102 @@ __device__ __forceinline__ float i16_float(uint32_t pair, int j) {
     return __uint_as_float(__byte_perm(pair ^ 0x80008000u, 0x4B000000u, j ? 0x7632 : 0x7610)) - 8421376.f;   // 2^23 + 2^15
 }
 
-// A 32x32 block of integers staged row by row (row r: 128 bytes, 16-byte chunks XOR-swizzled by r % 8), written out for filter
-// counts that are no multiple of four and for partial last blocks.  W columns per lane - 2 where rows start on even elements, else 1 - so that an
-// instruction writes W whole rows of the block, 32 * W consecutive elements of which are real: a lane writing its own row
-// instead (32 rows per instruction) took the L1 32 wavefronts for every store.
+// W consecutive elements (4, 2 or 1) as one access.
+template <int W> struct Cells { int v[W]; };
+template <int W>
+__device__ __forceinline__ Cells<W> ld_cells(const float* ptr) {
+    Cells<W> c;
+    if constexpr (W == 4) { const int4 q = __ldg(reinterpret_cast<const int4*>(ptr)); c.v[0] = q.x; c.v[1] = q.y; c.v[2] = q.z; c.v[3] = q.w; }
+    else if constexpr (W == 2) { const int2 q = __ldg(reinterpret_cast<const int2*>(ptr)); c.v[0] = q.x; c.v[1] = q.y; }
+    else c.v[0] = __ldg(reinterpret_cast<const int*>(ptr));
+    return c;
+}
+template <int W>
+__device__ __forceinline__ Cells<W> ld_cells(const int16_t* ptr) {                 // widened to floats
+    Cells<W> c;
+    if constexpr (W == 1) { c.v[0] = __float_as_int((float)__ldg(ptr)); }
+    else {
+        uint32_t q[W / 2];
+        if constexpr (W == 4) { const uint2 u = __ldg(reinterpret_cast<const uint2*>(ptr)); q[0] = u.x; q[1] = u.y; }
+        else q[0] = __ldg(reinterpret_cast<const uint32_t*>(ptr));
+#pragma unroll
+        for (int k = 0; k < W; k++) c.v[k] = __float_as_int(i16_float(q[k >> 1], k & 1));
+    }
+    return c;
+}
+
+// A 32x32 block of integers staged row by row (row r: 128 bytes, 16-byte chunks XOR-swizzled by r % 8), written out where rows do
+// not start on 32-byte boundaries and for partial last blocks.  W columns per lane - 4 where rows start on multiples of four
+// elements, 2 where on even ones, else 1 - so that an instruction writes W whole rows of the block, 32 * W consecutive elements of
+// which are real: a lane writing its own row instead (32 rows per instruction) took the L1 32 wavefronts for every store.
+// Bound by the instructions per element, hence the widest access the rows allow.  B200, us, with W = 4 / 2: 3x3 64x28x28x128->128 with an
+// fp32 residual that starts on 16 bytes and thresholds 26.0 / 34.6, 64x28x28x128->104 to 16 bits 14.1 / 17.5, 64x14x14x256->500 with
+// residual and thresholds 28.7 / 36.5.
 template <int FUSED, int W, bool E2M1>
 __device__ __forceinline__ void ragged_block(const TcConvParams& p, const SlabRows& sr, int nbase, int lane, uint32_t stage, double& dsum0, double& dsum1) {
     constexpr int LPR = 32 / W, BATCH = 4;                                 // lanes per row; rows in flight per lane
     constexpr bool has_res = FUSED >= 2;
+    const bool want_sum = has_res && p.abs_sums != nullptr, out16 = FUSED != 2 && p.y16 != nullptr;
     const int sub = lane / LPR, c = (lane % LPR) * W;
     const bool col_ok = nbase + c < p.KN;
-    // |y| of W values of block row r: floats, or integers in the low halves
-    auto add_sum = [&](int, int r, const int (&q)[W], bool ints) {
-        double a = 0.0;
-#pragma unroll
-        for (int k = 0; k < W; k++) a += ints ? (double)abs((int)(int16_t)(q[k] & 0xFFFF)) : (double)fabsf(__int_as_float(q[k]));
-        if (sr.fast) { if (r < sr.split) dsum0 += a; else dsum1 += a; }
-        else {
-            const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
-            if (img < p.N) atomicAdd(p.abs_sums + img, a);
-        }
-    };
 #pragma unroll 1
     for (int i0 = 0; i0 < LPR; i0 += BATCH) {
         int m[BATCH];
-        float res[BATCH][W];
+        Cells<W> res[BATCH];
 #pragma unroll
         for (int b = 0; b < BATCH; b++) {
             m[b] = __shfl_sync(0xFFFFFFFFu, sr.m_own, (i0 + b) * W + sub);
             if (!col_ok) m[b] = -1;
+            const long long at = (long long)m[b] * p.KN + nbase + c;
 #pragma unroll
-            for (int k = 0; k < W; k++) {
-                const long long at = (long long)m[b] * p.KN + nbase + c + k;
-                res[b][k] = !has_res || m[b] < 0 ? 0.f : (FUSED == 3 ? (float)__ldg(p.residual16 + at) : __ldg(p.residual + at));
+            for (int k = 0; k < W; k++) res[b].v[k] = 0;
+            if (has_res && m[b] >= 0) {
+                if constexpr (FUSED == 3) res[b] = ld_cells<W>(p.residual16 + at);
+                else res[b] = ld_cells<W>(p.residual + at);
             }
         }
 #pragma unroll
         for (int b = 0; b < BATCH; b++) {
             const int r = (i0 + b) * W + sub;
             const uint32_t at = stage + r * 128 + (((c >> 2) ^ (r & 7)) << 4) + (c & 3) * 4;
-            int raw[W];
+            Cells<W> raw;
+            if constexpr (W == 4) { const int4 q = lds_v4(at); raw.v[0] = q.x; raw.v[1] = q.y; raw.v[2] = q.z; raw.v[3] = q.w; }
+            else {
 #pragma unroll
-            for (int k = 0; k < W; k++) raw[k] = lds_b32(at + 4 * k);
+                for (int k = 0; k < W; k++) raw.v[k] = lds_b32(at + 4 * k);
+            }
             if (m[b] < 0) continue;
             const long long e = (long long)m[b] * p.KN + nbase + c;
-            if (FUSED != 2 && p.y16 != nullptr) {
-                if (E2M1)
-#pragma unroll
-                    for (int k = 0; k < W; k++) raw[k] = __float_as_int(__int_as_float(raw[k]) + res[b][k] + 12582912.f);   // low half: the integer
-                if (has_res && p.abs_sums != nullptr) add_sum(b, r, raw, true);
-                if (W == 2) *reinterpret_cast<uint32_t*>(p.y16 + e) = __byte_perm((uint32_t)raw[0], (uint32_t)raw[W - 1], 0x5410);
-                else p.y16[e] = (int16_t)raw[0];
-                continue;
-            }
             float o[W];
 #pragma unroll
-            for (int k = 0; k < W; k++) o[k] = (E2M1 ? __int_as_float(raw[k]) + 0.f : (float)raw[k]) + res[b][k];
-            if (W == 2) *reinterpret_cast<float2*>(p.y + e) = make_float2(o[0], o[W - 1]);
-            else p.y[e] = o[0];
-            if (has_res && p.abs_sums != nullptr) {
-                int bits[W];
+            for (int k = 0; k < W; k++) o[k] = E2M1 ? __int_as_float(raw.v[k]) + 0.f : (float)raw.v[k];
+            if (has_res) {
 #pragma unroll
-                for (int k = 0; k < W; k++) bits[k] = __float_as_int(o[k]);
-                add_sum(b, r, bits, false);
+                for (int k = 0; k < W; k++) o[k] += __int_as_float(res[b].v[k]);
+            }
+            double a = 0.0;                                                // |y| of the lane's W values
+            if (out16) {
+                uint32_t h[W];                                             // float + 1.5 * 2^23: the low 16 bits are the integer
+#pragma unroll
+                for (int k = 0; k < W; k++) h[k] = E2M1 ? __float_as_uint(o[k] + 12582912.f) : (uint32_t)raw.v[k];
+                if constexpr (W == 4) *reinterpret_cast<uint2*>(p.y16 + e) = make_uint2(__byte_perm(h[0], h[1], 0x5410), __byte_perm(h[2], h[3], 0x5410));
+                else if constexpr (W == 2) *reinterpret_cast<uint32_t*>(p.y16 + e) = __byte_perm(h[0], h[1], 0x5410);
+                else p.y16[e] = (int16_t)h[0];
+                if (!want_sum) continue;
+#pragma unroll
+                for (int k = 0; k < W; k++) a += (double)abs((int)(int16_t)(h[k] & 0xFFFFu));
+            } else {
+                if constexpr (W == 4) *reinterpret_cast<float4*>(p.y + e) = make_float4(o[0], o[1], o[2], o[3]);
+                else if constexpr (W == 2) *reinterpret_cast<float2*>(p.y + e) = make_float2(o[0], o[1]);
+                else p.y[e] = o[0];
+                if (!want_sum) continue;
+#pragma unroll
+                for (int k = 0; k < W; k++) a += (double)fabsf(o[k]);
+            }
+            if (sr.fast) { if (r < sr.split) dsum0 += a; else dsum1 += a; }
+            else {
+                const int img = (int)p.dVHW.div((uint32_t)(sr.Rw + r));
+                if (img < p.N) atomicAdd(p.abs_sums + img, a);
             }
         }
     }
@@ -706,6 +739,7 @@ __device__ __forceinline__ void slab_columns(const TcConvParams& p, uint32_t tad
                 sts_v4(stage + lane * 128 + ((q ^ (lane & 7)) << 4), v[4 * q], v[4 * q + 1], v[4 * q + 2], v[4 * q + 3]);
             __syncwarp();
             if (p.KN & 1) ragged_block<FUSED, 1, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
+            else if ((p.KN & 3) == 0) ragged_block<FUSED, 4, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
             else ragged_block<FUSED, 2, E2M1>(p, sr, nbase, lane, stage, dsum0, dsum1);
             __syncwarp();
         }

@@ -927,3 +927,44 @@ def test_meeting_points_on_several_streams(cuda, conv_path):
         graph.replay()
     assert all(torch.equal(u, v) for u, v in zip(out, want[0]))
     assert _cabi.lib().tab_device_status() == 0
+
+
+@pytest.mark.parametrize("KN", [4, 66, 100, 104, 128, 132, 99])
+@pytest.mark.parametrize("N,H", [(40, 3), (3, 15)])                         # several images per 32 rows of the grid, or one
+def test_rows_that_start_between_vectors(cuda, N, H, KN, conv_path):
+    """Rows and residuals on 16-, 8-, 4- and 2-byte boundaries: filter counts that are multiples of four, two and one, a residual
+    that starts 16 bytes into its allocation; fp32 and 16-bit residuals and results, byte and 4-bit operands."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    C, K = 130, 3
+    x, ths = make_input(5, N, H, H, C)
+    w, wths = make_input(6, KN, K, K, C)
+    qw, btn = O.quantize(w, wths, 2, KN, K, K, C)
+    geom = (1, 1, 1, 1, N, H, H, C, KN, K, K)
+    yo = torch.from_numpy(c_oracle.conv2d(x, qw, ths, btn, 0, *geom)).to(cuda)
+    qx = TAB.Quantize(dev_t(x, cuda), dev_t(ths, cuda), 2, N, H, H, C)[0]
+    w8 = TAB.ops.expand_weights(dev_t(qw, cuda), 2, KN, K, K, C)
+    w4 = TAB.ops.pack_weights(w8, KN, K, K, C)
+    state = TAB.ops.new_state(N, cuda)
+
+    def check(weights, r, **kw):
+        y, nxt = TAB.ops.conv2d_bits(qx, weights, 0, *geom, residual=r, threshold_scale=0.7, state=state, **kw)
+        want = yo if r is None else yo + r.float().reshape(yo.shape)
+        assert torch.equal(y.float(), want) and not state.any().item()
+        t = (float(np.float32(0.7)) * want.double().abs().reshape(N, -1).sum(dim=1) / want[0].numel()).float()
+        assert torch.allclose(nxt, t, rtol=1.2e-7, atol=0)                 # both are roundings of sums good to far less than that
+        assert torch.equal(TAB.ops.conv2d_bits(qx, weights, 0, *geom, residual=r, **kw)[0], y)
+
+    for off in (0, 4):
+        r = torch.round(torch.randn(yo.numel() + off, device=cuda) * 9)[off:].reshape(yo.shape)
+        for weights in (w8, w4):
+            check(weights, r)
+            check(weights, r + 0.25 if off == 0 else r)
+        r16 = torch.empty(yo.numel() + 2 * off, dtype=torch.int16, device=cuda)[2 * off:].reshape(yo.shape)
+        r16.copy_(r)
+        check(w4, r16)
+        check(w4, r16, out_int16=True)
+    for weights in (w8, w4):
+        check(weights, None)
+        check(weights, None, out_int16=True)
+    assert _cabi.lib().tab_device_status() == 0
