@@ -167,7 +167,8 @@ static int conv2d_impl(const float* x, const int64_t* qw, const float* ths, cons
     tc_forget_last_kernel();
     if (g_conv_path == TAB_PATH_AUTO && !misaligned(y, 15) && !misaligned(residual, 15)) {
         TcConvParams p = tc_geometry(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, oh, ow);
-        p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = reinterpret_cast<const int8_t*>(w4); p.e2m1 = 1;
+        p.qx = reinterpret_cast<const uint64_t*>(qx); p.w8 = reinterpret_cast<const int8_t*>(w4);
+        p.e2m1 = (long long)KH * KW * C < (1LL << 24);                     // longer sums: bytes, which accumulate in int32
         p.y = y; p.residual = residual; p.abs_sums = abs_sums;
         if (next_ths) { p.ths_out = next_ths; p.ths_scale = next_scale; p.done_counter = counter; }
         if (tc_conv_covers(p)) {
@@ -175,7 +176,8 @@ static int conv2d_impl(const float* x, const int64_t* qw, const float* ths, cons
             QuantExtras ex;
             ex.zero_sums = abs_sums;
             ex.zero_counter = next_ths ? counter : nullptr;
-            ex.qw = reinterpret_cast<const uint64_t*>(qw); ex.w4 = w4;
+            ex.qw = reinterpret_cast<const uint64_t*>(qw);
+            if (p.e2m1) ex.w4 = w4; else ex.w8 = reinterpret_cast<int8_t*>(w4);
             ex.words = (long long)KN * KH * KW * p.PC; ex.wbits = weight_bits(type); ex.PC = p.PC; ex.C = C;
             rc = quantize_dispatch(x, ths, qx, nullptr, act_bits(type), N, H, W, C, s, &ex);
             if (rc != TAB_OK) return rc;

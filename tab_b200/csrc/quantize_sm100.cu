@@ -120,9 +120,17 @@ __device__ __forceinline__ void quant_prologue(const QuantExtras& ex, int n) {
     pdl_wait();
     if (ex.qw != nullptr) {                                                // the weights, spread over all CTAs of the launch
         const long long stride = (long long)gridDim.x * gridDim.y * blockDim.x;
-        for (long long idx = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; idx < ex.words * 2; idx += stride) {
-            if (ex.wbits == 2) expand_half<2>(ex.qw, ex.w4, idx, ex.PC, ex.C);
-            else expand_half<1>(ex.qw, ex.w4, idx, ex.PC, ex.C);
+        const long long first = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
+        if (ex.w4 != nullptr) {
+            for (long long idx = first; idx < ex.words * 2; idx += stride) {
+                if (ex.wbits == 2) expand_half<2>(ex.qw, ex.w4, idx, ex.PC, ex.C);
+                else expand_half<1>(ex.qw, ex.w4, idx, ex.PC, ex.C);
+            }
+        } else {
+            for (long long idx = first; idx < ex.words * 4; idx += stride) {
+                if (ex.wbits == 2) expand_group<2>(ex.qw, ex.w8, idx, ex.PC, ex.C);
+                else expand_group<1>(ex.qw, ex.w8, idx, ex.PC, ex.C);
+            }
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {

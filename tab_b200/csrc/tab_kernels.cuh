@@ -63,6 +63,7 @@ struct QuantExtras {
     unsigned* zero_counter = nullptr;    // cleared
     const uint64_t* qw = nullptr;        // packed weights [KN][KH*KW*PC][wbits] to expand into w4 [KN][KH*KW*PC][32] (4-bit operands)
     uint8_t* w4 = nullptr;
+    int8_t* w8 = nullptr;                // or into bytes [KN][KH*KW*PC][64]
     long long words = 0;                 // KN*KH*KW*PC
     int wbits = 2, PC = 1, C = 64;       // of the weights
 };

@@ -968,3 +968,50 @@ def test_rows_that_start_between_vectors(cuda, N, H, KN, conv_path):
         check(weights, None)
         check(weights, None, out_int16=True)
     assert _cabi.lib().tab_device_status() == 0
+
+
+def _long_sums(cuda, C, KN, t):
+    """A 1x1 layer of C channels whose operands are all +1 but for a few: filter f has -1 in its first f channels and, if t is
+    ternary and f odd, 0 in channel 2000; pixel 0 is all +1, pixel 1 has -1 in the first 1000 channels, pixel 2 in the first half.
+    Returns the result and what it has to be, as whole numbers."""
+    PC, wb = C // 64, O.weight_bits(t)
+    sign = np.zeros((KN, 32 * 64), bool)
+    mag = np.ones((KN, 32 * 64), bool)
+    for f in range(KN):
+        sign[f, :f] = True
+        mag[f, 2000] = wb == 1 or f % 2 == 0
+    pack = lambda b: torch.from_numpy(np.packbits(b.reshape(KN, 32, 64), axis=2, bitorder="little").view(np.int64)[..., 0].copy()).to(cuda)
+    QW = torch.zeros(KN, 1, 1, PC, wb, dtype=torch.int64, device=cuda)
+    if wb == 2:
+        QW[..., 1] = -1
+        QW[:, 0, 0, :32, 1] = pack(mag)
+    QW[:, 0, 0, :32, 0] = pack(sign & mag)
+    x = torch.ones(1, 1, 3, C, device=cuda)
+    x[0, 0, 1, :1000] = -1.0
+    x[0, 0, 2, : C // 2] = -1.0
+    y = TAB.Conv2d(x, QW, torch.full((1,), 0.0 if t >= 2 else 0.5, device=cuda), torch.zeros(KN, dtype=torch.int32, device=cuda), t, 0, 0, 1, 1, 1, 1, 3, C, KN, 1, 1)
+    f = np.arange(KN, dtype=np.int64)
+    zero = np.where(mag[:, 2000], 0, 1)
+    want = np.stack([C - zero - 2 * f, C - zero - 2000 - 2 * f + 4 * np.minimum(f, 1000), C - 2 * (C // 2) + zero + 2 * f])
+    return y.reshape(3, KN).cpu().numpy(), want
+
+
+@pytest.mark.parametrize("KN", [17, 64, 128, 256])
+def test_sums_just_below_two_to_the_24(cuda, KN, conv_path):
+    """4-bit operands accumulate in fp32: exact up to the limit of the dispatch, on tiles of every width."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel")
+    y, want = _long_sums(cuda, (1 << 24) - 64, KN, 0)
+    assert "e2m1" in _cabi.lib().tab_last_conv_kernel().decode() and np.abs(want).max() > (1 << 24) - 128
+    assert np.array_equal(y.astype(np.int64), want) and _cabi.lib().tab_device_status() == 0
+
+
+@pytest.mark.parametrize("t", [0, 1])
+def test_sums_from_two_to_the_24(cuda, t, conv_path):
+    """Longer sums are multiplied as bytes on the tensor cores (int32 accumulators, rounded once to fp32)."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel")
+    y, want = _long_sums(cuda, (1 << 24) + 64, 5, t)
+    name = _cabi.lib().tab_last_conv_kernel().decode()
+    assert name.startswith("conv_umma") and "e2m1" not in name
+    assert np.array_equal(y, want.astype(np.float32)) and _cabi.lib().tab_device_status() == 0
