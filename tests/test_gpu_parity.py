@@ -1015,3 +1015,41 @@ def test_sums_from_two_to_the_24(cuda, t, conv_path):
     name = _cabi.lib().tab_last_conv_kernel().decode()
     assert name.startswith("conv_umma") and "e2m1" not in name
     assert np.array_equal(y, want.astype(np.float32)) and _cabi.lib().tab_device_status() == 0
+
+
+@pytest.mark.parametrize("geom", [
+    # p1 p2 s1 s2  N  H  W   C   KN KH KW       streamed filters, a last round that fills less than half of the SMs
+    (1, 1, 1, 1, 90, 14, 14, 256, 256, 3, 3),
+    (1, 1, 1, 1, 90, 14, 14, 256, 250, 3, 3),
+    (1, 1, 1, 1, 90, 14, 14, 256, 192, 3, 3),
+    (0, 0, 1, 1, 52, 14, 14, 512, 384, 1, 1),
+])
+def test_half_tiles_on_four_bit_operands(cuda, geom, conv_path):
+    """Tiles worked as halves (overlapping accumulators for 256 filters): the reported kernel says so, plain and with an fp32 and a
+    16-bit residual; results against the byte form, whose halves have a test of their own, and the oracle."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel's own entry point")
+    p1, p2, s1, s2, N, H, W, C, KN, KH, KW = geom
+    x, ths = make_input(95, N, H, W, C)
+    w, wths = make_input(96, KN, KH, KW, C)
+    qw, btn = O.quantize(w, wths, 2, KN, KH, KW, C)
+    qx = TAB.Quantize(dev_t(x, cuda), dev_t(ths, cuda), 2, N, H, W, C)[0]
+    w8 = TAB.ops.expand_weights(dev_t(qw, cuda), 2, KN, KH, KW, C)
+    w4 = TAB.ops.pack_weights(w8, KN, KH, KW, C)
+    y, _ = TAB.ops.conv2d_bits(qx, w8, 0, *geom)
+    n = N - 1
+    yo = c_oracle.conv2d(x[n:], qw, ths[n:], btn, 0, p1, p2, s1, s2, 1, H, W, C, KN, KH, KW)
+    assert np.array_equal(y.reshape(N, -1)[n].cpu().numpy(), yo.reshape(-1))
+    r = torch.round(torch.randn(*y.shape, device=cuda) * 5)
+    state = TAB.ops.new_state(N, cuda)
+    for residual in (None, r, r.to(torch.int16)):
+        for scale in (None, 0.7):
+            got = TAB.ops.conv2d_bits(qx, w4, 0, *geom, residual=residual, threshold_scale=scale, state=state)
+            name = _cabi.lib().tab_last_conv_kernel().decode()
+            assert "<1,256,4,0," in name and ",e2m1>" in name and " halves" in name, name
+            want = y if residual is None else y + r
+            assert torch.equal(got[0], want)
+            if scale:
+                t = (float(np.float32(0.7)) * (want.double().abs().reshape(N, -1).sum(dim=1) / want[0].numel())).float()
+                assert torch.equal(got[1], t)                              # whole numbers: exact sums, rounded once
+    assert _cabi.lib().tab_device_status() == 0
