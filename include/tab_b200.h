@@ -217,6 +217,15 @@ int tab_conv2d_packed4_launch(const int64_t* qx, const uint8_t* w4, void* y, int
 int tab_quantize_auto_launch(const float* x, float scale, void* state, float* ths, int64_t* qx, int bitwidth,
                              int N, int H, int W, int C, tab_stream_t stream);
 /*
+ * What precedes the GEMM stage of a layer that is kept as byte weights: tab_pack_weights_launch of the layer's
+ * `words` = KN*KH*KW*ceil(C/64) words and tab_quantize_launch's bit-planes (ths given), or, in one launch with the packing,
+ * tab_quantize_auto_launch's and the thresholds it finds (ths NULL: state, ths_out).  tab_conv2d_packed4_covers: whether
+ * tab_conv2d_packed4_launch covers a geometry (plain result), to ask before.
+ */
+int tab_quantize_pack_launch(const float* x, const float* ths, float scale, void* state, float* ths_out, int64_t* qx, int bitwidth,
+                             int N, int H, int W, int C, const int8_t* w8, uint8_t* w4, long long words, tab_stream_t stream);
+int tab_conv2d_packed4_covers(int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW);
+/*
  * A chained layer that also hands the next convolution its input: after the GEMM stage (tab_conv2d_bits_launch, or the int16
  * form when y_is_int16) the same launch computes the next thresholds and quantises the result against them into next_qx,
  * [N][OH][OW][ceil(KN/64)][next_bitwidth] 64-bit words - exactly what tab_quantize_launch(y, next_ths, next_qx, ...) writes

@@ -35,6 +35,8 @@ SYMBOLS = {
     "tab_pack_weights_many_launch": (_c.c_int, [_c.c_int] + [_c.c_void_p] * 4),
     "tab_conv2d_packed4_launch": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_int] * 13 + [_c.c_void_p, _c.c_int] + [_c.c_void_p] * 2 + [_c.c_float, _c.c_void_p, _c.c_int, _c.c_void_p]),
     "tab_quantize_auto_launch": (_c.c_int, [_c.c_void_p, _c.c_float, _c.c_void_p, _c.c_void_p, _c.c_void_p] + [_c.c_int] * 5 + [_c.c_void_p]),
+    "tab_quantize_pack_launch": (_c.c_int, [_c.c_void_p] * 2 + [_c.c_float] + [_c.c_void_p] * 3 + [_c.c_int] * 5 + [_c.c_void_p] * 2 + [_c.c_longlong, _c.c_void_p]),
+    "tab_conv2d_packed4_covers": (_c.c_int, [_c.c_int] * 12),
     "tab_quantize_i16_launch": (_c.c_int, [_c.c_void_p] * 3 + [_c.c_int] * 5 + [_c.c_void_p]),
     "tab_last_conv_kernel": (_c.c_char_p, []),
     "tab_device_status": (_c.c_int, []),

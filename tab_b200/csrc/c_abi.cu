@@ -176,8 +176,9 @@ static int conv2d_impl(const float* x, const int64_t* qw, const float* ths, cons
             QuantExtras ex;
             ex.zero_sums = abs_sums;
             ex.zero_counter = next_ths ? counter : nullptr;
-            ex.qw = reinterpret_cast<const uint64_t*>(qw);
-            if (p.e2m1) ex.w4 = w4; else ex.w8 = reinterpret_cast<int8_t*>(w4);
+            if (p.e2m1) { ex.qw = reinterpret_cast<const uint64_t*>(qw); ex.w4 = w4; }
+            else rc = expand_weights_dispatch(qw, reinterpret_cast<int8_t*>(w4), weight_bits(type), KN, KH, KW, C, s);
+            if (rc != TAB_OK) return rc;
             ex.words = (long long)KN * KH * KW * p.PC; ex.wbits = weight_bits(type); ex.PC = p.PC; ex.C = C;
             rc = quantize_dispatch(x, ths, qx, nullptr, act_bits(type), N, H, W, C, s, &ex);
             if (rc != TAB_OK) return rc;
@@ -353,6 +354,34 @@ int tab_quantize_auto_launch(const float* x, float scale, void* state, float* th
     int* status = device_status_word();
     if (stalled(status)) return TAB_E_STALLED;
     return quantize_auto_dispatch(x, scale, sums, bar, ths, qx, bitwidth == 1 ? 1 : 2, N, H, W, C, status, s);
+}
+
+int tab_conv2d_packed4_covers(int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW) {
+    if (conv_args_ok(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW) != TAB_OK) return 0;
+    const long long oh = ((long long)H + 2LL * p1 - KH + 1) / s1, ow = ((long long)W + 2LL * p2 - KW + 1) / s2;
+    if (N == 0 || KN == 0 || oh <= 0 || ow <= 0) return 0;
+    TcConvParams p = tc_geometry(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW, oh, ow);
+    p.e2m1 = 1;
+    return tc_conv_covers(p) ? 1 : 0;
+}
+
+int tab_quantize_pack_launch(const float* x, const float* ths, float scale, void* state, float* ths_out, int64_t* qx, int bitwidth,
+                             int N, int H, int W, int C, const int8_t* w8, uint8_t* w4, long long words, tab_stream_t stream) {
+    if (N < 1 || H < 1 || W < 1 || C < 1 || bitwidth < 1 || words < 1) return TAB_E_BAD_ARGUMENT;
+    if (!x || !qx || !w8 || !w4 || (!ths && (!state || !ths_out))) return TAB_E_NULL_POINTER;
+    if (misaligned(x, 3) || misaligned(ths, 3) || misaligned(ths_out, 3) || misaligned(qx, 7) || misaligned(state, 7) || misaligned(w8, 15) || misaligned(w4, 15))
+        return TAB_E_ALIGNMENT;
+    if ((long long)H * W >= (1LL << 31)) return TAB_E_TOO_LARGE;
+    cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+    const int bits = bitwidth == 1 ? 1 : 2;
+    if (ths) {                                                     // the streaming quantiser is left as it is: two launches
+        const int rc = pack_weights_dispatch(1, &w8, &w4, &words, s);
+        return rc != TAB_OK ? rc : quantize_dispatch(x, ths, qx, nullptr, bits, N, H, W, C, s);
+    }
+    int* status = device_status_word();
+    if (stalled(status)) return TAB_E_STALLED;
+    double* sums = reinterpret_cast<double*>(state);
+    return quantize_auto_dispatch(x, scale, sums, reinterpret_cast<unsigned*>(sums + N) + 1, ths_out, qx, bits, N, H, W, C, status, s, PackJob{w8, w4, words});
 }
 
 int tab_quantize_i16_launch(const int16_t* x, const float* ths, int64_t* qx, int bitwidth, int N, int H, int W, int C, tab_stream_t stream) {

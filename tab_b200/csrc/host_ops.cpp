@@ -168,12 +168,42 @@ py::object conv2d_packed4(const Tensor& QX, const Tensor& weights, int type, int
     return py::make_tuple(Y, th);
 }
 
+// Both launches of a layer kept as byte weights: quantiser (against the thresholds given, or against those it finds) with the
+// weights packed on the side, then the GEMM stage.
+py::object layer(const Tensor& X, const Tensor& W8, int type, int p1, int p2, int s1, int s2, int N, int H, int W, int C, int KN, int KH, int KW,
+                 const OptTensor& thresholds, double scale, const OptTensor& state) {
+    Tensor Y;
+    {
+        py::gil_scoped_release nogil;
+        Conv g{type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW};
+        if (g.good() && plain(X, at::kFloat) && plain(W8, at::kChar) && W8.device() == X.device() && g.activations(X.numel(), C) && g.weights(W8.numel(), 64) &&
+            (thresholds.has_value() ? plain(*thresholds, at::kFloat) && thresholds->numel() == N : state.has_value() && state->defined() && state->is_cuda())) {
+            const c10::cuda::CUDAGuard guard(X.device());
+            if (tab_conv2d_packed4_covers(type, p1, p2, s1, s2, N, H, W, C, KN, KH, KW)) {
+                const int bits = type == 2 || type == 3 ? 1 : 2;
+                const bool find = !thresholds.has_value();
+                Tensor QX = make(X, {N, H, W, g.PC, bits}, at::kLong), W4 = make(X, {W8.numel() / 2}, at::kByte), found;
+                if (find) found = make(X, {N}, at::kFloat);
+                Y = make(X, {N, KN, g.OH, g.OW}, at::kFloat);
+                int rc = tab_quantize_pack_launch(X.data_ptr<float>(), find ? nullptr : thresholds->data_ptr<float>(), (float)scale, find ? state->data_ptr() : nullptr,
+                                                  find ? found.data_ptr<float>() : nullptr, QX.data_ptr<int64_t>(), bits, N, H, W, C, W8.data_ptr<int8_t>(),
+                                                  W4.data_ptr<uint8_t>(), W8.numel() / 64, stream_of(X));
+                if (rc == TAB_OK) rc = tab_conv2d_packed4_launch(QX.data_ptr<int64_t>(), W4.data_ptr<uint8_t>(), Y.data_ptr(), 0, type, p1, p2, s1, s2, N, H, W, C,
+                                                                 KN, KH, KW, nullptr, 0, nullptr, nullptr, 0.f, nullptr, 0, stream_of(X));
+                if (rc != TAB_OK) Y.reset();
+            }
+        }
+    }
+    return Y.defined() ? py::cast(Y) : py::none();
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("quantize", &quantize);
     m.def("conv2d", &conv2d);
     m.def("quantize_auto", &quantize_auto);
+    m.def("layer", &layer);
     m.def("pack_weights", &pack_weights);
     m.def("conv2d_packed4", &conv2d_packed4);
 }

@@ -16,6 +16,7 @@
 // Inside a convolution call the same launch also does the call's small set-up jobs (QuantExtras), so that they cost no
 // launch of their own: all CTAs share the expansion of the packed weights to the bytes the tensor-core kernel
 // multiplies, and the first CTA of every image clears that image's |y| sum (the first of all the completion counter).
+#include <algorithm>
 #include <mutex>
 #include "tab_kernels.cuh"
 #include "umma_common.cuh"
@@ -70,6 +71,23 @@ __device__ __forceinline__ void expand_half(const uint64_t* __restrict__ qw, uin
     *reinterpret_cast<uint4*>(w4 + word * 32 + h * 16) = nibbles32(m, s & m);
 }
 
+// One thread per 32 channels of byte weights: 32 bytes -> 16 bytes of e2m1 nibbles.
+__device__ __forceinline__ void pack_half(const int8_t* __restrict__ w8, uint8_t* __restrict__ w4, long long idx) {
+    uint32_t m = 0, s = 0;
+#pragma unroll
+    for (int k = 0; k < 2; k++) {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(w8 + idx * 32) + k);
+        const uint32_t q[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 16; i++) {
+            const uint32_t b = (q[i >> 2] >> (8 * (i & 3))) & 0xFFu;
+            m |= (b & 1u) << (16 * k + i);
+            s |= (b >> 7) << (16 * k + i);
+        }
+    }
+    *reinterpret_cast<uint4*>(w4 + idx * 16) = nibbles32(m, s & m);
+}
+
 // Byte weights -> 4-bit operands, several layers in one launch: a CTA takes 256 halves (32 channels: 32 bytes in, 16 out) of the
 // layer whose range of CTAs it lies in.  Bound by the launch: a prepared layer's bytes are the registered weights and are
 // packed again by every pass, so that whoever writes them is followed; a network does that once per pass for all its layers.
@@ -84,26 +102,12 @@ struct PackList {
     int count;
 };
 __global__ void __launch_bounds__(256) pack_weights_kernel(const __grid_constant__ PackList list) {
+    pdl_launch_dependents();                                               // the convolution sets itself up meanwhile; this grid leaves it room
     pdl_wait();                                                            // the bytes may be the previous launch's, the nibbles its operands
     int l = 0;
     while (l + 1 < list.count && blockIdx.x >= list.first[l + 1]) l++;
     const long long idx = (long long)(blockIdx.x - list.first[l]) * 256 + threadIdx.x;
-    if (idx < list.halves[l]) {
-        uint32_t m = 0, s = 0;
-#pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const uint4 v = __ldg(reinterpret_cast<const uint4*>(list.w8[l] + idx * 32) + k);
-            const uint32_t q[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-            for (int i = 0; i < 16; i++) {
-                const uint32_t b = (q[i >> 2] >> (8 * (i & 3))) & 0xFFu;
-                m |= (b & 1u) << (16 * k + i);
-                s |= (b >> 7) << (16 * k + i);
-            }
-        }
-        *reinterpret_cast<uint4*>(list.w4[l] + idx * 16) = nibbles32(m, s & m);
-    }
-    pdl_launch_dependents();
+    if (idx < list.halves[l]) pack_half(list.w8[l], list.w4[l], idx);
 }
 
 template <int WB>
@@ -120,17 +124,9 @@ __device__ __forceinline__ void quant_prologue(const QuantExtras& ex, int n) {
     pdl_wait();
     if (ex.qw != nullptr) {                                                // the weights, spread over all CTAs of the launch
         const long long stride = (long long)gridDim.x * gridDim.y * blockDim.x;
-        const long long first = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x;
-        if (ex.w4 != nullptr) {
-            for (long long idx = first; idx < ex.words * 2; idx += stride) {
-                if (ex.wbits == 2) expand_half<2>(ex.qw, ex.w4, idx, ex.PC, ex.C);
-                else expand_half<1>(ex.qw, ex.w4, idx, ex.PC, ex.C);
-            }
-        } else {
-            for (long long idx = first; idx < ex.words * 4; idx += stride) {
-                if (ex.wbits == 2) expand_group<2>(ex.qw, ex.w8, idx, ex.PC, ex.C);
-                else expand_group<1>(ex.qw, ex.w8, idx, ex.PC, ex.C);
-            }
+        for (long long idx = ((long long)blockIdx.y * gridDim.x + blockIdx.x) * blockDim.x + threadIdx.x; idx < ex.words * 2; idx += stride) {
+            if (ex.wbits == 2) expand_half<2>(ex.qw, ex.w4, idx, ex.PC, ex.C);
+            else expand_half<1>(ex.qw, ex.w4, idx, ex.PC, ex.C);
         }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -437,12 +433,15 @@ static unsigned ctas_per_image(long long words_per_image, long long words_per_st
     return (unsigned)(per_image < 1 ? 1 : per_image);
 }
 
-// A launch that also expands weights gets enough CTAs for that, 32 channels per thread up to four CTAs per SM: the tensor of a
+// A launch that also prepares weights gets enough CTAs for that, 32 channels per thread up to four CTAs per SM: the tensor of a
 // single image fills 4 CTAs, which took 65 us for the weights of a 3x3x512 -> 512 layer.
+static long long ctas_for_weights(long long words) {
+    const long long groups = (words * 2 + QTHREADS - 1) / QTHREADS;
+    return groups < 148 * 4 ? groups : 148 * 4;
+}
 static dim3 quantize_grid(unsigned per_image, int N, const QuantExtras& ex) {
     if (ex.qw) {
-        const long long groups = (ex.words * 2 + QTHREADS - 1) / QTHREADS, want = groups < 148 * 4 ? groups : 148 * 4;
-        const unsigned share = (unsigned)((want + N - 1) / N);
+        const unsigned share = (unsigned)((ctas_for_weights(ex.words) + N - 1) / N);
         if (per_image < share) per_image = share;
     }
     return dim3(per_image, (unsigned)N);
@@ -516,6 +515,7 @@ int quantize_dispatch(const void* x, const float* ths, int64_t* qx, int32_t* btn
 // bounded and reports in *status), then every CTA quantises, last unit first, the units it has just summed - the end of its share is
 // what the L2 still holds, and its last unit is still in registers.  A unit is one CTA step (QUNROLL passes) of one image; a
 // CTA owns consecutive units, so that its sum leaves the registers once per image and not once per unit.
+// The weights of the layer that reads the planes may be packed on the side (see PackJob).
 // FULL: C % 64 == 0 and 32-byte rows (every lane has eight real channels); else V and L as in quantize_any_kernel.
 constexpr uint32_t QA_WAIT_LIMIT = 1u << 21;                               // a second or two; the slowest CTA of 180 GB of input needs 30 ms
 
@@ -523,8 +523,9 @@ template <int BITS, int V, int L, bool FULL>
 __global__ void __launch_bounds__(QTHREADS, 4)
 quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restrict__ sums, unsigned* __restrict__ bar,
                      float* __restrict__ ths_out, uint64_t* __restrict__ qx, long long words_per_image, long long elems_per_image, int C, int PC,
-                     const FastDiv dPC, long long steps_per_image, long long units, int N, int* __restrict__ status) {
+                     const FastDiv dPC, long long steps_per_image, long long units, int N, int* __restrict__ status, const PackJob pack) {
     pdl_wait();
+    for (long long idx = (long long)blockIdx.x * QTHREADS + threadIdx.x; idx < pack.words * 2; idx += (long long)gridDim.x * QTHREADS) pack_half(pack.w8, pack.w4, idx);
     constexpr int PASS = words_per_pass<L>(), STEP = PASS * QUNROLL;
     const int slot = threadIdx.x / L;
     const bool wide = words_per_image >= (1LL << 31);
@@ -547,7 +548,7 @@ quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restric
         }
     };
     // phase 1: sums
-    const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1LL) / gridDim.x;     // grid <= units: never empty
+    const long long ub = units * blockIdx.x / gridDim.x, ue = units * (blockIdx.x + 1LL) / gridDim.x;     // empty where the grid is larger, for weights to prepare
     long long n = ub / steps_per_image, st = ub - n * steps_per_image;
     double acc = 0.0;
     for (long long u = ub; u < ue; u++) {
@@ -630,7 +631,7 @@ quantize_auto_kernel(const float* __restrict__ x, float scale, double* __restric
 
 template <int BITS, int V, int L, bool FULL>
 static int launch_quantize_auto(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx,
-                                int N, int H, int W, int C, int* status, cudaStream_t stream) {
+                                int N, int H, int W, int C, int* status, cudaStream_t stream, const PackJob& pack) {
     const int PC = (C + 63) / 64;
     const long long pixels = (long long)H * W, wpi = pixels * PC, step = (long long)words_per_pass<L>() * QUNROLL;
     const long long spi = (wpi + step - 1) / step, units = spi * N;
@@ -652,16 +653,17 @@ static int launch_quantize_auto(const float* x, float scale, double* sums, unsig
             if (dev < 64) capacity[dev] = cap;
         }
     }
-    const unsigned grid = (unsigned)(units < cap ? units : cap);
+    const long long want = std::max(units, ctas_for_weights(pack.words));
+    const unsigned grid = (unsigned)(want < cap ? want : cap);
     return launch_pdl_as(true, 1, quantize_auto_kernel<BITS, V, L, FULL>, dim3(grid), dim3(QTHREADS), 0, stream, x, scale, sums, bar, ths_out,
-                      reinterpret_cast<uint64_t*>(qx), wpi, pixels * C, C, PC, make_fastdiv((uint32_t)PC), spi, units, N, status);
+                      reinterpret_cast<uint64_t*>(qx), wpi, pixels * C, C, PC, make_fastdiv((uint32_t)PC), spi, units, N, status, pack);
 }
 
 template <int BITS>
 static int quantize_auto_by_width(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx,
-                                  int N, int H, int W, int C, int* status, cudaStream_t s) {
+                                  int N, int H, int W, int C, int* status, cudaStream_t s, const PackJob& pack) {
     const int V = load_width(x, C, false);
-#define TAB_QAUTO(VV, LL, FF) return launch_quantize_auto<BITS, VV, LL, FF>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, s)
+#define TAB_QAUTO(VV, LL, FF) return launch_quantize_auto<BITS, VV, LL, FF>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, s, pack)
     if (C <= 8) {
         if (V == 8) TAB_QAUTO(8, 1, false);
         if (V == 4) TAB_QAUTO(4, 1, false);
@@ -677,9 +679,9 @@ static int quantize_auto_by_width(const float* x, float scale, double* sums, uns
 }
 
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
-                           int N, int H, int W, int C, int* status, cudaStream_t stream) {
-    return bits == 2 ? quantize_auto_by_width<2>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream)
-                     : quantize_auto_by_width<1>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream);
+                           int N, int H, int W, int C, int* status, cudaStream_t stream, const PackJob& pack) {
+    return bits == 2 ? quantize_auto_by_width<2>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream, pack)
+                     : quantize_auto_by_width<1>(x, scale, sums, bar, ths_out, qx, N, H, W, C, status, stream, pack);
 }
 
 int pack_weights_dispatch(int count, const int8_t* const* w8, uint8_t* const* w4, const long long* words, cudaStream_t stream) {

