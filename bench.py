@@ -262,7 +262,8 @@ def step_algorithmic_bytes(n_images):
     producer handed it over as int16) and 2 bits/element written by the quantiser; per convolution those bit-planes read, the
     4-bit weights read, the output written (4 B/element; 2 B for a block's first convolution, whose only reader is the next
     quantiser) and, where a shortcut is added, 4 B/element of residual read; the input statistics pass reads x once.  From the
-    first strided shortcut on large block results and shortcuts are 2 B/element too."""
+    first strided shortcut on large block results and shortcuts are 2 B/element too.  The registered byte weights are read and
+    packed to 4 bits once per step."""
     from tab_b200 import chain
     total = 4 * n_images * H0 * W0 * C0
     h = H0
@@ -282,6 +283,7 @@ def step_algorithmic_bytes(n_images):
         total += 2 * y_el + bits_mid                                       # quantise y1 (int16)
         total += bits_mid + bb.KN * 9 * bb.C // 2 + (short_bytes + out_bytes) * y_el         # conv_b + residual
         h, x_bytes = oh, out_bytes
+    total += 3 * sum(cs.KN * cs.K * cs.K * cs.C for cs in chain.conv_specs()) // 2
     return total
 
 
@@ -344,13 +346,14 @@ def main():
     launches = [0]
 
     class CountingConv(tab_nn.TABConv2d):
-        """tab_b200.nn.TABConv2d with a kernel-launch counter (quantize = one kernel, conv_bits = one kernel)."""
+        """tab_b200.nn.TABConv2d with a kernel-launch counter (quantize = one kernel, conv_bits = one kernel, and one more where it
+        packs its weights itself)."""
         def quantize(self, x, thresholds=None):
             launches[0] += 1
             return super().quantize(x, thresholds)
 
         def conv_bits(self, *a, **k):
-            launches[0] += 1
+            launches[0] += 1 if k.get("packed") is not None else 2
             out = super().conv_bits(*a, **k)
             # the quantised hand-over to the next layer comes from the same kernel ("+next") or from a quantiser launch behind it
             if k.get("next_bitwidth") is not None and "+next" not in lib.tab_last_conv_kernel().decode():
@@ -407,9 +410,9 @@ def main():
 
     def forward(cset, x_in, nb, count=True):
         if cset is convs:
-            # thresholds of the chain's input and its bit-planes from one launch
+            # thresholds of the chain's input and its bit-planes from one launch, all layers' weights packed by another
             if count:
-                launches[0] += 1
+                launches[0] += 2
             qx0, ths = convs[first_conv].quantize_auto(x_in)
             y, _, _, _ = chain.forward_prepared(cset, x_in, ths, nb, compact_mid=True, fused_quant=True, qx0=qx0)
             return y, ths
@@ -760,7 +763,7 @@ def main():
     popc_achieved = sums["ops"] / (sums["popc_ms"] * 1e-3) / 1e12 if sums["popc_ms"] else None
     l1_images = n_local
     roofline = {
-        "kernel": "whole step: %d launches (conv_umma_persist_kernel x19, quantize_auto_kernel x1 for the chain's input and its thresholds, quantize_c64_kernel x%d - the other convolutions' inputs are quantised by the kernel that wrote them)" % (launches_per_step, launches_per_step - 20),
+        "kernel": "whole step: %d launches (conv_umma_persist_kernel x19, quantize_auto_kernel x1 for the chain's input and its thresholds, pack_weights_kernel x1 for all layers' weights, quantize_c64_kernel x%d - the other convolutions' inputs are quantised by the kernel that wrote them)" % (launches_per_step, launches_per_step - 21),
         "bound": "hbm", "achieved": step_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": step_gbs / hbm_peak, "peak_source": hbm_src,
         "algorithmic_bytes_per_step": step_bytes, "images_per_gpu": n_local,
         "traffic": (L1_TRAFFIC_PER_IMAGE * l1_images) if L1_TRAFFIC_PER_IMAGE else None,
@@ -809,7 +812,7 @@ def main():
     line = {
         "metric": "TAB_Conv2d binary-op TOPS", "value": value, "unit": "TOPS", "n_gpus": world, "steps": args.steps,
         "warmup": max(args.warmup, 3), "ms_per_step": ms_step, "higher_is_better": True, "scaling": "strong",
-        "vs_baseline": None, "dtype": "s8 (ternary values on the integer tensor cores, s32 accumulate; exact)", "data": "synthetic",
+        "vs_baseline": None, "dtype": "e2m1 (ternary values as 4-bit floats on the tensor cores, fp32 accumulate; exact); e2e: s8, s32 accumulate; exact", "data": "synthetic",
         "config": config,
         "e2e": {"value": e2e_value, "unit": "TOPS", "ms_per_step": ms_e2e / args.steps,
                 "h2d_bytes_per_step": int(x_host.numel() * 4), "d2h_bytes_per_step": int(N * per_img_out * 4),

@@ -19,10 +19,18 @@ Results are those of ``Conv2d`` bit for bit.  Inference only: there is no backwa
 from __future__ import annotations
 
 import functools
+import inspect
 
 import torch
 
 from . import _cabi, ops
+
+@functools.lru_cache(maxsize=64)
+def _takes_packed(conv_bits):
+    """Whether a class's ``conv_bits`` - its own or one that passes keywords on - can be handed packed weights."""
+    parameters = inspect.signature(conv_bits).parameters
+    return "packed" in parameters or any(p.kind is p.VAR_KEYWORD for p in parameters.values())
+
 
 _state_bytes = functools.lru_cache(maxsize=256)(lambda N: _cabi.lib().tab_conv2d_state_bytes(N))
 
@@ -78,7 +86,7 @@ class TABConv2d(torch.nn.Module):
         """For a pass through several layers, name -> layer: name -> keywords for its ``conv_bits``, which then need not pack
         the weights by itself.  One launch for all of them instead of one per layer; the packed forms are of ``W8`` as it is
         now and serve this pass only."""
-        own = [(k, c._buffers["W8"]) for k, c in convs.items() if isinstance(c, TABConv2d) and type(c).conv_bits is TABConv2d.conv_bits and c._four_bit()]
+        own = [(k, c._buffers["W8"]) for k, c in convs.items() if isinstance(c, TABConv2d) and _takes_packed(type(c).conv_bits) and c._four_bit()]
         packed = ops.pack_weights_many([w for _, w in own])
         return {} if packed is None else {k: {"packed": p} for (k, _), p in zip(own, packed)}
 

@@ -285,3 +285,22 @@ def test_layer_with_stages_of_its_own(cuda):
             m(bad, torch.ones(2, device=cuda))
     with pytest.raises(RuntimeError, match="thresholds has"):
         m(x, torch.ones(3, device=cuda))
+
+
+def test_pack_together_asks_whether_a_layer_takes_it(cuda):
+    """Subclasses whose ``conv_bits`` passes keywords on get the packed weights, ones with a signature of their own do not."""
+    class Passing(tab_nn.TABConv2d):
+        def conv_bits(self, *a, **k):
+            return super().conv_bits(*a, **k)
+
+    class Own(tab_nn.TABConv2d):
+        def conv_bits(self, QX, N, H, W, residual=None, next_threshold_scale=None):
+            return super().conv_bits(QX, N, H, W, residual, next_threshold_scale)
+
+    w = torch.randn(8, 3, 3, 64, device=cuda)
+    layers = {kind.__name__: kind.from_float(w, 0, 1, 1) for kind in (tab_nn.TABConv2d, Passing, Own)}
+    kw = tab_nn.TABConv2d.pack_together(layers)
+    assert sorted(kw) == ["Passing", "TABConv2d"]
+    qx = layers["Own"].quantize(torch.randn(2, 6, 6, 64, device=cuda))
+    ys = [m.conv_bits(qx, 2, 6, 6, **kw.get(k, {}))[0] for k, m in layers.items()]
+    assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
