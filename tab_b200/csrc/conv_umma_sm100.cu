@@ -1677,11 +1677,13 @@ static bool tc_plan(const TcConvParams& p, int sms, TcPlan* best) {
         // second one empty and waits for its expansion all the same)
         if (pl.tiles_m * pl.tiles_n >= best->tiles_m * best->tiles_n) *best = pl;
     }
-    // A single small image: tiles of 32 filters where even those leave half of the SMs without one and the sum is long (short
-    // ones are done before the second CTA's set-up is: 32x32x64 6.7 us with 64 filters per tile, 7.1 with 32).  With the rule
-    // above, 7x7x512 -> 512: 16.9 -> 15.2 us.
+    // A single small image: tiles of 32 filters where even those leave half of the SMs without one, the sum is long and the
+    // filters are streamed anyway.  GEMM stage alone, us with 64 / 32 filters per tile: 7x7x512->512 3x3 9.76 / 9.60, 14x14x256->256
+    // 6.77 / 6.40, 7x7x2048->512 1x1 9.78 / 9.55, 9x9x448->100 10.26 / 10.08 (72, 36, 32, 63 words); of fewer words 7x7x128->256
+    // (18) 5.59 / 5.41, 14x14x64->64 (9) 4.48 / 4.74.  Filters that stay in shared memory with 64 per tile are better left there:
+    // 14x14x256->64 5.13 / 6.42, 14x14x128->64 5x5 6.01 / 8.19, 16x16x64->64 7x7 6.56 / 9.21.
     TcPlan half;
-    if (found && best->tn == 64 && p.KN > 32 && p.Kw >= 32 && best->tiles_m * best->tiles_n * 4 <= sms && plan_shape(p, sms, 1, 64, 6, &half, false, 32)) *best = half;
+    if (found && best->tn == 64 && !best->resident && p.KN > 32 && p.Kw >= 32 && best->tiles_m * best->tiles_n * 4 <= sms && plan_shape(p, sms, 1, 64, 6, &half, false, 32)) *best = half;
     return found;
 }
 

@@ -1053,3 +1053,16 @@ def test_half_tiles_on_four_bit_operands(cuda, geom, conv_path):
                 t = (float(np.float32(0.7)) * (want.double().abs().reshape(N, -1).sum(dim=1) / want[0].numel())).float()
                 assert torch.equal(got[1], t)                              # whole numbers: exact sums, rounded once
     assert _cabi.lib().tab_device_status() == 0
+
+
+@pytest.mark.parametrize("H,C,KN,K,resident", [(14, 256, 64, 3, 1), (14, 128, 64, 5, 1), (16, 64, 64, 7, 1), (7, 512, 512, 3, 0), (7, 300, 100, 3, 0)])
+def test_tile_rule_for_single_small_images(cuda, H, C, KN, K, resident, conv_path):
+    """Narrower tiles are not taken where that would turn filters that stay in shared memory into streamed ones."""
+    if conv_path != "tensor":
+        pytest.skip("the tensor-core kernel")
+    x, ths = make_input(21, 1, H, H, C)
+    w, wths = make_input(22, KN, K, K, C)
+    qw, btn = O.quantize(w, wths, 2, KN, K, K, C)
+    geom = (K // 2, K // 2, 1, 1, 1, H, H, C, KN, K, K)
+    assert np.array_equal(gpu_conv(cuda, x, qw, ths, btn, 0, *geom), c_oracle.conv2d(x, qw, ths, btn, 0, *geom))
+    assert _cabi.lib().tab_last_conv_kernel().decode().startswith("conv_umma_persist_kernel<1,64,6,%d," % resident)
