@@ -58,12 +58,12 @@ C0 = 64
 CONV_TYPE = 0
 WEIGHT_SEED = 5000
 INPUT_SEED = 5
-# dram__bytes_read.sum + dram__bytes_write.sum per image of the step's largest launch, conv_umma_persist_kernel<2,64,6,1,2,1>
-# (56x56x64 -> 64 with residual and next thresholds), from the ncu capture summarised under profiles/: 54.72 MB read +
-# 10.07 MB written at 64 images.  The bytes read (residual + bit-planes) are proportional to the images; of the 51.4 MB of
-# output only 10 MB had left the 126 MB L2 when that small launch ended, so the scaled figure is a lower bound for a launch
+# dram__bytes_read.sum + dram__bytes_write.sum per image of the step's largest launch, conv_umma_persist_kernel<2,64,6,1,2,1,e2m1>
+# (56x56x64 -> 64 with residual and next thresholds), from an ncu capture of run_case bits --residual --chain: 54.69 MB read +
+# 9.07 MB written at 64 images.  The bytes read (residual + bit-planes) are proportional to the images; of the 51.4 MB of
+# output only 9 MB had left the 126 MB L2 when that small launch ended, so the scaled figure is a lower bound for a launch
 # whose output exceeds the L2 (algorithmic: 1.66 MB per image, of which 0.80 MB output).
-L1_TRAFFIC_PER_IMAGE = (54.720256e6 + 10.072832e6) / 64
+L1_TRAFFIC_PER_IMAGE = (54.689536e6 + 9.072640e6) / 64
 
 
 def parse_args():
@@ -767,7 +767,7 @@ def main():
         "bound": "hbm", "achieved": step_gbs, "peak": hbm_peak, "unit": "GB/s", "frac": step_gbs / hbm_peak, "peak_source": hbm_src,
         "algorithmic_bytes_per_step": step_bytes, "images_per_gpu": n_local,
         "traffic": (L1_TRAFFIC_PER_IMAGE * l1_images) if L1_TRAFFIC_PER_IMAGE else None,
-        "traffic_note": "ncu dram bytes read + written of the step's largest launch (conv_umma_persist_kernel<2,64,6,1,2,1>, 56x56x64 -> 64 with "
+        "traffic_note": "ncu dram bytes read + written of the step's largest launch (conv_umma_persist_kernel<2,64,6,1,2,1,e2m1>, 56x56x64 -> 64 with "
                         "residual), captured at 64 images and scaled to this rank's %d images - a lower bound: at 64 images four fifths of the "
                         "output were still in the L2 when the launch ended; its algorithmic bytes are %.1fe6 (bit-planes + 4-bit weights + fp32 "
                         "residual read + fp32 output)"

@@ -174,8 +174,9 @@ def forward_prepared(convs, x, ths, N: int, H: int = 56, W: int = 56, compact_mi
             oh, ow = (h + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride, (w + 2 * b.conv_a.pad - b.conv_a.K + 1) // b.conv_a.stride
             # From the first strided shortcut on the block results are whole numbers too: conv + conv, conv + conv + conv, ...
             # They travel as int16 as well while their largest possible magnitude fits and the tensor is large enough for its
-            # bytes to matter (0.8M values, 8 images: 267 us with fp32 results and 275 with int16 ones; 6.4M and more, 256
-            # images: 1071 and 983).
+            # bytes to matter.  us with the line at 2^20 / 2^21 / 2^22 / 2^23 elements: 24 images 379.5 / 374.8 / 374.0 / 373.2,
+            # 48 images 442.6 / 441.1 / 439.6 / 449.7, 64 images 482.0 / 478.8 / 479.8 / 495.4, 128 images 612 / 614 / 621 / 634
+            # (fp32 results throughout: 373, 447, 496, 657).
             terms = b.conv_b.K * b.conv_b.K * b.conv_b.C
             short_bound = bound if sc is None else b.shortcut.K * b.shortcut.K * b.shortcut.C
             bound = None if short_bound is None else short_bound + terms

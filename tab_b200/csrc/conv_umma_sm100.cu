@@ -8,20 +8,21 @@
 // decode to +1 (the reference's padding rule), channel tails decode to 0.
 //
 // One CTA per SM walks over output tiles of 128*MT virtual rows x TN filters (see TcConvParams for the virtual grid):
-//   * expander warps (0, 12-15): stage the *patch* of a tile - the 128*MT + halo consecutive virtual rows all its
-//     taps read - for one pair of 64-channel words and one stride plane: 16 bytes of (sign, magnitude) per pixel and
-//     word are loaded from global memory (padding positions are not loaded at all) and expanded to 64 bytes of int8
-//     in the K-major, 128-byte-swizzled layout the MMA descriptors expect.  Two patch buffers; the expanders run up to
-//     two patches ahead of the MMAs, across tile boundaries.
-//   * warp 2: TMA copies of the filter slice (TN x 128 B per tap and channel pair) into a ring of SB stages, or - when
-//     the filters of all taps fit beside the patches (BRES) - once per CTA.
-//   * warps 1 and 3 (row block 0 and row block 1 of a tile): tcgen05.mma.cta_group::1.kind::i8, 128 x TN x 32 per
-//     instruction.  Tap (kh, kw) of the 128 rows of an MMA is 128 consecutive patch rows starting (kh/s1)*VW + kw/s2 rows
-//     into the patch: the A descriptor simply starts there (the 128-byte swizzle is a function of absolute shared-memory
-//     address bits).  Two TMEM accumulator buffers.
-//   * warps 4-11: epilogue of the other accumulator buffer: tcgen05.ld, then either a transposition through a private
-//     shared-memory block so that stores are coalesced, or (TEPI) TMA loads of the residual and TMA stores of the result;
-//     int -> float, residual, per-image sums of |y|.
+//   * expander warps (0, 12 and up, 3 where it has no MMAs to issue): stage the *patch* of a tile - the 128*MT + halo consecutive
+//     virtual rows all its taps read - for the 64-channel words of one 128-byte operand row (four of 4-bit operands, two of
+//     bytes) and one stride plane: 16 bytes of (sign, magnitude) per pixel and word are loaded from global memory (padding
+//     positions are not loaded at all) and expanded to 32 bytes of e2m1 nibbles or 64 of int8 in the K-major, 128-byte-swizzled
+//     layout the MMA descriptors expect.  Two patch buffers; the expanders run up to two patches ahead of the MMAs, across tile
+//     boundaries.
+//   * warp 2: TMA copies of the filter slice (TN x 128 B: up to 256 channels of a tap, or several taps of few channels; of bytes
+//     128 channels of a tap) into a ring of SB stages, or - when the filters of all taps fit beside the patches (BRES) - once per CTA.
+//   * warps 1 and 3 (row block 0 and row block 1 of a tile): tcgen05.mma.cta_group::1, kind::mxf4 (128 x TN x 64 per instruction)
+//     or kind::i8 (128 x TN x 32).  Tap (kh, kw) of the 128 rows of an MMA is 128 consecutive patch rows starting
+//     (kh/s1)*VW + kw/s2 rows into the patch: the A descriptor simply starts there (the 128-byte swizzle is a function of
+//     absolute shared-memory address bits).  Two TMEM accumulator buffers.
+//   * warps 4-11: epilogue of the other accumulator buffer: tcgen05.ld, then a transposition through a private shared-memory block
+//     so that stores are coalesced, or whole rows straight from registers, or (TEPI) TMA loads of the residual and TMA stores of
+//     the result; int -> float, residual, per-image sums of |y|.
 //   * the CTA that finishes last turns the sums into the next layer's thresholds - or, second phase, the whole grid meets
 //     at a counter and quantises the result it has just written for the next convolution (quantize_tail).
 //   * PAIR: the same roles on clusters of two CTAs with one tcgen05.mma.cta_group::2 stream for both (see the kernel).

@@ -172,7 +172,7 @@ __device__ __forceinline__ void umma_i8(uint32_t tmem_d, uint64_t da, uint64_t d
 // kind::mxf4 multiplies e2m1 floats - {-1, 0, +1} are the nibbles 0xA, 0x0, 0x2 - with a power-of-two scale per 32 of them, here
 // always 1, into fp32: 128 x N x 64 in the cycles kind::i8 takes for 128 x N x 32 (measured on B200: 48 / 64 / 128 cycles at N = 64 /
 // 128 / 256 for both).  Products of {-1, 0, +1} accumulate exactly while the sum stays below 2^24 in magnitude, which
-// KH*KW*C < 2^24 guarantees; measured exact with running sums up to 15.4 million.
+// KH*KW*C < 2^24 guarantees (tested with sums just below that, on every tile width).
 // Order of the channels inside a word: the sum does not depend on it as long as both operands agree, so the order is the one
 // that needs no bit spreading - 32-bit word 4h + k of the eight holds channels 32h + 4i + k, i = 0..7 (channel 32h + 4i + k in
 // nibble i), a shift and a mask of plane bits.

@@ -691,9 +691,9 @@ def test_quantize_i16_any_channels(cuda, conv_path, C):
     (1, 1, 1, 1, 2, 14, 14, 256, 259, 3, 3),
     (1, 1, 1, 1, 90, 14, 14, 130, 300, 3, 3),    # CTA pairs of 160-filter tiles
     (1, 1, 1, 1, 60, 14, 14, 64, 450, 3, 3),
-    (0, 0, 1, 1, 30, 28, 28, 64, 384, 1, 1),     # two tiles of 192 filters; last round in halves of 96 or whole
-    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # 150 tiles: two halves of 128 filters, the last partial
-    (0, 0, 1, 1, 75, 16, 16, 64, 222, 1, 1),     # the same with 224-wide tiles, not split
+    (0, 0, 1, 1, 30, 28, 28, 64, 384, 1, 1),     # two tiles of 192 filters
+    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # 150 tiles, the last block partial (filters resident: no halves)
+    (0, 0, 1, 1, 75, 16, 16, 64, 222, 1, 1),     # the same with 224-wide tiles
     (1, 1, 1, 1, 1, 12, 12, 64, 60, 3, 3),       # the TMA epilogue with a partial block
     (1, 1, 1, 1, 1, 12, 12, 64, 28, 3, 3),
 ])
@@ -739,7 +739,7 @@ def test_weight_expansion_inside_a_call(cuda, conv_path, N, KN, K, C):
     (1, 2, 3, 2, 3, 9, 8, 130, 70, 3, 3),
     (1, 1, 1, 1, 40, 3, 3, 64, 67, 3, 3),        # a 32-row slab spans three images
     (1, 1, 1, 1, 40, 3, 3, 64, 64, 3, 3),
-    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # halves
+    (0, 0, 1, 1, 75, 16, 16, 64, 250, 1, 1),     # a second round of two tiles
     (1, 1, 1, 1, 200, 14, 14, 64, 256, 3, 3),    # several tiles per CTA: accumulators that overlap, one row block
     (1, 1, 1, 1, 200, 14, 14, 64, 456, 3, 3),    # 256-filter tiles, the last block of the second one without filters
     (1, 1, 1, 1, 60, 28, 28, 128, 128, 3, 3),    # the same with two row blocks
