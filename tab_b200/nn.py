@@ -86,7 +86,8 @@ class TABConv2d(torch.nn.Module):
         """For a pass through several layers, name -> layer: name -> keywords for its ``conv_bits``, which then need not pack
         the weights by itself.  One launch for all of them instead of one per layer; the packed forms are of ``W8`` as it is
         now and serve this pass only."""
-        own = [(k, c._buffers["W8"]) for k, c in convs.items() if isinstance(c, TABConv2d) and _takes_packed(type(c).conv_bits) and c._four_bit()]
+        own = [(k, c._buffers["W8"]) for k, c in convs.items()
+               if isinstance(c, TABConv2d) and _takes_packed(type(c).conv_bits) and c._four_bit() and c._buffers.get("W8") is not None]
         packed = ops.pack_weights_many([w for _, w in own])
         return {} if packed is None else {k: {"packed": p} for (k, _), p in zip(own, packed)}
 

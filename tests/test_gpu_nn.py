@@ -301,6 +301,11 @@ def test_pack_together_asks_whether_a_layer_takes_it(cuda):
     layers = {kind.__name__: kind.from_float(w, 0, 1, 1) for kind in (tab_nn.TABConv2d, Passing, Own)}
     kw = tab_nn.TABConv2d.pack_together(layers)
     assert sorted(kw) == ["Passing", "TABConv2d"]
+    bare = tab_nn.TABConv2d.from_float(w, 0, 1, 1)
+    w8 = bare.W8
+    del bare.W8
+    bare.__dict__["W8"] = w8                                               # no buffer any more: conv_bits packs it
+    assert tab_nn.TABConv2d.pack_together({"bare": bare}) == {}
     qx = layers["Own"].quantize(torch.randn(2, 6, 6, 64, device=cuda))
     ys = [m.conv_bits(qx, 2, 6, 6, **kw.get(k, {}))[0] for k, m in layers.items()]
     assert torch.equal(ys[0], ys[1]) and torch.equal(ys[0], ys[2])
