@@ -174,7 +174,9 @@ static int conv2d_impl(const float* x, const int64_t* qw, const float* ths, cons
         if (tc_conv_covers(p)) {
             // launch 1: quantise (TAB_GEMM.cu:419-426) + weight expansion + clears; launch 2: the GEMM
             QuantExtras ex;
-            ex.zero_sums = abs_sums;
+            if (N <= 65535) ex.zero_sums = abs_sums;
+            else rc = clear_sums();                                        // the quantiser runs in several launches then, the first of which does the extras
+            if (rc != TAB_OK) return rc;
             ex.zero_counter = next_ths ? counter : nullptr;
             if (p.e2m1) { ex.qw = reinterpret_cast<const uint64_t*>(qw); ex.w4 = w4; }
             else rc = expand_weights_dispatch(qw, reinterpret_cast<int8_t*>(w4), weight_bits(type), KN, KH, KW, C, s);

@@ -1066,3 +1066,24 @@ def test_tile_rule_for_single_small_images(cuda, H, C, KN, K, resident, conv_pat
     geom = (K // 2, K // 2, 1, 1, 1, H, H, C, KN, K, K)
     assert np.array_equal(gpu_conv(cuda, x, qw, ths, btn, 0, *geom), c_oracle.conv2d(x, qw, ths, btn, 0, *geom))
     assert _cabi.lib().tab_last_conv_kernel().decode().startswith("conv_umma_persist_kernel<1,64,6,%d," % resident)
+
+
+def test_sums_of_more_images_than_one_quantiser_launch_takes(cuda, conv_path):
+    """|y| sums and next thresholds of 66000 one-pixel images, into a buffer that holds something else."""
+    N, C, KN = 66000, 64, 5
+    x, ths = make_input(31, N, 1, 1, C)
+    w, wths = make_input(32, KN, 1, 1, C)
+    qw, btn = O.quantize(w, wths, 2, KN, 1, 1, C)
+    lib, geom = _cabi.lib(), (0, 0, 0, 1, 1, N, 1, 1, C, KN, 1, 1)
+    xd, td, qd, bd = (dev_t(a, cuda) for a in (x, ths, qw, btn))
+    y = torch.empty(N * KN, device=cuda)
+    ws = torch.empty(lib.tab_conv2d_workspace_bytes(*geom), dtype=torch.uint8, device=cuda)
+    sums, nxt = torch.full((N,), 1e9, dtype=torch.float64, device=cuda), torch.empty(N, device=cuda)
+    stream = torch.cuda.current_stream(cuda).cuda_stream
+    _cabi.check(lib.tab_conv2d_chain_launch(xd.data_ptr(), qd.data_ptr(), td.data_ptr(), bd.data_ptr(), y.data_ptr(), ws.data_ptr(), ws.numel(), *geom,
+                                            None, sums.data_ptr(), nxt.data_ptr(), 0.7, stream), "chain")
+    yo = c_oracle.conv2d(x, qw, ths, btn, *geom).reshape(N, KN)
+    assert np.array_equal(y.cpu().numpy().reshape(N, KN), yo)
+    total = np.abs(yo.astype(np.float64)).sum(axis=1)
+    assert np.array_equal(sums.cpu().numpy(), total)
+    assert np.array_equal(nxt.cpu().numpy(), (np.float64(np.float32(0.7)) * (total / KN)).astype(np.float32))
